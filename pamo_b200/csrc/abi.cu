@@ -1433,7 +1433,7 @@ int pamo_batch_destroy(pamo_batch *b)
     b->S.release();
     if (b->S.slots) cudaFree(b->S.slots);
     if (b->S.scnt) cudaFree(b->S.scnt);
-    if (b->S.roots) cudaFree(b->S.roots);
+    if (b->S.ranges) cudaFree(b->S.ranges);
     if (b->S.vslot) cudaFree(b->S.vslot);
     if (b->S.gmap) cudaFree(b->S.gmap);
     if (b->S.line_list) cudaFree(b->S.line_list);

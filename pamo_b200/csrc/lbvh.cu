@@ -172,12 +172,8 @@ __device__ __forceinline__ int delta(const uint32_t *keys, int L, int i, int j)
 }
 
 // Karras (2012) hierarchy construction, one thread per internal node.
-// roots (batch of meshes, rank in the key bits above `rank_shift`): the child
-// of a node spanning several ranks that holds one rank only is that rank's
-// whole subtree (keys of one rank are contiguous and share every bit above the
-// split), recorded as the start node of the rank's queries.
 __global__ void __launch_bounds__(kThreads) k_karras(const uint32_t *keys, const int *scene, BvhNode *nodes,
-                                                     int *parent, int *roots, int rank_shift)
+                                                     int *parent)
 {
     const int L = scene[7];
     PAMO_GRID_STRIDE(ii, (long long)L - 1)
@@ -210,13 +206,6 @@ __global__ void __launch_bounds__(kThreads) k_karras(const uint32_t *keys, const
         parent[lid] = (i << 2) | tile | 0;
         parent[rid] = (i << 2) | tile | 1;
         if (i == 0) parent[0] = -1;
-        if (roots) {
-            const uint32_t rlo = keys[lo] >> rank_shift, rhi = keys[hi] >> rank_shift;
-            if (rlo != rhi) {
-                if (rlo == (keys[gamma] >> rank_shift)) roots[rlo] = left;
-                if (rhi == (keys[gamma + 1] >> rank_shift)) roots[rhi] = right;
-            }
-        }
     }
 }
 
@@ -295,54 +284,6 @@ __global__ void __launch_bounds__(kRefitTile) k_refit(const float4 *pts, const i
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_refit_dirty(const float4 *pts, const int4 *tris, const int *vals,
-                                                          int *scene, const int *parent, BvhNode *nodes, int *claim,
-                                                          int *dmask, int *dcount, const int *dlist)
-{
-    const int L = scene[7];
-    const int n = scene[9];
-    PAMO_GRID_STRIDE(k, n)
-    {
-        const int p = dlist[k];
-        claim[p] = 0;
-        const int f = vals[p];
-        int4 t = f >= 0 ? tris[f] : make_int4(-1, -1, -1, 0);
-        float3 lo, hi;
-        if (face_dead(t)) {
-            lo = make_float3(INFINITY, INFINITY, INFINITY);
-            hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
-        } else {
-            face_box(pts, t, lo, hi);
-        }
-        int code = parent[(L - 1) + p];
-        store_child_box(nodes, code, ~p, lo, hi);
-        int node = code >> 2;
-        for (int depth = 0;; ++depth) {
-            if (depth > 256) {
-                atomicExch(&scene[8], 1);
-                break;
-            }
-            // the marks were set by an earlier kernel; read them before arriving,
-            // since the last child to arrive clears them
-            const int need = __popc(__ldcg(&dmask[node]));
-            __threadfence();
-            const int old = atomicAdd(&dcount[node], 1);
-            if (old + 1 < need) break;  // the other dirty child merges this node
-            __threadfence();
-            float4 a = __ldcg(&nodes[node].llo), b = __ldcg(&nodes[node].lhi);
-            float4 c = __ldcg(&nodes[node].rlo), d = __ldcg(&nodes[node].rhi);
-            lo = make_float3(fminf(a.x, c.x), fminf(a.y, c.y), fminf(a.z, c.z));
-            hi = make_float3(fmaxf(b.x, d.x), fmaxf(b.y, d.y), fmaxf(b.z, d.z));
-            dmask[node] = 0;
-            dcount[node] = 0;
-            const int pc = parent[node];
-            if (pc < 0) break;  // root
-            store_child_box(nodes, pc, node, lo, hi);
-            node = pc >> 2;
-        }
-    }
-}
-
 __global__ void k_count_leaves(int m, int *scene) { scene[7] = m - scene[6]; }
 
 }  // namespace
@@ -374,24 +315,14 @@ cudaError_t Lbvh::ensure(long long n)
     ALLOC(flags, c * 4);
     ALLOC(leaf_of_face, c * 4);
     ALLOC(scene, 64);
-    ALLOC(claim, c * 4);
-    ALLOC(dmask, c * 4);
-    ALLOC(dcount, c * 4);
-    ALLOC(dlist, c * 4);
 #undef ALLOC
-    if ((e = cudaMemset(claim, 0, c * 4)) != cudaSuccess || (e = cudaMemset(dmask, 0, c * 4)) != cudaSuccess ||
-        (e = cudaMemset(dcount, 0, c * 4)) != cudaSuccess) {
-        release();
-        return e;
-    }
     cap = c;
     return cudaSuccess;
 }
 
 void Lbvh::release()
 {
-    void *p[] = {keys, keys2, vals, vals2, hist, hist_scratch, nodes, parent, flags, leaf_of_face, scene, claim, dmask,
-                 dcount, dlist};
+    void *p[] = {keys, keys2, vals, vals2, hist, hist_scratch, nodes, parent, flags, leaf_of_face, scene};
     for (void *q : p)
         if (q) cudaFree(q);
     keys = keys2 = nullptr;
@@ -399,54 +330,52 @@ void Lbvh::release()
     hist = hist_scratch = nullptr;
     nodes = nullptr;
     parent = flags = leaf_of_face = scene = nullptr;
-    claim = dmask = dcount = dlist = nullptr;
     cap = 0;
     leaves_built = 0;
 }
 
-cudaError_t lbvh_build(Lbvh &b, const float4 *pts, const int4 *tris, int m, cudaStream_t s, const int *vslot,
-                       int n_ranks, int *roots)
+cudaError_t morton_order(const float4 *pts, const int4 *tris, int m, int *scene, uint32_t *keys, uint32_t *keys2,
+                         int *vals, int *vals2, int *hist, int *hist_scratch, const int *vslot, int n_ranks,
+                         int &rank_shift, cudaStream_t s)
 {
-    cudaError_t e = b.ensure(m);
-    if (e != cudaSuccess) return e;
-    b.leaves_built = m;
-    launch(k_scene_init, 1, 32, 0, s, b.scene);
+    launch(k_scene_init, 1, 32, 0, s, scene);
     if (m == 0) return cudaGetLastError();
-    launch(k_scene_bounds, grid_for(m), kThreads, 0, s, pts, tris, m, b.scene);
+    launch(k_scene_bounds, grid_for(m), kThreads, 0, s, pts, tris, m, scene);
     // Morton bits per axis: 10, or fewer to leave room for the rank (keys of live
     // faces stay below 2^31, under the key of removed faces)
     int rank_bits = 0;
     while (vslot && (1 << rank_bits) < n_ranks) ++rank_bits;
     const int bits = vslot ? (31 - rank_bits) / 3 : 10;
-    if (roots) {
-        e = cudaMemsetAsync(roots, 0, (size_t)n_ranks * 4, s);  // one rank: the whole tree
-        if (e != cudaSuccess) return e;
-    }
-    launch(k_morton, grid_for(m), kThreads, 0, s, pts, tris, m, b.scene, b.keys, b.vals, vslot, bits);
-    int tiles = (m + kSortTile - 1) / kSortTile;
-    uint32_t *k_in = b.keys, *k_out = b.keys2;
-    int *v_in = b.vals, *v_out = b.vals2;
+    rank_shift = 3 * bits;
+    launch(k_morton, grid_for(m), kThreads, 0, s, pts, tris, m, (const int *)scene, keys, vals, vslot, bits);
+    const int tiles = (m + kSortTile - 1) / kSortTile;
+    uint32_t *k_in = keys, *k_out = keys2;
+    int *v_in = vals, *v_out = vals2;
     for (int shift = 0; shift < 32; shift += 8) {
-        launch(k_radix_hist, tiles, kSortThreads, 0, s, k_in, m, shift, tiles, b.hist);
-        e = exclusive_scan(b.hist, b.hist, (long long)256 * tiles, nullptr, b.hist_scratch, nullptr, s);
+        launch(k_radix_hist, tiles, kSortThreads, 0, s, k_in, m, shift, tiles, hist);
+        cudaError_t e = exclusive_scan(hist, hist, (long long)256 * tiles, nullptr, hist_scratch, nullptr, s);
         if (e != cudaSuccess) return e;
-        launch(k_radix_scatter, tiles, kSortThreads, 0, s, k_in, v_in, m, shift, tiles, b.hist, k_out, v_out);
+        launch(k_radix_scatter, tiles, kSortThreads, 0, s, k_in, v_in, m, shift, tiles, hist, k_out, v_out);
         uint32_t *tk = k_in; k_in = k_out; k_out = tk;
         int *tv = v_in; v_in = v_out; v_out = tv;
     }
     // after an even number of passes the sorted data is back in keys/vals
-    launch(k_count_leaves, 1, 1, 0, s, m, b.scene);
-    launch(k_karras, grid_for(m), kThreads, 0, s, b.keys, b.scene, b.nodes, b.parent, vslot ? roots : nullptr,
-           3 * bits);
-    launch(k_leaf_map, grid_for(m), kThreads, 0, s, b.vals, b.scene, b.leaf_of_face, m);
     return cudaGetLastError();
 }
 
-cudaError_t lbvh_refit_dirty(Lbvh &b, const float4 *pts, const int4 *tris, long long max_dirty, cudaStream_t s)
+cudaError_t lbvh_build(Lbvh &b, const float4 *pts, const int4 *tris, int m, cudaStream_t s)
 {
-    if (b.leaves_built < 2 || max_dirty <= 0) return cudaSuccess;
-    launch(k_refit_dirty, grid_for(max_dirty), kThreads, 0, s, pts, tris, (const int *)b.vals, b.scene,
-           (const int *)b.parent, b.nodes, b.claim, b.dmask, b.dcount, (const int *)b.dlist);
+    cudaError_t e = b.ensure(m);
+    if (e != cudaSuccess) return e;
+    b.leaves_built = m;
+    int shift = 0;
+    e = morton_order(pts, tris, m, b.scene, b.keys, b.keys2, b.vals, b.vals2, b.hist, b.hist_scratch, nullptr, 0,
+                     shift, s);
+    if (e != cudaSuccess) return e;
+    if (m == 0) return cudaGetLastError();
+    launch(k_count_leaves, 1, 1, 0, s, m, b.scene);
+    launch(k_karras, grid_for(m), kThreads, 0, s, b.keys, b.scene, b.nodes, b.parent);
+    launch(k_leaf_map, grid_for(m), kThreads, 0, s, b.vals, b.scene, b.leaf_of_face, m);
     return cudaGetLastError();
 }
 

@@ -1,4 +1,4 @@
-// Linear BVH over the faces of one mesh round (used by the stage-2 undo check).
+// Linear BVH over the faces of a mesh (stage 3 and the acceptance checks).
 //
 // Build: 30-bit Morton code of each face's box centre (10 bits per axis over the
 // scene box) -> stable LSD radix sort (4 x 8-bit digits, hand written) ->
@@ -10,8 +10,7 @@
 // geometry then); a caller that removes and renumbers faces may keep the tree by
 // rewriting the leaves' face indices (-1 for a removed face).  Refit recomputes every leaf box from the current
 // geometry (a dead face gets the empty box lo=+inf, hi=-inf, which overlaps
-// nothing) and rebuilds the inner boxes, so the undo passes never rebuild the
-// hierarchy.
+// nothing) and rebuilds the inner boxes.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -54,53 +53,27 @@ struct Lbvh {
     int *scene = nullptr;       // 6 ordered ints + n_dead + n_leaves
     int sort_tiles = 0;
     long long leaves_built = 0;  // faces of the last build: bound on the leaf count
-    // incremental refit (lbvh_mark_dirty_leaf / lbvh_refit_dirty); all zero between refits
-    int *claim = nullptr;   // [cap] leaf listed as dirty
-    int *dmask = nullptr;   // [cap] per inner node: which children hold a dirty leaf (bit 0 left, 1 right)
-    int *dcount = nullptr;  // [cap] per inner node: dirty children merged so far
-    int *dlist = nullptr;   // [cap] dirty leaves; their count is scene[9]
 
     cudaError_t ensure(long long n_faces);
     void release();
 };
 
+// The order of the faces [0, m) by the Morton code of their box centre, 10 bits
+// per axis over the scene box (written to scene[0..5], the removed faces' count
+// to scene[6]), by a stable radix sort: keys and vals (face indices) ascending,
+// removed faces last.  For a batch of meshes (vslot: each vertex's mesh rank <
+// n_ranks) the rank is the top of the key, from bit rank_shift up, and the codes
+// have fewer bits.  hist: 256 counts per tile of kLbvhSortTile faces.
+cudaError_t morton_order(const float4 *pts, const int4 *tris, int m, int *scene, uint32_t *keys, uint32_t *keys2,
+                         int *vals, int *vals2, int *hist, int *hist_scratch, const int *vslot, int n_ranks,
+                         int &rank_shift, cudaStream_t s);
+
 // Builds the hierarchy for faces [0, m): leaves are the faces live in `tris`
-// (the round input), ordered by the Morton code of their box centre.  For a
-// batch of meshes, vslot gives each vertex's mesh rank (< n_ranks): each mesh
-// gets its own subtree, whose start node (internal index, or ~leaf position for
-// a one-face mesh) is written to roots[rank].
-cudaError_t lbvh_build(Lbvh &b, const float4 *pts, const int4 *tris, int m, cudaStream_t s,
-                       const int *vslot = nullptr, int n_ranks = 0, int *roots = nullptr);
+// (the round input), ordered by the Morton code of their box centre.
+cudaError_t lbvh_build(Lbvh &b, const float4 *pts, const int4 *tris, int m, cudaStream_t s);
 
 // Recomputes all boxes from the current geometry (pts, tris).  A leaf whose face
 // index is negative (a face removed after the build) gets the empty box.
 cudaError_t lbvh_refit(Lbvh &b, const float4 *pts, const int4 *tris, int m, cudaStream_t s);
-
-// Incremental refit, for boxes that were all up to date before some faces
-// changed: the caller lists the changed faces' leaves with lbvh_mark_dirty_leaf
-// (in a kernel, after zeroing scene[9]); lbvh_refit_dirty then recomputes those
-// leaves and, bottom-up, exactly the inner nodes above them (a node is merged by
-// the last of its dirty children to arrive).  Leaves the marks zero again.
-__device__ __forceinline__ void lbvh_mark_dirty_leaf(int p, int L, const int *parent, int *claim, int *dmask,
-                                                     int *dlist, int *scene)
-{
-    if (atomicExch(&claim[p], 1) != 0) return;  // listed already
-    {  // one counter atomic per group of lanes listing together
-        cooperative_groups::coalesced_group g = cooperative_groups::coalesced_threads();
-        int base = 0;
-        if (g.thread_rank() == 0) base = atomicAdd(&scene[9], (int)g.size());
-        dlist[g.shfl(base, 0) + (int)g.thread_rank()] = p;
-    }
-    int code = parent[(L - 1) + p];
-    // mark the path to the root; a node already marked has its path marked (or
-    // being marked) by the leaf that got there first
-    for (int depth = 0; depth < 256 && code >= 0; ++depth) {
-        const int node = code >> 2;
-        if (atomicOr(&dmask[node], 1 << (code & 1)) != 0) break;
-        code = parent[node];
-    }
-}
-
-cudaError_t lbvh_refit_dirty(Lbvh &b, const float4 *pts, const int4 *tris, long long max_dirty, cudaStream_t s);
 
 }  // namespace pamo

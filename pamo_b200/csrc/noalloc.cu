@@ -4,6 +4,7 @@
 #include <cstring>
 
 #include "lbvh.cuh"
+#include "ptree.cuh"
 #include "scan.cuh"
 #include "stage2.cuh"
 
@@ -13,29 +14,27 @@ namespace {
 constexpr int kMaxFaces = 32768;   // limit of this entry point
 constexpr int kMaxVerts = 65536;
 constexpr int kPairsPerFace = 24;  // sizes the pair buffer: 24 * kMaxFaces candidate pairs in total
-constexpr int kTiles = (kMaxFaces + kLbvhSortTile - 1) / kLbvhSortTile;  // lbvh_build's sort tiles
+constexpr int kTiles = (kMaxFaces + kLbvhSortTile - 1) / kLbvhSortTile;  // the Morton sort's tiles
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // byte offsets inside the scratch array
 constexpr size_t kOffPts = 0;
 constexpr size_t kOffTris = kOffPts + align256(sizeof(float4) * kMaxVerts);
-constexpr size_t kOffActive = kOffTris + align256(sizeof(int4) * kMaxFaces);
-constexpr size_t kOffKeys = kOffActive + align256(kMaxFaces);
+constexpr size_t kOffKeys = kOffTris + align256(sizeof(int4) * kMaxFaces);
 constexpr size_t kOffKeys2 = kOffKeys + align256(4 * (size_t)kMaxFaces);
 constexpr size_t kOffVals = kOffKeys2 + align256(4 * (size_t)kMaxFaces);
 constexpr size_t kOffVals2 = kOffVals + align256(4 * (size_t)kMaxFaces);
 constexpr size_t kOffHist = kOffVals2 + align256(4 * (size_t)kMaxFaces);
 constexpr size_t kOffHistScratch = kOffHist + align256(4 * (256 * (size_t)kTiles + 64));
-constexpr size_t kOffNodes = kOffHistScratch + align256(4 * (size_t)scan_scratch_ints(256LL * kTiles));
-constexpr size_t kOffParent = kOffNodes + align256(sizeof(BvhNode) * kMaxFaces);
-constexpr size_t kOffFlags = kOffParent + align256(4 * 2 * (size_t)kMaxFaces);
-constexpr size_t kOffLeafOfFace = kOffFlags + align256(4 * (size_t)kMaxFaces);
-constexpr size_t kOffScene = kOffLeafOfFace + align256(4 * (size_t)kMaxFaces);
+constexpr size_t kOffBoxes = kOffHistScratch + align256(4 * (size_t)scan_scratch_ints(256LL * kTiles));
+constexpr size_t kOffLeaf = kOffBoxes + align256(2 * sizeof(float4) * (size_t)tree_nodes(kMaxFaces));
+constexpr size_t kOffQuery = kOffLeaf + align256(sizeof(int4) * (size_t)kMaxFaces);
+constexpr size_t kOffScene = kOffQuery + align256(4 * (size_t)kMaxFaces);
 constexpr size_t kOffPairs = kOffScene + align256(64);
 constexpr size_t kOffCounters = kOffPairs + align256(sizeof(uint2) * kPairsPerFace * (size_t)kMaxFaces);
 constexpr size_t kOffBad = kOffCounters + align256(sizeof(RoundCounters));
-constexpr size_t kScratchBytes = kOffBad + 256;  // about 11 MB
+constexpr size_t kScratchBytes = kOffBad + 256;  // about 10 MB
 static_assert(kOffHistScratch - kOffHist >= 4 * (256 * (size_t)kTiles), "radix histogram area");
 static_assert(kOffPairs - kOffScene >= 64, "scene area");
 
@@ -101,40 +100,33 @@ extern "C" int pamo_self_intersect_noalloc(const float *d_points, const int *d_t
 
     float4 *p4 = reinterpret_cast<float4 *>(base + kOffPts);
     int4 *t4 = reinterpret_cast<int4 *>(base + kOffTris);
-    uint8_t *active = base + kOffActive;
     uint2 *pairs = reinterpret_cast<uint2 *>(base + kOffPairs);
     RoundCounters *cnt = reinterpret_cast<RoundCounters *>(base + kOffCounters);
-    Lbvh b;  // views into the scratch array; never released (nothing was allocated)
+    int *qlist = reinterpret_cast<int *>(base + kOffQuery);
+    PackedTree b;  // views into the scratch array; never released (nothing was allocated)
     b.cap = kMaxFaces;
-    b.sort_tiles = kTiles;
     b.keys = reinterpret_cast<uint32_t *>(base + kOffKeys);
     b.keys2 = reinterpret_cast<uint32_t *>(base + kOffKeys2);
     b.vals = reinterpret_cast<int *>(base + kOffVals);
     b.vals2 = reinterpret_cast<int *>(base + kOffVals2);
     b.hist = reinterpret_cast<int *>(base + kOffHist);
     b.hist_scratch = reinterpret_cast<int *>(base + kOffHistScratch);
-    b.nodes = reinterpret_cast<BvhNode *>(base + kOffNodes);
-    b.parent = reinterpret_cast<int *>(base + kOffParent);
-    b.flags = reinterpret_cast<int *>(base + kOffFlags);
-    b.leaf_of_face = reinterpret_cast<int *>(base + kOffLeafOfFace);
+    b.boxes = reinterpret_cast<float4 *>(base + kOffBoxes);
+    b.leaf = reinterpret_cast<int4 *>(base + kOffLeaf);
     b.scene = reinterpret_cast<int *>(base + kOffScene);
 
     // the array keeps the previous call's contents: reset what must start at zero
     launch(k_na_convert, grid_for(n_pts > n_tris ? n_pts : n_tris), kThreads, 0, s, d_points, n_pts, d_tris, n_tris, p4,
                                                                                t4);
-    if (cudaMemsetAsync(active, 1, (size_t)n_tris, s) != cudaSuccess) return PAMO_ERR_DEVICE;
     if (cudaMemsetAsync(cnt, 0, sizeof(RoundCounters), s) != cudaSuccess) return PAMO_ERR_DEVICE;
-    if (cudaMemsetAsync(d_out_flags, 0, (size_t)n_tris, s) != cudaSuccess) return PAMO_ERR_DEVICE;
-    if (lbvh_build(b, p4, t4, n_tris, s) != cudaSuccess) return PAMO_ERR_DEVICE;
-    if (lbvh_refit(b, p4, t4, n_tris, s) != cudaSuccess) return PAMO_ERR_DEVICE;
+    if (tree_build(b, p4, t4, n_tris, s) != cudaSuccess) return PAMO_ERR_DEVICE;
     const long long cap_pairs = (long long)kPairsPerFace * kMaxFaces;
-    if (query_and_test_pairs(b.nodes, b.vals, b.scene, p4, t4, active, n_tris, pairs, cap_pairs, cnt, d_out_flags, s) !=
-        cudaSuccess)
+    if (query_and_test_pairs(b, p4, t4, n_tris, qlist, pairs, cap_pairs, cnt, d_out_flags, s) != cudaSuccess)
         return PAMO_ERR_DEVICE;
     RoundCounters h{};
     if (cudaMemcpyAsync(&h, cnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s) != cudaSuccess) return PAMO_ERR_DEVICE;
     if (cudaStreamSynchronize(s) != cudaSuccess) return PAMO_ERR_DEVICE;
-    if (h.pair_overflow > 0 || h.stack_overflow > 0) return PAMO_ERR_CAPACITY;
+    if (h.pair_overflow > 0) return PAMO_ERR_CAPACITY;
     if (out_n_pairs) *out_n_pairs = h.n_pairs;
     return PAMO_OK;
 }

@@ -431,11 +431,10 @@ __device__ __forceinline__ int chunk_edges(const int *order, const int *first_ed
 }
 
 template <bool QUALITY>
-__global__ void __launch_bounds__(kThreads) k_edge_cost(CostArgs A, const int *order, const int *scene,
+__global__ void __launch_bounds__(kThreads) k_edge_cost(CostArgs A, const int *order, int L,
                                                         const int *first_edge)
 {
     __shared__ int s_list[kChunkEdges];
-    const int L = scene[7];
     for (long long base = (long long)blockIdx.x * kChunkFaces; base < L; base += (long long)gridDim.x * kChunkFaces) {
         const int total = chunk_edges(order, first_edge, L, base, s_list);
         for (int q = threadIdx.x; q < total; q += kThreads) {
@@ -703,21 +702,20 @@ __global__ void __launch_bounds__(kLineThreads) k_line_apply(const int2 *edges, 
     cnt->n_considered = cnt->n_total < window ? cnt->n_total : window;
 }
 
-__global__ void k_mark_active(const int *collapsed, const RoundCounters *cnt, const int2 *edges,
-                              const int *first_near, const int *near_tris, uint8_t *active)
+// The faces of the one-rings of the listed edges: those that query the tree.
+__global__ void k_mark_active(const int *list, const int *n_list, const int2 *edges, const int *first_near,
+                              const int *near_tris, uint8_t *active)
 {
-    const int N = cnt->n_considered;
+    const int N = *n_list;
     PAMO_GRID_STRIDE(p, N)
     {
-        int2 ed = edges[collapsed[p]];
+        int2 ed = edges[list[p]];
         for (int a = first_near[ed.x]; a < first_near[ed.x + 1]; ++a) active[near_tris[a]] = 1;
         for (int a = first_near[ed.y]; a < first_near[ed.y + 1]; ++a) active[near_tris[a]] = 1;
     }
 }
 
-constexpr int kStack = 96;
-
-__device__ __forceinline__ bool box_overlap(float4 alo, float4 ahi, float3 qlo, float3 qhi)
+__device__ __forceinline__ bool box_overlap(float4 alo, float4 ahi, float4 qlo, float4 qhi)
 {
     return !(ahi.x < qlo.x || qhi.x < alo.x || ahi.y < qlo.y || qhi.y < alo.y || ahi.z < qlo.z || qhi.z < alo.z);
 }
@@ -728,100 +726,91 @@ __device__ __forceinline__ int shared_indices(int4 a, int4 b)
            (a.z == b.x) + (a.z == b.y) + (a.z == b.z);
 }
 
-// The active live faces in leaf (Morton) order, appended a warp at a time, so
-// the query threads that follow all have a face and neighbouring lanes walk
-// neighbouring paths.  In a batch, only the faces of meshes whose undo loop
-// still runs (a mesh whose last check found nothing would find nothing again
-// on its unchanged geometry, and pairs never cross meshes).
-__global__ void k_active_list(const int *__restrict__ vals, const int *scene, const uint8_t *__restrict__ active,
-                              const int4 *__restrict__ tris, int *qlist, RoundCounters *cnt, const SlotInfo *slots,
-                              const int *vslot)
-{
-    const int L = scene[7];
-    const int lane = threadIdx.x & 31;
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < L; base += (long long)blockDim.x * gridDim.x) {
-        const long long p = base + threadIdx.x;
-        int f = p < L ? vals[p] : -1;
-        bool ok = f >= 0 && active[f];
-        if (ok) {
-            const int v0 = tris[f].x;
-            ok = v0 != -1 && (!slots || slots[vslot[v0]].in_undo);
-        }
-        unsigned ball = __ballot_sync(0xffffffffu, ok);
-        int first = 0;
-        if (lane == 0 && ball) first = atomicAdd(&cnt->n_query, __popc(ball));
-        first = __shfl_sync(0xffffffffu, first, 0);
-        if (ok) qlist[first + __popc(ball & ((1u << lane) - 1u))] = f;
-    }
-}
+// The leaves whose boxes overlap each listed leaf's, as candidate pairs: a group
+// of eight lanes per query (TreeWalk), four queries a warp.  A pair of two
+// selected faces is emitted once (by the lower index); pairs sharing
+// `skip_shared` or more vertex indices are dropped: 2 for the reference's test,
+// which never reports pairs sharing an edge; 4 (none) for the exact test of
+// quality mode.  ranges (a batch): a query stays in its own mesh's run of leaves.
+//
+// A walk is a chain of dependent loads, so its length sets the time: one thread
+// per query on a binary hierarchy followed ~100 nodes and loaded each leaf's
+// face, flag and corners one after another (81 / 141 / 239 us a pass, mean over
+// the rounds of meshes of 5k / 200k / 2M faces).  Here a step tests eight boxes,
+// and a leaf's record comes with its box: 18 / 28 / 82 us.  The pairs gather in
+// shared memory and leave 32 at a time, one counter update for each 32.
+constexpr int kQueryThreads = 256;
 
-// For each active live face, enumerate overlapping leaves and append candidate
-// pairs.  A pair of two active faces is emitted once (by the lower index);
-// pairs sharing `skip_shared` or more vertex indices are dropped: 2 for the
-// reference's test, which never reports pairs sharing an edge; 4 (none) for
-// the exact test of quality mode.
-__global__ void __launch_bounds__(kThreads) k_query(const BvhNode *__restrict__ nodes, const int *__restrict__ vals,
-                                                    const int *scene, const float4 *__restrict__ pts,
-                                                    const int4 *__restrict__ tris, const uint8_t *__restrict__ active,
-                                                    int m, uint2 *pairs, long long cap_pairs, RoundCounters *cnt,
-                                                    const int *roots, const int *vslot, const int *qlist,
-                                                    int skip_shared)
+template <bool BATCH>
+__global__ void __launch_bounds__(kQueryThreads) k_query(TreeView T, const int *__restrict__ qlist,
+                                                         RoundCounters *cnt, uint2 *pairs, long long cap_pairs,
+                                                         int skip_shared, const int2 *__restrict__ ranges,
+                                                         const int *__restrict__ vslot)
 {
-    const int L = scene[7];
-    int stack[kStack];
-    // queries from the list of active faces (k_active_list), or every leaf in
-    // leaf order with the inactive ones skipped
-    const int N = qlist ? cnt->n_query : L;
-    PAMO_GRID_STRIDE(pp, N)
-    {
-        const int f = qlist ? qlist[pp] : vals[pp];
-        if (f < 0 || !active[f] || L < 2) continue;
-        int4 t = tris[f];
-        if (t.x == -1) continue;
-        float4 a = pts[t.x], b = pts[t.y], c = pts[t.z];
-        float3 qlo = make_float3(fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)));
-        float3 qhi = make_float3(fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)));
-        // a batch starts at the face's own mesh subtree (a leaf: a one-face mesh)
-        const int start = roots ? roots[vslot[t.x]] : 0;
-        if (start < 0) continue;
-        int sp = 0;
-        stack[sp++] = start;
-        // a tree visits each of its L-1 inner nodes at most once per query; the
-        // bound only guards against a corrupted hierarchy
-        int budget = 2 * L + 16;
-        while (sp > 0) {
-            if (--budget < 0) {
-                atomicAdd(&cnt->stack_overflow, 1);
-                break;
-            }
-            const BvhNode nd = nodes[stack[--sp]];
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                float4 lo = side ? nd.rlo : nd.llo;
-                float4 hi = side ? nd.rhi : nd.lhi;
-                if (!box_overlap(lo, hi, qlo, qhi)) continue;
-                int child = __float_as_int(lo.w);
-                if (child < 0) {
-                    int g = vals[~child];
-                    if (g < 0 || g == f) continue;  // empty leaves have empty boxes; guard anyway
-                    if (active[g] && g < f) continue;
-                    int4 tg = tris[g];
-                    if (shared_indices(t, tg) >= skip_shared) continue;
-                    // one atomic per group of lanes appending together
-                    cg::coalesced_group grp = cg::coalesced_threads();
-                    int base = 0;
-                    if (grp.thread_rank() == 0) base = atomicAdd(&cnt->n_pairs, (int)grp.size());
-                    int pos = grp.shfl(base, 0) + (int)grp.thread_rank();
-                    if (pos < cap_pairs) pairs[pos] = make_uint2((unsigned)f, (unsigned)g);
-                    else atomicAdd(&cnt->pair_overflow, 1);
-                } else if (sp < kStack) {
-                    stack[sp++] = child;
-                } else {
-                    atomicAdd(&cnt->stack_overflow, 1);
+    __shared__ uint2 s_pairs[kQueryThreads / 32][64];
+    uint2 *buf = s_pairs[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
+    const unsigned below = (1u << lane) - 1u;
+    const int N = cnt->n_query;
+    int held = 0;  // pairs in buf
+    auto flush = [&](int n) {
+        int first = 0;
+        if (lane == 0) first = atomicAdd(&cnt->n_pairs, n);
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (lane < n) {
+            const long long pos = (long long)first + lane;
+            if (pos < cap_pairs) pairs[pos] = buf[lane];
+            else atomicAdd(&cnt->pair_overflow, 1);
+        }
+    };
+    const long long warps = (long long)gridDim.x * (kQueryThreads / 32);
+    for (long long w = ((long long)blockIdx.x * kQueryThreads + threadIdx.x) >> 5; w * 4 < N; w += warps) {
+        const long long k = w * 4 + (lane >> 3);
+        const bool has = k < N;
+        const int q = has ? qlist[k] : 0;
+        const int4 t = T.leaf[q];
+        const float4 qlo = T.boxes[2 * (size_t)q], qhi = T.boxes[2 * (size_t)q + 1];
+        int2 rg = make_int2(0, 0);
+        if (BATCH && has) rg = ranges[vslot[t.x]];
+        TreeWalk wk;
+        wk.start(T, has);
+        while (__any_sync(0xffffffffu, wk.run)) {
+            bool hit = false, emit = false;
+            int other = 0;
+            if (wk.run) {
+                const int node = 8 * wk.g + gl;
+                const size_t b = 2 * ((size_t)T.off[wk.lvl] + node);
+                const float4 lo = T.boxes[b], hi = T.boxes[b + 1];
+                const bool leaf = wk.lvl == 0 && node < T.L;
+                const int4 r = leaf ? T.leaf[node] : make_int4(-1, -1, -1, kLeafDead);
+                hit = box_overlap(lo, hi, qlo, qhi);
+                if (BATCH) {
+                    const long long first = (long long)node << (3 * wk.lvl), end = ((long long)node + 1) << (3 * wk.lvl);
+                    hit = hit && first < rg.y && end > rg.x;
+                }
+                if (leaf && hit && node != q && r.w != kLeafDead) {
+                    other = leaf_face(r.w);
+                    emit = !(r.w >= 0 && other < t.w) && shared_indices(t, r) < skip_shared;
                 }
             }
+            const unsigned hits = __ballot_sync(0xffffffffu, hit), em = __ballot_sync(0xffffffffu, emit);
+            if (em) {
+                if (emit) buf[held + __popc(em & below)] = make_uint2((unsigned)t.w, (unsigned)other);
+                held += __popc(em);
+                __syncwarp();
+                if (held >= 32) {
+                    flush(32);
+                    held -= 32;
+                    const uint2 rest = buf[32 + lane];
+                    __syncwarp();
+                    buf[lane] = rest;
+                    __syncwarp();
+                }
+            }
+            if (wk.run) wk.advance(T, (hits >> shift) & 255u);
         }
     }
+    if (held > 0) flush(held);
 }
 
 __device__ __forceinline__ void load_face(const float4 *pts, int4 t, float out[3][3], int idx[3])
@@ -956,40 +945,13 @@ __global__ void k_compact(const float4 *pts, const int *occ, const int *pts_map,
     }
 }
 
-// After compaction: leaf p's face gets its compacted index, or -1 if removed
-// (every surviving face is a leaf, so leaf_of_face is complete again).
-__global__ void k_remap_leaves(int *vals, const int *scene, const int *fflag, const int *fpos, int *leaf_of_face)
+// After compaction: leaf p's face gets its compacted index, or -1 if removed.
+__global__ void k_remap_leaves(int *vals, int L, const int *fflag, const int *fpos)
 {
-    const int L = scene[7];
     PAMO_GRID_STRIDE(p, L)
     {
-        int f = vals[p];
-        int nf = (f >= 0 && fflag[f]) ? fpos[f] : -1;
-        vals[p] = nf;
-        if (nf >= 0) leaf_of_face[nf] = (int)p;
-    }
-}
-
-// Leaves whose boxes changed since the last refit: the faces of the one-rings of
-// the listed edges (collapses, coincident-endpoint collapses and undos only
-// change those faces and their vertices).
-__global__ void k_mark_dirty(const int *elist, const int *n_list, const int2 *edges, const int *first_near,
-                             const int *near_tris, const int *leaf_of_face, const int *parent, int *claim,
-                             int *dmask, int *dlist, int *scene)
-{
-    const int N = *n_list;
-    const int L = scene[7];
-    if (L < 2) return;
-    PAMO_GRID_STRIDE(k, N)
-    {
-        const int2 ed = edges[elist[k]];
-        for (int side = 0; side < 2; ++side) {
-            const int w = side ? ed.y : ed.x;
-            for (int a = first_near[w]; a < first_near[w + 1]; ++a) {
-                const int p = leaf_of_face[near_tris[a]];
-                if (p >= 0) lbvh_mark_dirty_leaf(p, L, parent, claim, dmask, dlist, scene);
-            }
-        }
+        const int f = vals[p];
+        vals[p] = (f >= 0 && fflag[f]) ? fpos[f] : -1;
     }
 }
 
@@ -1302,10 +1264,8 @@ void Stage2::release()
     nxt = nullptr;
     vmin = nullptr; eflag = collapsed = nullptr; active = isect = nullptr; uflag = undo_edges = fflag = nullptr;
     pairs = nullptr; scan_scratch = nullptr; dev_misc = nullptr; dcnt = nullptr; hcnt = nullptr; h_scalars = nullptr;
-    bvh.release();
-    bvh_carried = false;
-    bvh_leaves = 0;
-    bvh_boxes_valid = false;
+    tree.release();
+    tree_carried = false;
     cap_pts = cap_tris = cap_edges = cap_undo = cap_pairs = 0;
 }
 
@@ -1379,7 +1339,7 @@ int Stage2::ensure(long long n, long long m)
     cap_tris = ct;
     cap_edges = ce;
     cap_undo = cu;
-    if (bvh.ensure(ct) != cudaSuccess) {
+    if (tree.ensure(ct) != cudaSuccess) {
         release();
         return PAMO_ERR_OOM;
     }
@@ -1407,36 +1367,38 @@ int Stage2::ensure_pairs(long long n)
         if (_e != cudaSuccess) return map_cuda_error(_e); \
     } while (0)
 
-// dirty_edges / n_dirty: when the boxes were up to date before this round's
-// changes, the edges whose one-rings changed since (incremental refit);
-// otherwise null (full refit).
-static cudaError_t isect_pass(Stage2 &S, int m, cudaStream_t s, const int *dirty_edges = nullptr,
-                              const int *n_dirty = nullptr)
+// Selects the faces that query: the one-rings of the listed edges.
+static cudaError_t mark_active(Stage2 &S, int m, const int *list, const int *n_list, cudaStream_t s)
+{
+    cudaError_t e = cudaMemsetAsync(S.active, 0, (size_t)m, s);
+    if (e != cudaSuccess) return e;
+    launch(k_mark_active, grid_for(3LL * m), kThreads, 0, s, list, n_list, (const int2 *)S.edges,
+           (const int *)S.first_near, (const int *)S.near_tris, S.active);
+    return cudaGetLastError();
+}
+
+// Flags every face of an intersecting pair that has a selected face.  The first
+// pass of a round selects the one-rings of all the collapses that the undo check
+// considers, a later pass only those of the edges the previous check undid: every
+// pair that intersected had a face of such a ring, so all of its one-ring was
+// selected again, and a pair of two faces outside them is as it was, apart.  (The
+// rings of an independent set's collapses are disjoint, so undoing one moves no
+// other face; after coincident-endpoint collapses, which may chain, every pass
+// selects what the first one did.)
+static cudaError_t isect_pass(Stage2 &S, int m, cudaStream_t s)
 {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(S.isect, 0, (size_t)m, s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(&S.dcnt->n_pairs, 0, 2 * sizeof(int), s)) != cudaSuccess) return e;  // n_pairs, overflow
+    if ((e = cudaMemsetAsync(&S.dcnt->n_pairs, 0, 3 * sizeof(int), s)) != cudaSuccess) return e;  // pairs, overflow, queries
     S.prof.begin(PH_REFIT, s);
-    if (dirty_edges && S.bvh_boxes_valid && S.bvh.leaves_built >= 2) {
-        if ((e = cudaMemsetAsync(S.bvh.scene + 9, 0, sizeof(int), s)) != cudaSuccess) return e;
-        launch(k_mark_dirty, grid_for(3LL * m), kThreads, 0, s, dirty_edges, n_dirty, (const int2 *)S.edges,
-               (const int *)S.first_near, (const int *)S.near_tris, (const int *)S.bvh.leaf_of_face,
-               (const int *)S.bvh.parent, S.bvh.claim, S.bvh.dmask, S.bvh.dlist, S.bvh.scene);
-        if ((e = lbvh_refit_dirty(S.bvh, S.pts, S.tris, S.bvh.leaves_built, s)) != cudaSuccess) return e;
-    } else {
-        if ((e = lbvh_refit(S.bvh, S.pts, S.tris, m, s)) != cudaSuccess) return e;
-    }
-    S.bvh_boxes_valid = true;
+    if ((e = tree_refit(S.tree, S.pts, S.tris, S.active, S.fflag, &S.dcnt->n_query, S.isect, m, s)) != cudaSuccess)
+        return e;
     S.prof.begin(PH_QUERY, s);
-    const bool batch = S.n_slots > 0;
-    if ((e = cudaMemsetAsync(&S.dcnt->n_query, 0, sizeof(int), s)) != cudaSuccess) return e;
-    launch(k_active_list, grid_for(m), kThreads, 0, s, (const int *)S.bvh.vals, (const int *)S.bvh.scene,
-           (const uint8_t *)S.active, (const int4 *)S.tris, S.fflag, S.dcnt,
-           batch ? (const SlotInfo *)S.slots : nullptr, batch ? (const int *)S.vslot : nullptr);
-    launch(k_query, grid_for(m), kThreads, 0, s, (const BvhNode *)S.bvh.nodes, (const int *)S.bvh.vals,
-           (const int *)S.bvh.scene, (const float4 *)S.pts, (const int4 *)S.tris, (const uint8_t *)S.active, m,
-           S.pairs, S.cap_pairs, S.dcnt, batch ? (const int *)S.roots : nullptr,
-           batch ? (const int *)S.vslot : nullptr, (const int *)S.fflag, S.quality ? 4 : 2);
+    if (S.n_slots > 0)
+        launch(k_query<true>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.fflag, S.dcnt,
+               S.pairs, S.cap_pairs, 2, (const int2 *)S.ranges, (const int *)S.vslot);
+    else
+        launch(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.fflag, S.dcnt,
+               S.pairs, S.cap_pairs, S.quality ? 4 : 2, (const int2 *)nullptr, (const int *)nullptr);
     S.prof.begin(PH_PAIRS, s);
     if (S.quality)
         launch(k_pairs<true>, grid_for(S.cap_pairs), kThreads, 0, s, S.pairs, S.dcnt, S.cap_pairs, S.pts, S.tris,
@@ -1503,18 +1465,15 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
         launch(k_vertex_quadric64, grid_for(n), kThreads, 0, s, (const int *)first_near, (const int *)near_tris,
                (const float4 *)pts, (const int4 *)tris, quad64, n);
     }
-    // The hierarchy only needs the round input's faces as leaves: build it, or
-    // keep the previous round's (leaves renumbered by compact(), removed faces
+    // The tree only needs an order of the round input's faces: sort them, or keep
+    // the previous round's order (leaves renumbered by compact(), removed faces
     // as empty leaves) while at least kRebuildFraction of its leaves are faces.
-    // Queries find every overlapping leaf whatever the tree, so the pairs found
+    // Queries find every overlapping leaf whatever the order, so the pairs found
     // do not depend on this choice; the refit before each query sets the boxes.
     prof.begin(PH_LBVH_BUILD, s);
-    if (!(keep_bvh && bvh_carried && m <= bvh_leaves && (double)m >= kRebuildFraction * (double)bvh_leaves)) {
-        S2_TRY(lbvh_build(bvh, pts, tris, m, s));
-        bvh_leaves = m;
-        bvh_boxes_valid = false;
-    }
-    bvh_carried = false;
+    if (!(keep_bvh && tree_carried && m <= tree.leaves && (double)m >= kRebuildFraction * (double)tree.leaves))
+        S2_TRY(tree_build(tree, pts, tris, m, s));
+    tree_carried = false;
 
     const long long EMAX = 3LL * m;
     prof.begin(PH_EDGE_COST, s);
@@ -1522,9 +1481,9 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
                 edge_cost, vmin, tres, edge_s, is_stuck ? 1 : 0, nullptr, nullptr, nullptr,
                 quality ? (const double *)quad64 : nullptr, quality ? epos : nullptr};
     if (quality)
-        launch(k_edge_cost<true>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, bvh.vals, bvh.scene, first_edge);
+        launch(k_edge_cost<true>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, (const int *)tree.vals, tree.leaves, (const int *)first_edge);
     else
-        launch(k_edge_cost<false>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, bvh.vals, bvh.scene, first_edge);
+        launch(k_edge_cost<false>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, (const int *)tree.vals, tree.leaves, (const int *)first_edge);
     CollapseArgs cl{edges, d_n_edges, edge_cost, vmin, first_near, near_tris, opts, otris, pts, tris, occ, eflag,
                     collapse_t, nullptr, nullptr, nullptr, quality ? (const float4 *)epos : nullptr};
     prof.begin(PH_COLLAPSE, s);
@@ -1543,9 +1502,7 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
     launch(k_line_apply, 1, kLineThreads, 0, s, edges, d_n_edges, eflag, first_near, near_tris, pts, tris, occ, collapsed,
            dcnt);
 
-    S2_TRY(cudaMemsetAsync(active, 0, (size_t)m, s));
-    launch(k_mark_active, grid_for(EMAX), kThreads, 0, s, collapsed, dcnt, edges, first_near, near_tris, active);
-    // a full refit: the collapses change too many leaves for the incremental one to pay
+    S2_TRY(mark_active(*this, m, collapsed, &dcnt->n_considered, s));
     S2_TRY(isect_pass(*this, m, s));
     S2_TRY(undo_check(*this, s));
     S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
@@ -1562,7 +1519,6 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
         S2_TRY(cudaStreamSynchronize(s));
         if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
     }
-    if (hcnt->stack_overflow > 0) return PAMO_ERR_CAPACITY;
     if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
     last_stats[0] = hcnt->n_edges;
     last_stats[1] = hcnt->n_main;
@@ -1581,7 +1537,8 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
         if (nvu - first > 0)
             launch(k_rearrange, grid_for(nvu - first), kThreads, 0, s, tmp_undo, pts_map, undo_list, first, nvu - first);
         first += 2 * cnt_undo;
-        S2_TRY(isect_pass(*this, m, s, undo_edges, &dcnt->n_undo));  // only the undone one-rings changed
+        if (hcnt->n_line == 0) S2_TRY(mark_active(*this, m, undo_edges, &dcnt->n_undo, s));  // the undone one-rings
+        S2_TRY(isect_pass(*this, m, s));
         S2_TRY(undo_check(*this, s));
         S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
         S2_TRY(cudaStreamSynchronize(s));
@@ -1590,13 +1547,12 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
             long long need = (long long)hcnt->n_pairs + hcnt->n_pairs / 2 + 1024;
             int rc = ensure_pairs(need);
             if (rc) return rc;
-            S2_TRY(isect_pass(*this, m, s, undo_edges, &dcnt->n_undo));
+            S2_TRY(isect_pass(*this, m, s));  // the same selection: `active` is as marked
             S2_TRY(undo_check(*this, s));
             S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
             S2_TRY(cudaStreamSynchronize(s));
             if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
         }
-        if (hcnt->stack_overflow > 0) return PAMO_ERR_CAPACITY;
     if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
         cnt_undo = hcnt->n_undo;
         nvu += 2 * cnt_undo;
@@ -1613,12 +1569,14 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
     return PAMO_OK;
 }
 
-cudaError_t query_and_test_pairs(const BvhNode *nodes, const int *vals, const int *scene, const float4 *pts,
-                                 const int4 *tris, const uint8_t *active, int m, uint2 *pairs, long long cap_pairs,
-                                 RoundCounters *cnt, uint8_t *isect, cudaStream_t s)
+cudaError_t query_and_test_pairs(PackedTree &tree, const float4 *pts, const int4 *tris, int m, int *qlist,
+                                 uint2 *pairs, long long cap_pairs, RoundCounters *cnt, uint8_t *isect,
+                                 cudaStream_t s)
 {
-    launch(k_query, grid_for(m), kThreads, 0, s, nodes, vals, scene, pts, tris, active, m, pairs, cap_pairs, cnt,
-           (const int *)nullptr, (const int *)nullptr, (const int *)nullptr, 2);
+    cudaError_t e = tree_refit(tree, pts, tris, nullptr, qlist, &cnt->n_query, isect, m, s);
+    if (e != cudaSuccess) return e;
+    launch(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, tree.view(), (const int *)qlist, cnt, pairs,
+           cap_pairs, 2, (const int2 *)nullptr, (const int *)nullptr);
     launch(k_pairs<false>, grid_for(cap_pairs), kThreads, 0, s, pairs, cnt, cap_pairs, pts, tris, isect, 1e-3f);
     return cudaGetLastError();
 }
@@ -1646,15 +1604,13 @@ int Stage2::ensure_quality(long long n_pts, long long n_edges)
 
 int Stage2::self_intersect_all(int n, int m, cudaStream_t s)
 {
-    bvh_carried = false;
-    bvh_leaves = 0;
+    tree_carried = false;
     // faces of opts/otris; every live face queries the hierarchy
     launch(k_round_init, grid_for((n + 1 > m ? n + 1 : m)), kThreads, 0, s, opts, otris, pts, tris, occ, first_near,
                                                                        cursor, vmin, n, m);
     S2_TRY(cudaMemsetAsync(dcnt, 0, sizeof(RoundCounters), s));
     S2_TRY(cudaMemsetAsync(active, 1, (size_t)m, s));
-    S2_TRY(lbvh_build(bvh, pts, tris, m, s));
-    bvh_boxes_valid = false;
+    S2_TRY(tree_build(tree, pts, tris, m, s));
     S2_TRY(isect_pass(*this, m, s));
     S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
     S2_TRY(cudaStreamSynchronize(s));
@@ -1667,7 +1623,6 @@ int Stage2::self_intersect_all(int n, int m, cudaStream_t s)
         S2_TRY(cudaStreamSynchronize(s));
         if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
     }
-    if (hcnt->stack_overflow > 0) return PAMO_ERR_CAPACITY;
     if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
     return PAMO_OK;
 }
@@ -1679,10 +1634,10 @@ int Stage2::compact(int n, int m, cudaStream_t s)
     S2_TRY(exclusive_scan(fflag, uflag, m, nullptr, scan_scratch, nullptr, s, &dcnt->scan_fault));
     launch(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, pts, occ, pts_map, n, tris, fflag, uflag, m, opts, otris,
                                                            dcnt);
-    if (bvh_leaves > 0 && bvh_leaves >= m) {
-        launch(k_remap_leaves, grid_for(bvh_leaves), kThreads, 0, s, bvh.vals, (const int *)bvh.scene,
-               (const int *)fflag, (const int *)uflag, bvh.leaf_of_face);
-        bvh_carried = true;
+    if (tree.leaves > 0 && tree.leaves >= m) {
+        launch(k_remap_leaves, grid_for(tree.leaves), kThreads, 0, s, tree.vals, tree.leaves, (const int *)fflag,
+               (const int *)uflag);
+        tree_carried = true;
     }
     prof.end(s);
     S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
@@ -1705,15 +1660,15 @@ int Stage2::ensure_batch(int K)
     if (cap_pts <= 0 || cap_tris <= 0) return PAMO_ERR_INVALID_ARG;  // ensure() first
     if (slots) cudaFree(slots);
     if (scnt) cudaFree(scnt);
-    if (roots) cudaFree(roots);
+    if (ranges) cudaFree(ranges);
     if (hslots) cudaFreeHost(hslots);
     if (hscnt) cudaFreeHost(hscnt);
-    slots = nullptr; scnt = nullptr; roots = nullptr; hslots = nullptr; hscnt = nullptr;
+    slots = nullptr; scnt = nullptr; ranges = nullptr; hslots = nullptr; hscnt = nullptr;
     cap_slots = 0;
     int c = K > 16 ? K : 16;
     if (cudaMalloc((void **)&slots, (size_t)c * sizeof(SlotInfo)) != cudaSuccess ||
         cudaMalloc((void **)&scnt, (size_t)c * sizeof(SlotCounters)) != cudaSuccess ||
-        cudaMalloc((void **)&roots, (size_t)c * 4) != cudaSuccess ||
+        cudaMalloc((void **)&ranges, (size_t)c * sizeof(int2)) != cudaSuccess ||
         cudaMallocHost((void **)&hslots, (size_t)c * sizeof(SlotInfo)) != cudaSuccess ||
         cudaMallocHost((void **)&hscnt, (size_t)c * sizeof(SlotCounters)) != cudaSuccess)
         return PAMO_ERR_OOM;
@@ -1751,7 +1706,7 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
 {
     if (K <= 0 || K > cap_slots) return PAMO_ERR_INVALID_ARG;
     n_slots = K;
-    bvh_carried = false;
+    tree_carried = false;
     std::vector<int> nvu(K), first(K), cnt_undo(K);
     long long max_n = 0, max_undo_in = 0, max_cap_v = 0;
     for (int r = 0; r < K; ++r) {
@@ -1759,7 +1714,6 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
         nvu[r] = first[r] = h.is_stuck ? h.n_undo_in : 0;
         h.pass_first = h.pass_count = 0;
         h.nvu = 0;
-        h.in_undo = 1;
         max_n = h.n > max_n ? h.n : max_n;
         max_undo_in = h.n_undo_in > max_undo_in ? h.n_undo_in : max_undo_in;
         max_cap_v = h.cap_v > max_cap_v ? h.cap_v : max_cap_v;
@@ -1784,15 +1738,13 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     launch(k_vertex_quadric, grid_for(n), kThreads, 0, s, first_near, near_tris, plane, tris, quad, nxt, n);
     launch(k_b_edge_off, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)first_edge, scnt, K);
     prof.begin(PH_LBVH_BUILD, s);
-    S2_TRY(lbvh_build(bvh, pts, tris, m, s, vslot, K, roots));
-    bvh_boxes_valid = false;
-    bvh_leaves = m;
+    S2_TRY(tree_build(tree, pts, tris, m, s, vslot, K, ranges));
 
     const long long EMAX = 3LL * m;
     prof.begin(PH_EDGE_COST, s);
     CostArgs ca{edges, d_n_edges, pts, tris, first_near, near_tris, nxt, plane, elen4, quad, nullptr,
                 nullptr, vmin, 0.f, 1.f, 0, slots, scnt, vslot, nullptr, nullptr};
-    launch(k_edge_cost<false>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, bvh.vals, bvh.scene, first_edge);
+    launch(k_edge_cost<false>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, (const int *)tree.vals, tree.leaves, (const int *)first_edge);
     CollapseArgs cl{edges, d_n_edges, nullptr, vmin, first_near, near_tris, opts, otris, pts, tris, occ, eflag,
                     0u, slots, scnt, vslot, nullptr};
     prof.begin(PH_COLLAPSE, s);
@@ -1810,12 +1762,11 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     launch(k_b_cand_fill, grid_for(EMAX), kThreads, 0, s, (const int *)collapsed, (const int *)line_list, edges,
            (const int *)vslot, (const RoundCounters *)dcnt, (const SlotCounters *)scnt, cand);
 
-    S2_TRY(cudaMemsetAsync(active, 0, (size_t)m, s));
-    launch(k_mark_active, grid_for(EMAX), kThreads, 0, s, cand, dcnt, edges, first_near, near_tris, active);
-    // the first pass refits the round's new hierarchy; the undo passes refit only
-    // the one-rings of the edges they undid
+    // as in the single-mesh round, each undo pass queries only the one-rings undone
     auto pass = [&](bool undo) -> int {
-        S2_TRY(isect_pass(*this, m, s, undo ? undo_edges : nullptr, undo ? &dcnt->n_undo : nullptr));
+        if (!undo || hcnt->n_line == 0)
+            S2_TRY(mark_active(*this, m, undo ? undo_edges : cand, undo ? &dcnt->n_undo : &dcnt->n_considered, s));
+        S2_TRY(isect_pass(*this, m, s));
         S2_TRY(undo_check_batch(*this, K, s));
         S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
         S2_TRY(cudaMemcpyAsync(hscnt, scnt, (size_t)K * sizeof(SlotCounters), cudaMemcpyDeviceToHost, s));
@@ -1825,14 +1776,13 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
             long long need = (long long)hcnt->n_pairs + hcnt->n_pairs / 2 + 1024;
             int rc = ensure_pairs(need);
             if (rc) return rc;
-            S2_TRY(isect_pass(*this, m, s, undo ? undo_edges : nullptr, undo ? &dcnt->n_undo : nullptr));
+            S2_TRY(isect_pass(*this, m, s));
             S2_TRY(undo_check_batch(*this, K, s));
             S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
             S2_TRY(cudaMemcpyAsync(hscnt, scnt, (size_t)K * sizeof(SlotCounters), cudaMemcpyDeviceToHost, s));
             S2_TRY(cudaStreamSynchronize(s));
             if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
         }
-        if (hcnt->stack_overflow > 0) return PAMO_ERR_CAPACITY;
     if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
         return PAMO_OK;
     };
@@ -1860,7 +1810,6 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
         for (int r = 0; r < K; ++r) {
             hslots[r].pass_first = first[r];
             hslots[r].pass_count = nvu[r] - first[r];
-            hslots[r].in_undo = cnt_undo[r] != 0 ? 1 : 0;
             max_cnt = hslots[r].pass_count > max_cnt ? hslots[r].pass_count : max_cnt;
             first[r] += 2 * cnt_undo[r];
         }

@@ -4,7 +4,7 @@
 #include <vector>
 
 #include "common.cuh"
-#include "lbvh.cuh"
+#include "ptree.cuh"
 
 namespace pamo {
 
@@ -17,13 +17,12 @@ struct RoundCounters {
     int n_undo;          // undo edges found by the last check
     int n_pairs;         // candidate pairs found by the last query
     int pair_overflow;   // pairs dropped for lack of buffer space
-    int stack_overflow;  // traversals that ran out of stack
+    int n_query;         // faces in this pass's query list (reset with the two above)
     int n_pts_next;      // compaction result
     int n_tris_next;
     int n_edges;
-    int n_query;         // faces in this pass's query list
     int scan_fault;      // a prefix scan's wait ran out (see scan.cuh)
-    int pad[3];
+    int pad[4];
 };
 
 // ---------------------------------------------------------------------------
@@ -39,8 +38,8 @@ struct RoundCounters {
 // invalid-vertex table) lives in a region of the mesh's own (`SlotInfo`
 // pointers, indexed by mesh-local numbers), the parameters (scale, threshold,
 // stuck mode) are per mesh, the undo check's collapsed-list window is per mesh,
-// and the hierarchy keeps each mesh in its own subtree (the mesh's rank is the
-// top of the sort key), which each query starts from.
+// and the hierarchy keeps each mesh's leaves in one run (the mesh's rank is the
+// top of the sort key), which each query stays in.
 struct SlotInfo {        // uploaded by the host before each round, indexed by rank
     int vert_off, n;     // packed vertex range of the mesh
     int face_off, m;     // packed face range
@@ -51,7 +50,6 @@ struct SlotInfo {        // uploaded by the host before each round, indexed by r
     float tres;          // threshold
     int pass_first, pass_count;  // undo pass: rearrangement window of the undo list
     int nvu;             // undo-list length at the end of the round
-    int in_undo;         // the mesh's undo loop still runs: its faces are queried this pass
     const float *scale;  // device scalar: the mesh's scale (max bbox extent)
     uint32_t *edge_cost; // [3 m0 + 1] edge costs (stale between rounds)
     int *pts_map;        // [n0 + 1] the previous round's vertex map
@@ -78,11 +76,11 @@ struct SlotCounters {    // written on the device during a round, read by the ho
 // the round's synchronisation points).
 enum Phase {
     PH_SETUP = 0,   // round init, face pass A, CSR/edge scans, face pass B, quadrics
-    PH_LBVH_BUILD,  // Morton codes, radix sort, hierarchy
+    PH_LBVH_BUILD,  // Morton codes, radix sort
     PH_EDGE_COST,   // k_edge_cost
     PH_COLLAPSE,    // k_collapse + collapsed-list compaction
     PH_CLEANUP,     // degenerate faces, coincident-endpoint collapses
-    PH_REFIT,       // leaf boxes + bottom-up refit
+    PH_REFIT,       // boxes of every level, query list
     PH_QUERY,       // hierarchy traversal -> candidate pairs
     PH_PAIRS,       // triangle-pair tests
     PH_UNDO,        // undo candidates, restore, list rearrangement
@@ -157,12 +155,10 @@ struct Stage2 {
     RoundCounters *dcnt = nullptr;
     RoundCounters *hcnt = nullptr;  // pinned
     float *h_scalars = nullptr;     // pinned: [0..2] offset, [3] scale
-    Lbvh bvh;
-    // The hierarchy of the previous round, its leaves renumbered by compact():
+    PackedTree tree;
+    // The order of the previous round, its leaves renumbered by compact():
     // reused (refit only) while enough of its leaves are still faces.
-    bool bvh_carried = false;
-    long long bvh_leaves = 0;  // faces the hierarchy was built over
-    bool bvh_boxes_valid = false;  // every box matches the geometry of the last refit
+    bool tree_carried = false;
 
     // batch mode (see SlotInfo); unused by the single-mesh rounds
     int n_slots = 0, cap_slots = 0;
@@ -171,7 +167,7 @@ struct Stage2 {
     SlotCounters *scnt = nullptr;    // device [cap_slots]
     SlotCounters *hscnt = nullptr;   // pinned host copy
     int *vslot = nullptr;            // device [cap_pts + 1]: rank of each packed vertex
-    int *roots = nullptr;            // device [cap_slots]: subtree of each rank in the hierarchy
+    int2 *ranges = nullptr;          // device [cap_slots]: each rank's run of leaves in the hierarchy
     int *line_list = nullptr;        // device [cap_edges + 1]
     int *cand = nullptr;             // device [cap_edges + 1]: per-mesh undo-candidate windows
     int *gmap = nullptr;             // device [cap_pts + 1]: packed vertex map
@@ -225,10 +221,10 @@ struct Stage2 {
 
 int stage2_shuffle_faces(int4 *tris, int m, cudaStream_t s);  // reference init permutation
 
-// Hierarchy query of the faces flagged in `active` and the pair tests, on
-// caller-provided buffers (cnt->n_pairs / pair_overflow must be zero).
-cudaError_t query_and_test_pairs(const BvhNode *nodes, const int *vals, const int *scene, const float4 *pts,
-                                 const int4 *tris, const uint8_t *active, int m, uint2 *pairs, long long cap_pairs,
-                                 RoundCounters *cnt, uint8_t *isect, cudaStream_t s);
+// Refit, query of every live face and the pair tests, on caller-provided buffers
+// (cnt zero; qlist holds m entries).
+cudaError_t query_and_test_pairs(PackedTree &tree, const float4 *pts, const int4 *tris, int m, int *qlist,
+                                 uint2 *pairs, long long cap_pairs, RoundCounters *cnt, uint8_t *isect,
+                                 cudaStream_t s);
 
 }  // namespace pamo
