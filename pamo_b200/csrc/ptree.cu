@@ -55,7 +55,8 @@ __device__ __forceinline__ Box union8(Box b)
 // the query list, mean over the rounds of meshes of 5k / 200k / 2M faces, against
 // 27 / 44 / 84 us for the bottom-up refit of the binary hierarchy (22 / 39 / 74
 // in its kernel) and a launch for the list.
-__global__ void __launch_bounds__(kTreeTile) k_tree_refit(TreeView T, const float4 *__restrict__ pts,
+__global__ void __launch_bounds__(kTreeTile) k_tree_refit(const __grid_constant__ TreeView T,
+                                                          const float4 *__restrict__ pts,
                                                           const int4 *__restrict__ tris,
                                                           const uint8_t *__restrict__ sel, int *qlist, int *n_query,
                                                           uint8_t *flags, int m, int *ticket)

@@ -465,6 +465,223 @@ __global__ void __launch_bounds__(kThreads) k_edge_cost(CostArgs A, const int *o
     }
 }
 
+// The cost of an edge, by a group of eight lanes: lane gl takes every eighth face
+// of u's one-ring, then of v's, so an edge's dozen faces are two steps instead of
+// a chain of twelve.  What the reference adds up face by face is added in that
+// order: each lane leaves its face's terms in `terms` (the group's eight entries
+// in shared memory; a term that is not counted is 0, which changes no
+// non-negative sum) and every lane adds the eight entries one after another.
+// All 32 lanes of a warp call this together (has: the group holds an edge), and
+// a group's results are the same in all of its lanes.  Returns true when the
+// reference writes a new cost for the edge.  QUALITY: quality mode (FP64 quadric
+// terms and the chosen collapse position in epos); compiled separately so the
+// reference's path carries none of it.
+template <bool QUALITY>
+__device__ __forceinline__ bool edge_cost_group(const CostArgs &A, bool has, int u, int v, bool inv_u, bool inv_v,
+                                                float tres, float edge_s, int is_stuck, uint32_t &out, int e,
+                                                float4 *terms)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const int gl = threadIdx.x & 7, shift = threadIdx.x & 24;
+    bool written = false, live = has;
+    out = 0xFFFFFFFFu;
+    V3 v0 = {0.f, 0.f, 0.f}, v1 = v0;
+    int ua = 0, ub = 0, va = 0, vb = 0;
+    if (has) {
+        v0 = v3(A.pts[u]);
+        v1 = v3(A.pts[v]);
+        if constexpr (QUALITY) {  // an edge whose cost is not rewritten collapses to its midpoint
+            const V3 m0 = vmid(v0, v1);
+            if (gl == 0) A.epos[e] = make_float4(m0.x, m0.y, m0.z, 0.f);
+        }
+        if (inv_u && inv_v) {
+            written = true;
+            live = false;
+        } else if (is_stuck) {
+            live = false;
+        } else {
+            ua = A.first_near[u];
+            ub = A.first_near[u + 1];
+            va = A.first_near[v];
+            vb = A.first_near[v + 1];
+        }
+    }
+    // the link condition: pairs of equal next vertices, exactly two wanted
+    int dup = 0;
+    for (int a0 = ua; __any_sync(kAll, live && a0 < ub); a0 += 8) {
+        const int a = a0 + gl;
+        const bool ha = live && a < ub;
+        const int iu = ha ? A.nxt[a] : 0;
+        for (int b0 = va; __any_sync(kAll, live && a0 < ub && b0 < vb); b0 += 8) {
+            const int b = b0 + gl;
+            const int iv = live && b < vb ? A.nxt[b] : 0;
+            const int n = live ? vb - b0 : 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int x = __shfl_sync(kAll, iv, j, 8);
+                dup += ha && j < n && x == iu;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) dup += __shfl_xor_sync(kAll, dup, o);
+    if (live && dup != 2) {
+        written = dup > 2;
+        live = false;
+    }
+    // the collapse position: the midpoint (the reference), or in quality mode
+    // the FP64 quadric's minimiser
+    V3 mid = vmid(v0, v1);
+    if constexpr (QUALITY) {
+        if (live) {
+            mid = qem_position(A.quad64 + 10 * (size_t)u, A.quad64 + 10 * (size_t)v, v0, v1);
+            if (gl == 0) A.epos[e] = make_float4(mid.x, mid.y, mid.z, 0.f);
+        }
+    }
+    float elen = 0.0f, Qa = 0.0f;
+    int nedge = 0, ntri = 0;
+    bool flip = false;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+        const int w = pass ? v : u, other = pass ? u : v;
+        const int lo = pass ? va : ua, hi = pass ? vb : ub;
+        for (int a0 = lo; __any_sync(kAll, live && a0 < hi); a0 += 8) {
+            const int a = a0 + gl;
+            float4 term = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live && a < hi) {
+                const int f = A.near_tris[a];
+                const int4 t = A.tris[f];
+                const float4 l = A.elen[f];
+                if (t.x > t.y) { term.x = l.x; nedge++; }
+                if (t.y > t.z) { term.y = l.y; nedge++; }
+                if (t.z > t.x) { term.z = l.z; nedge++; }
+                if (!face_has(t, other)) {
+                    const V3 o0 = v3(A.pts[t.x]), o1 = v3(A.pts[t.y]), o2 = v3(A.pts[t.z]);
+                    const V3 n0 = t.x == w ? mid : o0;
+                    const V3 n1 = t.y == w ? mid : o1;
+                    const V3 n2 = t.z == w ? mid : o2;
+                    // the unchanged face's unit normal is the face plane's (same expression)
+                    const V3 on = v3(A.plane[f]);
+                    const V3 c = vcross(vsub(n1, n0), vsub(n2, n0));
+                    flip = flip || normal_flips(on, c);
+                    term.w = skinny_term(n0, n1, n2);
+                    ntri++;
+                }
+            }
+            terms[gl] = term;
+            __syncwarp();
+            if (live && a0 < hi) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float4 x = terms[j];
+                    elen += x.x;
+                    elen += x.y;
+                    elen += x.z;
+                    Qa += x.w;
+                }
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        nedge += __shfl_xor_sync(kAll, nedge, o);
+        ntri += __shfl_xor_sync(kAll, ntri, o);
+    }
+    const bool any_flip = (__ballot_sync(kAll, flip) >> shift & 255u) != 0;
+    if (!live) return written;
+    if (any_flip) return true;
+    elen = elen / (float)nedge / edge_s * tres;
+    elen = elen + vnorm(vsub(v0, v1)) / edge_s * tres;
+    Qa = 5.0f * Qa;
+    if constexpr (QUALITY) {  // the quadric error in FP64 at the chosen position
+        const double *qu = A.quad64 + 10 * (size_t)u, *qv = A.quad64 + 10 * (size_t)v;
+        double q[10];
+        for (int k = 0; k < 10; ++k) q[k] = qu[k] + qv[k];
+        const double x = mid.x, y = mid.y, z = mid.z;
+        const double qe = x * (q[0] * x + q[1] * y + q[2] * z + q[3]) + y * (q[1] * x + q[4] * y + q[5] * z + q[6]) +
+                          z * (q[2] * x + q[5] * y + q[7] * z + q[8]) + (q[3] * x + q[6] * y + q[8] * z + q[9]);
+        const float cost = (float)(qe / ((double)edge_s * (double)edge_s));
+        out = quantise_cost(cost + elen + Qa / (float)ntri * tres);
+        return true;
+    }
+    float4 a0 = A.quad[3 * u], a1 = A.quad[3 * u + 1], a2 = A.quad[3 * u + 2];
+    float4 b0 = A.quad[3 * v], b1 = A.quad[3 * v + 1], b2 = A.quad[3 * v + 2];
+    float m00 = a0.x + b0.x, m01 = a0.y + b0.y, m02 = a0.z + b0.z, m03 = a0.w + b0.w;
+    float m11 = a1.x + b1.x, m12 = a1.y + b1.y, m13 = a1.z + b1.z, m22 = a1.w + b1.w;
+    float m23 = a2.x + b2.x, m33 = a2.y + b2.y;
+    float x = mid.x, y = mid.y, z = mid.z, w = 1.0f;
+    float r0 = m00 * x + m01 * y + m02 * z + m03 * w;
+    float r1 = m01 * x + m11 * y + m12 * z + m13 * w;
+    float r2 = m02 * x + m12 * y + m22 * z + m23 * w;
+    float r3 = m03 * x + m13 * y + m23 * z + m33 * w;
+    float qe = r0 * x + r1 * y + r2 * z + r3 * w;
+    float cost = qe / (edge_s * edge_s);
+    out = quantise_cost(cost + elen + Qa / (float)ntri * tres);
+    return true;
+}
+
+// The edge-cost pass by groups, in leaf order too: a warp takes kGroupLeaves
+// consecutive leaves, lists their faces' edges in shared memory (each face owns
+// its 0-3 descending edges) and its four groups take the list in turn, so
+// neighbouring groups gather neighbouring vertices.  Costs are indexed by edge,
+// so the order of work does not change them.
+constexpr int kGroupLeaves = 8;  // few, so that a small mesh has a warp for every dozen edges
+
+template <bool QUALITY>
+__global__ void __launch_bounds__(kThreads, 4) k_edge_cost_group(CostArgs A, const int *order, int L, const int *first_edge)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ int s_list[kThreads / 32][3 * kGroupLeaves];
+    __shared__ float4 s_terms[kThreads];
+    const int lane = threadIdx.x & 31;
+    int *list = s_list[threadIdx.x >> 5];
+    float4 *terms = s_terms + (threadIdx.x & ~7);
+    const long long step = (long long)gridDim.x * (kThreads / 32) * kGroupLeaves;
+    for (long long base = (((long long)blockIdx.x * kThreads + threadIdx.x) >> 5) * kGroupLeaves; base < L; base += step) {
+        const long long p = base + lane;
+        const int f = lane < kGroupLeaves && p < L ? order[p] : -1;  // -1: past the end, or removed since the sort
+        const int fe = f >= 0 ? first_edge[f] : 0;
+        const int c = f >= 0 ? first_edge[f + 1] - fe : 0;
+        const int inc = warp_incl_scan(c), total = __shfl_sync(kAll, inc, 31);
+        for (int j = 0; j < c; ++j) list[inc - c + j] = fe + j;
+        __syncwarp();
+        for (int q0 = 0; q0 < total; q0 += 4) {
+            const int q = q0 + (lane >> 3);
+            const bool has = q < total;
+            const int e = has ? list[q] : 0;
+            const int2 ed = has ? A.edges[e] : make_int2(0, 0);
+            // a batch has its mesh's own parameters, invalid table and stale costs (mesh-local numbers)
+            bool inv_u = false, inv_v = false;
+            float tres = A.tres, edge_s = A.edge_s;
+            int stuck = A.is_stuck;
+            uint32_t *stale = A.edge_cost + e;
+            if (has && A.slots) {
+                const int r = A.vslot[ed.x];
+                const SlotInfo &S = A.slots[r];
+                stale = S.edge_cost + (e - A.scnt[r].edge_off);
+                inv_u = S.invalid[ed.x - S.vert_off];
+                inv_v = S.invalid[ed.y - S.vert_off];
+                tres = S.tres;
+                edge_s = *S.scale;
+                stuck = S.is_stuck;
+            } else if (has) {
+                inv_u = A.invalid[ed.x];
+                inv_v = A.invalid[ed.y];
+            }
+            uint32_t c;
+            const bool written = edge_cost_group<QUALITY>(A, has, ed.x, ed.y, inv_u, inv_v, tres, edge_s, stuck, c, e,
+                                                          terms);
+            if (has && (lane & 7) < 2) {
+                if (!written) c = *stale;  // the reference keeps the previous round's value
+                else if ((lane & 7) == 0) *stale = c;
+                atomicMin(&A.vmin[(lane & 7) ? ed.y : ed.x], ((unsigned long long)c << 32) | (unsigned)e);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 __device__ __forceinline__ bool is_skinny(V3 p, V3 q, V3 r)
 {
     V3 pq = vsub(q, p), pr = vsub(r, p), qr = vsub(r, q);
@@ -742,12 +959,18 @@ __device__ __forceinline__ int shared_indices(int4 a, int4 b)
 constexpr int kQueryThreads = 256;
 
 template <bool BATCH>
-__global__ void __launch_bounds__(kQueryThreads) k_query(TreeView T, const int *__restrict__ qlist,
+__global__ void __launch_bounds__(kQueryThreads) k_query(const __grid_constant__ TreeView T,
+                                                         const int *__restrict__ qlist,
                                                          RoundCounters *cnt, uint2 *pairs, long long cap_pairs,
                                                          int skip_shared, const int2 *__restrict__ ranges,
                                                          const int *__restrict__ vslot)
 {
     __shared__ uint2 s_pairs[kQueryThreads / 32][64];
+    __shared__ int s_off[kTreeMaxLevels];  // indexed by a lane's own level
+#pragma unroll
+    for (int l = 0; l < kTreeMaxLevels; ++l)
+        if (threadIdx.x == l) s_off[l] = T.off[l];
+    __syncthreads();
     uint2 *buf = s_pairs[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
     const unsigned below = (1u << lane) - 1u;
@@ -779,7 +1002,7 @@ __global__ void __launch_bounds__(kQueryThreads) k_query(TreeView T, const int *
             int other = 0;
             if (wk.run) {
                 const int node = 8 * wk.g + gl;
-                const size_t b = 2 * ((size_t)T.off[wk.lvl] + node);
+                const size_t b = 2 * ((size_t)s_off[wk.lvl] + node);
                 const float4 lo = T.boxes[b], hi = T.boxes[b + 1];
                 const bool leaf = wk.lvl == 0 && node < T.L;
                 const int4 r = leaf ? T.leaf[node] : make_int4(-1, -1, -1, kLeafDead);
@@ -1410,6 +1633,22 @@ static cudaError_t isect_pass(Stage2 &S, int m, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// A thread per edge follows a chain of a dozen faces (~33 us a pass at least,
+// however few the edges); a group of eight lanes halves that chain's time several
+// times over but spends ~1.3 times the instructions, as a ring of six leaves two
+// lanes idle.  The pass over a mesh of a few thousand faces takes 23 us by groups
+// and 44 by threads, that over 2M faces 1.3 times as long by groups; the two meet
+// near 100,000 faces (50,000 in quality mode, whose FP64 terms groups repeat).
+template <bool QUALITY>
+static void launch_edge_cost(const CostArgs &A, const int *order, int m, int L, const int *first_edge, cudaStream_t s)
+{
+    if (m <= (QUALITY ? 50000 : 100000))
+        launch(k_edge_cost_group<QUALITY>, grid_for(L, kThreads / 32 * kGroupLeaves), kThreads, 0, s, A, order, L,
+               first_edge);
+    else
+        launch(k_edge_cost<QUALITY>, grid_for(L, kChunkFaces), kThreads, 0, s, A, order, L, first_edge);
+}
+
 static cudaError_t undo_check(Stage2 &S, cudaStream_t s)
 {
     S.prof.begin(PH_UNDO, s);
@@ -1481,9 +1720,9 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
                 edge_cost, vmin, tres, edge_s, is_stuck ? 1 : 0, nullptr, nullptr, nullptr,
                 quality ? (const double *)quad64 : nullptr, quality ? epos : nullptr};
     if (quality)
-        launch(k_edge_cost<true>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, (const int *)tree.vals, tree.leaves, (const int *)first_edge);
+        launch_edge_cost<true>(ca, tree.vals, m, tree.leaves, first_edge, s);
     else
-        launch(k_edge_cost<false>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, (const int *)tree.vals, tree.leaves, (const int *)first_edge);
+        launch_edge_cost<false>(ca, tree.vals, m, tree.leaves, first_edge, s);
     CollapseArgs cl{edges, d_n_edges, edge_cost, vmin, first_near, near_tris, opts, otris, pts, tris, occ, eflag,
                     collapse_t, nullptr, nullptr, nullptr, quality ? (const float4 *)epos : nullptr};
     prof.begin(PH_COLLAPSE, s);
@@ -1744,7 +1983,7 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     prof.begin(PH_EDGE_COST, s);
     CostArgs ca{edges, d_n_edges, pts, tris, first_near, near_tris, nxt, plane, elen4, quad, nullptr,
                 nullptr, vmin, 0.f, 1.f, 0, slots, scnt, vslot, nullptr, nullptr};
-    launch(k_edge_cost<false>, grid_for(m, kChunkFaces), kThreads, 0, s, ca, (const int *)tree.vals, tree.leaves, (const int *)first_edge);
+    launch_edge_cost<false>(ca, tree.vals, m, tree.leaves, first_edge, s);
     CollapseArgs cl{edges, d_n_edges, nullptr, vmin, first_near, near_tris, opts, otris, pts, tris, occ, eflag,
                     0u, slots, scnt, vslot, nullptr};
     prof.begin(PH_COLLAPSE, s);
