@@ -2,99 +2,71 @@
 
 namespace pamo {
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int *__restrict__ in, long long n_max,
-                                                              const int *d_n, int *__restrict__ tile_sums)
+namespace {
+
+struct ScanPair {
+    ScanJob j[2];
+};
+
+__device__ __forceinline__ int scan_value(const ScanJob &J, long long i)
 {
-    long long n = d_n ? (long long)*d_n : n_max;
-    long long base = (long long)blockIdx.x * kScanTile;
-    int sum = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        long long i = base + (long long)k * kScanThreads + threadIdx.x;
-        if (i < n) sum += in[i];
-    }
-    int r = block_reduce_sum<kScanThreads>(sum);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = r;
+    return J.faces ? (J.faces[i].x >= 0) : J.in[i];
 }
 
-// One block: exclusive scan of the tile sums in place, in chunks of 1024.
-__global__ void __launch_bounds__(1024) k_scan_tile_sums(int *tile_sums, long long n_tiles_max, long long n_max,
-                                                         const int *d_n, int *d_total)
-{
-    long long n = d_n ? (long long)*d_n : n_max;
-    long long n_tiles = (n + kScanTile - 1) / kScanTile;
-    if (n_tiles > n_tiles_max) n_tiles = n_tiles_max;
-    int carry = 0;
-    for (long long c = 0; c < n_tiles; c += 1024) {
-        long long i = c + threadIdx.x;
-        int v = i < n_tiles ? tile_sums[i] : 0;
-        int tot;
-        int ex = block_excl_scan<1024>(v, tot);
-        if (i < n_tiles) tile_sums[i] = ex + carry;
-        carry += tot;
-    }
-    if (threadIdx.x == 0 && d_total) *d_total = carry;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_down(const int *in, int *out, long long n_max, const int *d_n,
-                                                            const int *__restrict__ tile_sums)
-{
-    __shared__ int tile[kScanTile];
-    long long n = d_n ? (long long)*d_n : n_max;
-    long long base = (long long)blockIdx.x * kScanTile;
-    if (base >= n) return;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        long long i = base + (long long)k * kScanThreads + threadIdx.x;
-        tile[k * kScanThreads + threadIdx.x] = i < n ? in[i] : 0;
-    }
-    __syncthreads();
-    int local[kScanItems];
-    int s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        local[k] = s;
-        s += tile[threadIdx.x * kScanItems + k];
-    }
-    int tot;
-    int ex = block_excl_scan<kScanThreads>(s, tot);
-    int off = tile_sums[blockIdx.x] + ex;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) tile[threadIdx.x * kScanItems + k] = local[k] + off;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        long long i = base + (long long)k * kScanThreads + threadIdx.x;
-        if (i < n) out[i] = tile[k * kScanThreads + threadIdx.x];
-    }
-}
-
-// Small inputs: one block, 16 consecutive items per thread.
+// Small inputs: one block per job, 16 consecutive items per thread (four vector
+// loads and stores where the job's arrays lie on 16-byte boundaries).
 constexpr int kSingleThreads = 1024;
 constexpr int kSingleItems = 16;
 
-__global__ void __launch_bounds__(kSingleThreads) k_scan_single(const int *in, int *out, long long n_max,
-                                                                const int *d_n, int *d_total)
+__global__ void __launch_bounds__(kSingleThreads) k_scan_single(const __grid_constant__ ScanPair P)
 {
-    const long long n = d_n ? (long long)*d_n : n_max;
+    const ScanJob &J = P.j[blockIdx.x];
+    const long long n = J.d_n ? (long long)*J.d_n : J.n;
     const long long base = (long long)threadIdx.x * kSingleItems;
+    const bool vec = base + kSingleItems <= n && !J.faces &&
+                     ((reinterpret_cast<unsigned long long>(J.in) | reinterpret_cast<unsigned long long>(J.out)) & 15) == 0;
     int v[kSingleItems];
     int sum = 0;
+    if (vec) {
+        const int4 *in4 = reinterpret_cast<const int4 *>(J.in + base);
 #pragma unroll
-    for (int k = 0; k < kSingleItems; ++k) {
-        long long i = base + k;
-        v[k] = i < n ? in[i] : 0;
-        sum += v[k];
+        for (int k = 0; k < kSingleItems / 4; ++k) {
+            const int4 x = in4[k];
+            v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kSingleItems; ++k) v[k] = base + k < n ? scan_value(J, base + k) : 0;
     }
+#pragma unroll
+    for (int k = 0; k < kSingleItems; ++k) sum += v[k];
     int tot;
     int ex = block_excl_scan<kSingleThreads>(sum, tot);
+    if (J.list) {
+        int at = ex;
 #pragma unroll
-    for (int k = 0; k < kSingleItems; ++k) {
-        long long i = base + k;
-        if (i < n) out[i] = ex;
-        ex += v[k];
+        for (int k = 0; k < kSingleItems; ++k)
+            if (v[k]) J.list[at++] = (int)(base + k);
     }
-    if (threadIdx.x == 0 && d_total) *d_total = tot;
+    if (J.out && vec) {
+        int4 *out4 = reinterpret_cast<int4 *>(J.out + base);
+#pragma unroll
+        for (int k = 0; k < kSingleItems / 4; ++k) {
+            int4 x;
+            x.x = ex; ex += v[4 * k];
+            x.y = ex; ex += v[4 * k + 1];
+            x.z = ex; ex += v[4 * k + 2];
+            x.w = ex; ex += v[4 * k + 3];
+            out4[k] = x;
+        }
+    } else if (J.out) {
+#pragma unroll
+        for (int k = 0; k < kSingleItems; ++k) {
+            if (base + k < n) J.out[base + k] = ex;
+            ex += v[k];
+        }
+    }
+    if (threadIdx.x == 0 && J.d_total) *J.d_total = tot;
 }
 
 // Single pass with decoupled look-back (see scan.cuh).  Header: [0] next tile,
@@ -111,16 +83,19 @@ __device__ __forceinline__ unsigned long long status_word(unsigned epoch, unsign
 
 // spin_limit bounds each wait (polls); absent_tile >= 0 makes that tile never
 // publish (only the wait-timeout test passes one: its waiters must give up).
-__global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const int *in, int *out, long long n_max,
-                                                                const int *d_n, int *scratch, int *d_total,
+__global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const __grid_constant__ ScanPair P, int blocks0,
                                                                 int *fault, unsigned epoch, long long spin_limit,
                                                                 long long absent_tile)
 {
     __shared__ int tile[kScanTile];
     __shared__ long long s_t;
     __shared__ int s_prefix;
+    const int which = (int)blockIdx.x >= blocks0 ? 1 : 0;
+    const ScanJob &J = P.j[which];
+    int *scratch = J.scratch;
+    const int job_blocks = which ? (int)gridDim.x - blocks0 : blocks0;
     volatile unsigned long long *status = reinterpret_cast<volatile unsigned long long *>(scratch + kScanHeader);
-    const long long n = d_n ? (long long)*d_n : n_max;
+    const long long n = J.d_n ? (long long)*J.d_n : J.n;
     const long long n_tiles = (n + kScanTile - 1) / kScanTile;
     if (threadIdx.x == 0) s_t = atomicAdd(&scratch[0], 1);
     __syncthreads();
@@ -130,7 +105,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const int *in, i
 #pragma unroll
         for (int k = 0; k < kScanItems; ++k) {
             long long i = base + (long long)k * kScanThreads + threadIdx.x;
-            tile[k * kScanThreads + threadIdx.x] = i < n ? in[i] : 0;
+            tile[k * kScanThreads + threadIdx.x] = i < n ? scan_value(J, i) : 0;
         }
         __syncthreads();
         int local[kScanItems];
@@ -188,26 +163,34 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const int *in, i
                 }
                 if (t != absent_tile) status[t] = status_word(epoch, kFlagPrefix, prefix + agg);
                 s_prefix = prefix;
-                if (t == n_tiles - 1 && d_total) *d_total = prefix + agg;
+                if (t == n_tiles - 1 && J.d_total) *J.d_total = prefix + agg;
             }
         }
         __syncthreads();
         const int off = s_prefix + ex;
+        if (J.list) {
 #pragma unroll
-        for (int k = 0; k < kScanItems; ++k) tile[threadIdx.x * kScanItems + k] = local[k] + off;
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            long long i = base + (long long)k * kScanThreads + threadIdx.x;
-            if (i < n) out[i] = tile[k * kScanThreads + threadIdx.x];
+            for (int k = 0; k < kScanItems; ++k)
+                if (tile[threadIdx.x * kScanItems + k])
+                    J.list[off + local[k]] = (int)(base + threadIdx.x * kScanItems + k);
         }
-    } else if (n_tiles == 0 && t == 0 && threadIdx.x == 0 && d_total) {
-        *d_total = 0;
+        if (J.out) {
+#pragma unroll
+            for (int k = 0; k < kScanItems; ++k) tile[threadIdx.x * kScanItems + k] = local[k] + off;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kScanItems; ++k) {
+                long long i = base + (long long)k * kScanThreads + threadIdx.x;
+                if (i < n) J.out[i] = tile[k * kScanThreads + threadIdx.x];
+            }
+        }
+    } else if (n_tiles == 0 && t == 0 && threadIdx.x == 0 && J.d_total) {
+        *J.d_total = 0;
     }
     // the last block to finish leaves the header at zero for the next scan
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(&scratch[1], 1) == (int)gridDim.x - 1) {
+        if (atomicAdd(&scratch[1], 1) == job_blocks - 1) {
             scratch[0] = 0;
             scratch[1] = 0;
         }
@@ -216,29 +199,55 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const int *in, i
 
 constexpr long long kScanSpinLimit = 1LL << 22;  // ~0.1 s of polls: far beyond any real wait
 
+cudaError_t scan_pair(const ScanPair &P, int n_jobs, cudaStream_t s, int *fault, long long spin_limit,
+                      long long absent_tile)
+{
+    static std::atomic<unsigned> epochs{0};
+    bool single = true;
+    long long tiles[2] = {0, 0};
+    for (int k = 0; k < n_jobs; ++k) {
+        tiles[k] = (P.j[k].n + kScanTile - 1) / kScanTile;
+        single = single && P.j[k].n <= (long long)kSingleThreads * kSingleItems;
+    }
+    if (single) {
+        launch(k_scan_single, n_jobs, kSingleThreads, 0, s, P);
+        return cudaGetLastError();
+    }
+    const unsigned epoch = (epochs.fetch_add(1, std::memory_order_relaxed) + 1) & 0x3FFFFFFFu;
+    launch(k_scan_lookback, (unsigned)(tiles[0] + tiles[1]), kScanThreads, 0, s, P, (int)tiles[0], fault, epoch,
+           spin_limit, absent_tile);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t scan_job(const ScanJob &job, cudaStream_t s, int *fault)
+{
+    if (job.n <= 0) return job.d_total ? cudaMemsetAsync(job.d_total, 0, sizeof(int), s) : cudaSuccess;
+    return scan_pair(ScanPair{{job, ScanJob{}}}, 1, s, fault, kScanSpinLimit, -1);
+}
+
+cudaError_t scan_jobs(const ScanJob &a, const ScanJob &b, cudaStream_t s, int *fault)
+{
+    if (a.n <= 0 || b.n <= 0) {
+        const cudaError_t e = scan_job(a, s, fault);
+        return e != cudaSuccess ? e : scan_job(b, s, fault);
+    }
+    return scan_pair(ScanPair{{a, b}}, 2, s, fault, kScanSpinLimit, -1);
+}
+
 cudaError_t exclusive_scan(const int *in, int *out, long long n_max, const int *d_n, int *scratch, int *d_total,
                            cudaStream_t s, int *fault)
 {
-    return exclusive_scan_waits(in, out, n_max, d_n, scratch, d_total, s, fault, kScanSpinLimit, -1);
+    return scan_job(ScanJob{in, nullptr, out, nullptr, n_max, d_n, scratch, d_total}, s, fault);
 }
 
 cudaError_t exclusive_scan_waits(const int *in, int *out, long long n_max, const int *d_n, int *scratch, int *d_total,
                                  cudaStream_t s, int *fault, long long spin_limit, long long absent_tile)
 {
-    static std::atomic<unsigned> epochs{0};
-    if (n_max <= 0) {
-        if (d_total) return cudaMemsetAsync(d_total, 0, sizeof(int), s);
-        return cudaSuccess;
-    }
-    if (n_max <= (long long)kSingleThreads * kSingleItems) {
-        launch(k_scan_single, 1, kSingleThreads, 0, s, in, out, n_max, d_n, d_total);
-        return cudaGetLastError();
-    }
-    const long long tiles = (n_max + kScanTile - 1) / kScanTile;
-    const unsigned epoch = (epochs.fetch_add(1, std::memory_order_relaxed) + 1) & 0x3FFFFFFFu;
-    launch(k_scan_lookback, (unsigned)tiles, kScanThreads, 0, s, in, out, n_max, d_n, scratch, d_total, fault, epoch,
-           spin_limit, absent_tile);
-    return cudaGetLastError();
+    if (n_max <= 0) return d_total ? cudaMemsetAsync(d_total, 0, sizeof(int), s) : cudaSuccess;
+    const ScanJob job{in, nullptr, out, nullptr, n_max, d_n, scratch, d_total};
+    return scan_pair(ScanPair{{job, ScanJob{}}}, 1, s, fault, spin_limit, absent_tile);
 }
 
 }  // namespace pamo

@@ -56,29 +56,6 @@ __device__ __forceinline__ int block_excl_scan(int v, int &total)
     return excl;
 }
 
-template <int BLOCK>
-__device__ __forceinline__ int block_reduce_sum(int v)
-{
-    __shared__ int ws[BLOCK / 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) ws[wid] = v;
-    __syncthreads();
-    int r = 0;
-    if (wid == 0) {
-        r = lane < BLOCK / 32 ? ws[lane] : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-    }
-    __syncthreads();
-    return r;  // valid in thread 0
-}
-
-__global__ void k_scan_reduce(const int *__restrict__ in, long long n_max, const int *d_n, int *__restrict__ tile_sums);
-__global__ void k_scan_tile_sums(int *tile_sums, long long n_tiles_max, long long n_max, const int *d_n, int *d_total);
-__global__ void k_scan_down(const int *in, int *out, long long n_max, const int *d_n, const int *__restrict__ tile_sums);
-
 // Scratch needed by exclusive_scan for up to n_max items (ints): a header of
 // kScanHeader ints, then one 64-bit status word per tile.
 constexpr int kScanHeader = 8;
@@ -96,6 +73,25 @@ inline cudaError_t scan_scratch_init(int *scratch, long long ints, cudaStream_t 
 // copy in any case).
 cudaError_t exclusive_scan(const int *in, int *out, long long n_max, const int *d_n, int *scratch, int *d_total,
                            cudaStream_t s, int *fault = nullptr);
+
+// A scan of n (d_n: *d_n, at most n) values: in[i], or whether faces[i] is a
+// face (x >= 0) if `faces` is given.  out (may be null, may equal in) takes the
+// exclusive prefix, list (may be null) the indices of the non-zero values of 0/1
+// in order, d_total (may be null) the sum.  Each job has a scratch of its own.
+struct ScanJob {
+    const int *in;
+    const int4 *faces;
+    int *out;
+    int *list;
+    long long n;
+    const int *d_n;
+    int *scratch;
+    int *d_total;
+};
+cudaError_t scan_job(const ScanJob &job, cudaStream_t s, int *fault = nullptr);
+// Two independent scans in one launch (a round's scans are short: on a small mesh
+// each costs its launch and latency, ~5 us, and little else).
+cudaError_t scan_jobs(const ScanJob &a, const ScanJob &b, cudaStream_t s, int *fault = nullptr);
 
 // exclusive_scan with each look-back wait bounded by `spin_limit` polls, and
 // tile `absent_tile` (>= 0) never publishing -- for the test that makes the

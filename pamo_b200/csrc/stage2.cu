@@ -54,11 +54,14 @@ __device__ __forceinline__ uint32_t quantise_cost(float c)
     return (uint32_t)(tclamp(c, 0.0f, kCostRange) / kCostRange * 4294967296.0f);
 }
 
+// The round's working copies and everything that starts it at zero.
 __global__ void k_round_init(const float4 *__restrict__ opts, const int4 *__restrict__ otris, float4 *pts,
-                             int4 *tris, int *occ, int *deg, int *cursor, unsigned long long *vmin, int n, int m)
+                             int4 *tris, int *occ, int *deg, int *cursor, unsigned long long *vmin, int *first_edge,
+                             uint8_t *active, RoundCounters *cnt, int n, int m)
 {
-    long long N = (long long)(n + 1 > m ? n + 1 : m);
-    PAMO_GRID_STRIDE(i, N)
+    constexpr int kCounters = (int)(sizeof(RoundCounters) / sizeof(int));
+    const long long N = n + 1 > kCounters ? n + 1 : kCounters;
+    PAMO_GRID_STRIDE(i, N > m + 1 ? N : m + 1)
     {
         if (i < n) {
             pts[i] = opts[i];
@@ -70,7 +73,13 @@ __global__ void k_round_init(const float4 *__restrict__ opts, const int4 *__rest
             occ[n] = 0;
             deg[n] = 0;
         }
-        if (i < m) tris[i] = otris[i];
+        if (i < m) {
+            tris[i] = otris[i];
+            active[i] = 0;
+        } else if (i == m) {
+            first_edge[m] = 0;
+        }
+        if (i < kCounters) reinterpret_cast<int *>(cnt)[i] = 0;
     }
 }
 
@@ -713,147 +722,148 @@ struct CollapseArgs {
     const float4 *epos;  // quality mode: the position the edge cost chose (null: the midpoint)
 };
 
-__device__ __forceinline__ bool faces_min_ok(const CollapseArgs &A, int lo, int hi, unsigned long long key)
-{
-    for (int a = lo; a < hi; ++a) {
-        int4 t = A.otris[A.near_tris[a]];  // round input: never written during this pass
-        if (A.vmin[t.x] < key || A.vmin[t.y] < key || A.vmin[t.z] < key) return false;
-    }
-    return true;
-}
-
-// The independent set: one thread per edge tests the threshold and the key
-// (most edges fail at once) and flags the winners; the collapse list is their
-// scan.  The winners' collapses then run one thread per winner
-// (k_collapse_apply), so no warp carries idle lanes through a collapse.
-// Winners have disjoint one-rings, and the tests read only the round input
-// (otris) and the key minima, so splitting the two changes nothing.
+// The independent set: every lane tests its edge's threshold and key (most edges
+// fail at once); the one-rings of those that pass are then checked by groups of
+// eight lanes, four edges at a time -- a chain of a dozen faces, three dependent
+// loads each, when one thread walks it.  The flags' scan is the collapse list, and
+// the winners' collapses run over that list (k_collapse_apply), so no warp carries
+// idle lanes through a collapse.  Winners have disjoint one-rings, and the tests
+// read only the round input (otris) and the key minima, so splitting the two
+// changes nothing.
 __global__ void __launch_bounds__(kThreads) k_collapse(CollapseArgs A)
 {
+    constexpr unsigned kAll = 0xffffffffu;
     const int E = *A.n_edges;
-    PAMO_GRID_STRIDE(ee, E)
-    {
-        const int e = (int)ee;
-        int win = 0;
-        uint32_t c, collapse_t;
-        if (!A.slots) {
-            c = A.edge_cost[e];
-            collapse_t = A.collapse_t;
-        } else {
-            const int r = A.vslot[A.edges[e].x];
-            c = A.slots[r].edge_cost[e - A.scnt[r].edge_off];
-            collapse_t = A.slots[r].collapse_t;
+    const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < E; base += step) {
+        const int e = (int)(base + lane);
+        int2 ed = make_int2(0, 0);
+        unsigned long long key = 0;
+        bool pass = false;
+        if (base + lane < E) {
+            uint32_t c, collapse_t;
+            if (!A.slots) {
+                c = A.edge_cost[e];
+                collapse_t = A.collapse_t;
+            } else {
+                const int r = A.vslot[A.edges[e].x];
+                c = A.slots[r].edge_cost[e - A.scnt[r].edge_off];
+                collapse_t = A.slots[r].collapse_t;
+            }
+            if (c <= collapse_t) {
+                ed = A.edges[e];
+                key = ((unsigned long long)c << 32) | (unsigned)e;
+                pass = A.vmin[ed.x] == key && A.vmin[ed.y] == key;
+            }
         }
-        if (c <= collapse_t) {
-            const int2 ed = A.edges[e];
-            const int u = ed.x, v = ed.y;
-            const unsigned long long key = ((unsigned long long)c << 32) | (unsigned)e;
-            if (A.vmin[u] == key && A.vmin[v] == key)
-                win = faces_min_ok(A, A.first_near[u], A.first_near[u + 1], key) &&
-                      faces_min_ok(A, A.first_near[v], A.first_near[v + 1], key);
+        unsigned won = 0;
+        for (unsigned todo = __ballot_sync(kAll, pass); todo;) {
+            int src = 0;
+            bool has = false;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {  // the next four edges, one per group
+                if (shift == 8 * k && todo) {
+                    src = __ffs(todo) - 1;
+                    has = true;
+                }
+                todo &= todo - 1;
+            }
+            const int u = __shfl_sync(kAll, ed.x, src), v = __shfl_sync(kAll, ed.y, src);
+            const unsigned long long k0 = __shfl_sync(kAll, key, src);
+            int ua = 0, du = 0, va = 0, d = 0;  // the two rings as one list
+            if (has) {
+                ua = A.first_near[u];
+                du = A.first_near[u + 1] - ua;
+                va = A.first_near[v] - du;
+                d = A.first_near[v + 1] - va;
+            }
+            bool less = false;
+            for (int i0 = 0; __any_sync(kAll, i0 < d); i0 += 8) {
+                const int i = i0 + gl;
+                if (i < d) {
+                    const int4 t = A.otris[A.near_tris[(i < du ? ua : va) + i]];  // round input: never written here
+                    less = less || A.vmin[t.x] < k0 || A.vmin[t.y] < k0 || A.vmin[t.z] < k0;
+                }
+            }
+            const unsigned lost = __ballot_sync(kAll, less);
+            const unsigned mine = has && ((lost >> shift) & 255u) == 0 ? 1u << src : 0u;
+            won |= __reduce_or_sync(kAll, mine);
         }
-        A.eflag[e] = win;
+        if (base + lane < E) A.eflag[e] = (int)(won >> lane & 1u);
     }
 }
 
-// Collapse of each winner (list[0, *n_list)): u moves to the midpoint (the
-// quality mode's chosen position), v goes, faces holding both die and v's faces
-// take u; if a surviving one-ring face is skinny the one-rings are restored from
-// the round input, and the edge stays in the collapsed list.
+// Collapse of each winner (list[0, *n_list)), by a group of eight lanes: u moves to
+// the midpoint (the quality mode's chosen position), v goes, faces holding both
+// die and v's faces take u; if a surviving one-ring face would be skinny nothing
+// is changed, and the edge stays in the collapsed list.  The one-ring's faces are
+// marked as those that query the tree.
 template <bool QUALITY>
-__global__ void __launch_bounds__(kThreads) k_collapse_apply(CollapseArgs A, const int *list, const int *n_list)
+__global__ void __launch_bounds__(kThreads) k_collapse_apply(CollapseArgs A, const int *list, const int *n_list,
+                                                             uint8_t *active)
 {
+    constexpr unsigned kAll = 0xffffffffu;
     const int N = *n_list;
-    PAMO_GRID_STRIDE(k, N)
-    {
-        const int e = list[k];
-        const int2 ed = A.edges[e];
-        const int u = ed.x, v = ed.y;
-        const int ua = A.first_near[u], ub = A.first_near[u + 1];
-        const int va = A.first_near[v], vb = A.first_near[v + 1];
-        V3 mid;
-        if constexpr (QUALITY) mid = v3(A.epos[e]);  // the position the edge cost chose
-        else mid = vmid(v3(A.opts[u]), v3(A.opts[v]));
-        A.pts[u] = make_float4(mid.x, mid.y, mid.z, 0.f);
-        A.pts[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-        A.occ[v] = 0;
-        for (int a = ua; a < ub; ++a) {
-            const int f = A.near_tris[a];
-            const int4 t = A.tris[f];
-            if (face_has(t, v)) A.tris[f] = make_int4(-1, -1, -1, 0);
+    const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
+    const long long warps = (long long)gridDim.x * (kThreads / 32);
+    for (long long w = ((long long)blockIdx.x * kThreads + threadIdx.x) >> 5; w * 4 < N; w += warps) {
+        const long long k = w * 4 + (lane >> 3);
+        int u = 0, v = 0, ua = 0, du = 0, va = 0, d = 0;
+        V3 mid = {0.f, 0.f, 0.f};
+        if (k < N) {
+            const int e = list[k];
+            const int2 ed = A.edges[e];
+            u = ed.x;
+            v = ed.y;
+            ua = A.first_near[u];
+            du = A.first_near[u + 1] - ua;
+            va = A.first_near[v] - du;
+            d = A.first_near[v + 1] - va;
+            if constexpr (QUALITY) mid = v3(A.epos[e]);  // the position the edge cost chose
+            else mid = vmid(v3(A.opts[u]), v3(A.opts[v]));
         }
-        for (int a = va; a < vb; ++a) {
-            const int f = A.near_tris[a];
-            int4 t = A.tris[f];
-            if (face_has(t, u)) t = make_int4(-1, -1, -1, 0);
+        // the one-rings after the collapse, from the round input (no other winner touches them)
+        auto moved = [&](int i, int &f) {
+            f = A.near_tris[(i < du ? ua : va) + i];
+            int4 t = A.otris[f];
+            if (face_has(t, i < du ? v : u)) t = make_int4(-1, -1, -1, 0);
             else if (t.x == v) t.x = u;
             else if (t.y == v) t.y = u;
             else if (t.z == v) t.z = u;
-            A.tris[f] = t;
+            return t;
+        };
+        bool skinny = false;
+        for (int i0 = 0; __any_sync(kAll, i0 < d); i0 += 8) {
+            if (i0 + gl >= d) continue;
+            int f;
+            const int4 t = moved(i0 + gl, f);
+            active[f] = 1;
+            if (t.x == -1) continue;
+            auto at = [&](int x) { return x == u ? mid : v3(A.opts[x]); };
+            skinny = skinny || is_skinny(at(t.x), at(t.y), at(t.z));
         }
-        bool sk = false;
-        for (int pass = 0; pass < 2 && !sk; ++pass) {
-            const int lo = pass ? va : ua, hi = pass ? vb : ub;
-            for (int a = lo; a < hi; ++a) {
-                const int4 t = A.tris[A.near_tris[a]];
-                if (t.x == -1) continue;
-                if (is_skinny(v3(A.pts[t.x]), v3(A.pts[t.y]), v3(A.pts[t.z]))) {
-                    sk = true;
-                    break;
-                }
-            }
+        if (((__ballot_sync(kAll, skinny) >> shift) & 255u) != 0 || d == 0) d = 0;  // rolled back
+        for (int i0 = 0; __any_sync(kAll, i0 < d); i0 += 8) {
+            if (i0 + gl >= d) continue;
+            int f;
+            const int4 t = moved(i0 + gl, f);
+            if (t.x == -1 || i0 + gl >= du) A.tris[f] = t;
         }
-        if (sk) {  // roll back; the edge stays in the collapsed list
-            A.occ[v] = 1;
-            A.pts[u] = A.opts[u];
-            A.pts[v] = A.opts[v];
-            for (int a = ua; a < ub; ++a) A.tris[A.near_tris[a]] = A.otris[A.near_tris[a]];
-            for (int a = va; a < vb; ++a) A.tris[A.near_tris[a]] = A.otris[A.near_tris[a]];
+        if (d > 0 && gl == 0) {
+            A.pts[u] = make_float4(mid.x, mid.y, mid.z, 0.f);
+            A.pts[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+            A.occ[v] = 0;
         }
     }
 }
 
-// list[pos[i]] = i for flagged i (pos = exclusive scan of the flags)
-__global__ void k_scatter_flagged(const int *__restrict__ flags, const int *__restrict__ pos, const int *d_n,
-                                  int *list, int list_offset)
-{
-    const int N = *d_n;
-    PAMO_GRID_STRIDE(i, N)
-    {
-        if (flags[i]) list[list_offset + pos[i]] = (int)i;
-    }
-}
-
-__global__ void k_remove_invalid_faces(int4 *tris, int m)
-{
-    PAMO_GRID_STRIDE(f, m)
-    {
-        int4 t = tris[f];
-        if (face_dead(t)) continue;
-        if (t.x == t.y || t.y == t.z || t.z == t.x) tris[f] = make_int4(-1, -1, -1, 0);
-    }
-}
-
-__global__ void k_line_flags(const int2 *edges, const int *n_edges, const float4 *pts, int *eflag, int *count)
-{
-    const int E = *n_edges;
-    int local = 0;
-    PAMO_GRID_STRIDE(e, E)
-    {
-        int2 ed = edges[e];
-        float4 p = pts[ed.x], q = pts[ed.y];
-        int f = (p.x == q.x && p.y == q.y && p.z == q.z);
-        eflag[e] = f;
-        local += f;
-    }
-    if (local) atomicAdd(count, local);
-}
-
-// Coincident-endpoint collapses: positions were read (k_line_flags) before any
-// write; the writes are applied in edge order by one thread.  Flagged edges are
-// rare (exactly equal coordinates), so one block of kLineThreads finds them
-// chunk by chunk and its thread 0 applies each chunk's edges in order.
-constexpr int kLineThreads = 1024;
+// Coincident-endpoint collapses: positions are read (k_cleanup) before any write;
+// the writes are applied in edge order by one thread.  Flagged edges are rare
+// (exactly equal coordinates), so one block of kLineThreads finds them chunk by
+// chunk and its thread 0 applies each chunk's edges in order.  Other blocks of the
+// same launch may have written the faces and flags: these loads bypass the L1.
+constexpr int kLineThreads = 256;
 constexpr int kLinePerThread = 8;
 
 __device__ __forceinline__ void line_collapse(int u, int v, const int *first_near, const int *near_tris, float4 *pts,
@@ -863,11 +873,11 @@ __device__ __forceinline__ void line_collapse(int u, int v, const int *first_nea
     occ[v] = 0;
     for (int a = first_near[u]; a < first_near[u + 1]; ++a) {
         int f = near_tris[a];
-        if (face_has(tris[f], v)) tris[f] = make_int4(-1, -1, -1, 0);
+        if (face_has(__ldcg(&tris[f]), v)) tris[f] = make_int4(-1, -1, -1, 0);
     }
     for (int a = first_near[v]; a < first_near[v + 1]; ++a) {
         int f = near_tris[a];
-        int4 t = tris[f];
+        int4 t = __ldcg(&tris[f]);
         if (face_has(t, u)) t = make_int4(-1, -1, -1, 0);
         else if (t.x == v) t.x = u;
         else if (t.y == v) t.y = u;
@@ -887,7 +897,7 @@ __device__ __forceinline__ void for_flagged_in_order(const int *eflag, int E, On
 #pragma unroll
         for (int k = 0; k < kLinePerThread; ++k) {
             long long e = base + (long long)threadIdx.x * kLinePerThread + k;
-            if (e < E && eflag[e]) local[c++] = (int)e;
+            if (e < E && __ldcg(&eflag[e])) local[c++] = (int)e;
         }
         int total;
         int off = block_excl_scan<kLineThreads>(c, total);
@@ -899,37 +909,62 @@ __device__ __forceinline__ void for_flagged_in_order(const int *eflag, int E, On
     }
 }
 
-__global__ void __launch_bounds__(kLineThreads) k_line_apply(const int2 *edges, const int *n_edges, const int *eflag,
-                                                             const int *first_near, const int *near_tris, float4 *pts,
-                                                             int4 *tris, int *occ, int *collapsed, RoundCounters *cnt)
+// After the collapses: faces with a repeated index go, and edges with coincident
+// end points are flagged and counted; the last block to finish (a ticket, no
+// waiting) applies those, and sets the prefix of the collapsed list that the
+// reference's undo check looks at.  The faces of the considered coincident edges
+// join those that query the tree.  A batch applies them in k_b_line_apply.
+template <bool BATCH>
+__global__ void __launch_bounds__(kLineThreads) k_cleanup(int4 *tris, int m, const int2 *edges, const int *n_edges,
+                                                          float4 *pts, int *eflag, const int *first_near,
+                                                          const int *near_tris, int *occ, int *collapsed,
+                                                          uint8_t *active, RoundCounters *cnt)
 {
     const int E = *n_edges;
-    const int nm = cnt->n_main;
+    __shared__ bool s_last;
+    int local = 0;
+    PAMO_GRID_STRIDE(i, m > E ? m : E)
+    {
+        if (i < m) {
+            const int4 t = tris[i];
+            if (!face_dead(t) && (t.x == t.y || t.y == t.z || t.z == t.x)) tris[i] = make_int4(-1, -1, -1, 0);
+        }
+        if (i < E) {
+            const int2 ed = edges[i];
+            const float4 p = pts[ed.x], q = pts[ed.y];
+            const int f = p.x == q.x && p.y == q.y && p.z == q.z;
+            eflag[i] = f;
+            local += f;
+        }
+    }
+    if (local) atomicAdd(&cnt->n_line, local);
+    if (BATCH) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&cnt->ticket, 1) == (int)gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    const int nm = cnt->n_main, lines = *(volatile int *)&cnt->n_line;
+    const int window = ((nm + 511) / 512) * 512;  // grid of the reference's undo-candidate launch
     int k = 0;
-    if (cnt->n_line > 0)
+    if (lines > 0)
         for_flagged_in_order(eflag, E, [&](int e) {
-            int u = edges[e].x, v = edges[e].y;
+            const int u = edges[e].x, v = edges[e].y;
+            if (nm + k < window)
+                for (int side = 0; side < 2; ++side) {
+                    const int w = side ? v : u;
+                    for (int a = first_near[w]; a < first_near[w + 1]; ++a) active[near_tris[a]] = 1;
+                }
             collapsed[nm + k++] = e;
             line_collapse(u, v, first_near, near_tris, pts, tris, occ);
         });
     if (threadIdx.x != 0) return;
     cnt->n_line = k;
     cnt->n_total = nm + k;
-    int window = ((nm + 511) / 512) * 512;  // grid of the reference's undo-candidate launch
     cnt->n_considered = cnt->n_total < window ? cnt->n_total : window;
-}
-
-// The faces of the one-rings of the listed edges: those that query the tree.
-__global__ void k_mark_active(const int *list, const int *n_list, const int2 *edges, const int *first_near,
-                              const int *near_tris, uint8_t *active)
-{
-    const int N = *n_list;
-    PAMO_GRID_STRIDE(p, N)
-    {
-        int2 ed = edges[list[p]];
-        for (int a = first_near[ed.x]; a < first_near[ed.x + 1]; ++a) active[near_tris[a]] = 1;
-        for (int a = first_near[ed.y]; a < first_near[ed.y + 1]; ++a) active[near_tris[a]] = 1;
-    }
 }
 
 __device__ __forceinline__ bool box_overlap(float4 alo, float4 ahi, float4 qlo, float4 qhi)
@@ -1047,7 +1082,7 @@ __device__ __forceinline__ void load_face(const float4 *pts, int4 t, float out[3
 }
 
 template <bool EXACT>
-__global__ void __launch_bounds__(kThreads) k_pairs(const uint2 *pairs, const RoundCounters *cnt,
+__global__ void __launch_bounds__(kThreads) k_pairs(const uint2 *pairs, RoundCounters *cnt,
                                                     long long cap_pairs, const float4 *__restrict__ pts,
                                                     const int4 *__restrict__ tris, uint8_t *isect, float eps)
 {
@@ -1067,12 +1102,10 @@ __global__ void __launch_bounds__(kThreads) k_pairs(const uint2 *pairs, const Ro
                 Q[c] = {b.x, b.y, b.z};
             }
             const bool da = exact::tri_degenerate(P, ia), db = exact::tri_degenerate(Q, ib);
-            if (da) isect[pr.x] = 1;
-            if (db) isect[pr.y] = 1;
-            if (!da && !db && exact::faces_intersect(P, ia, Q, ib)) {
-                isect[pr.x] = 1;
-                isect[pr.y] = 1;
-            }
+            const bool hit = !da && !db && exact::faces_intersect(P, ia, Q, ib);
+            if (da || hit) isect[pr.x] = 1;
+            if (db || hit) isect[pr.y] = 1;
+            if (da || db || hit) cnt->n_hit = 1;
             continue;
         }
         float A[3][3], B[3][3];
@@ -1082,14 +1115,19 @@ __global__ void __launch_bounds__(kThreads) k_pairs(const uint2 *pairs, const Ro
         if (pair_flag_directed(A, ia, B, ib, eps) || pair_flag_directed(B, ib, A, ia, eps)) {
             isect[pr.x] = 1;
             isect[pr.y] = 1;
+            cnt->n_hit = 1;
         }
     }
 }
 
-__global__ void k_undo_flags(const int *collapsed, const RoundCounters *cnt, const int2 *edges,
+// The considered edges with an intersecting face in their one-rings: flags and
+// count.  The host scans the flags into the undo list only if there are any.
+__global__ void k_undo_flags(const int *collapsed, RoundCounters *cnt, const int2 *edges,
                              const int *first_near, const int *near_tris, const uint8_t *isect, int *uflag)
 {
+    if (!cnt->n_hit) return;  // no pair intersects (n_undo is 0)
     const int N = cnt->n_considered;
+    int local = 0;
     PAMO_GRID_STRIDE(p, N)
     {
         int2 ed = edges[collapsed[p]];
@@ -1097,44 +1135,54 @@ __global__ void k_undo_flags(const int *collapsed, const RoundCounters *cnt, con
         for (int a = first_near[ed.x]; a < first_near[ed.x + 1] && !hit; ++a) hit = isect[near_tris[a]];
         for (int a = first_near[ed.y]; a < first_near[ed.y + 1] && !hit; ++a) hit = isect[near_tris[a]];
         uflag[p] = hit;
+        local += hit;
     }
+    if (local) atomicAdd(&cnt->n_undo, local);
 }
 
-__global__ void k_undo_scatter(const int *uflag, const int *upos, const RoundCounters *cnt, const int *collapsed,
-                               const int2 *edges, int *undo_edges, int *tmp_undo)
-{
-    const int N = cnt->n_considered;
-    PAMO_GRID_STRIDE(p, N)
-    {
-        if (!uflag[p]) continue;
-        int k = upos[p];
-        int e = collapsed[p];
-        int2 ed = edges[e];
-        undo_edges[k] = e;
-        tmp_undo[2 * k] = ed.x;
-        tmp_undo[2 * k + 1] = ed.y;
-    }
-}
-
-__global__ void k_undo_apply(const int *undo_edges, const RoundCounters *cnt, const int2 *edges,
+// The listed collapses taken back (undo_idx: positions in the collapsed list): the
+// one-rings restored from the round input and, if `active` is given, selected for
+// the next query (they alone: cleared before).  The undo list gets the end
+// points' vertices from `first` on, through the previous round's map: pts_map at
+// this point (cusimp_free.cu:869-878 runs before :1042-1045).  Thread 0 resets the
+// pass's counters.
+__global__ void k_undo_apply(const int *undo_idx, int N, const int *collapsed, const int2 *edges,
                              const int *first_near, const int *near_tris, const float4 *opts, const int4 *otris,
-                             float4 *pts, int4 *tris, int *occ)
+                             float4 *pts, int4 *tris, int *occ, uint8_t *active, const int *pts_map, int *undo_list,
+                             int first, const SlotInfo *slots, const SlotCounters *scnt, const int *vslot,
+                             RoundCounters *cnt)
 {
-    const int N = cnt->n_undo;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        cnt->n_pairs = cnt->pair_overflow = cnt->n_query = cnt->n_hit = cnt->n_undo = 0;
     PAMO_GRID_STRIDE(k, N)
     {
-        int2 ed = edges[undo_edges[k]];
-        int u = ed.x, v = ed.y;
+        const int2 ed = edges[collapsed[undo_idx[k]]];
+        const int u = ed.x, v = ed.y;
         occ[v] = 1;
         pts[u] = opts[u];
         pts[v] = opts[v];
-        for (int a = first_near[u]; a < first_near[u + 1]; ++a) tris[near_tris[a]] = otris[near_tris[a]];
-        for (int a = first_near[v]; a < first_near[v + 1]; ++a) tris[near_tris[a]] = otris[near_tris[a]];
+        for (int side = 0; side < 2; ++side) {
+            const int w = side ? v : u;
+            for (int a = first_near[w]; a < first_near[w + 1]; ++a) {
+                const int f = near_tris[a];
+                tris[f] = otris[f];
+                if (active) active[f] = 1;
+            }
+        }
+        if (!slots) {
+            undo_list[first + 2 * k] = pts_map[u];
+            undo_list[first + 2 * k + 1] = pts_map[v];
+        } else {  // the mesh's own list and map, in its own numbers
+            const int r = vslot[u];
+            const SlotInfo &S = slots[r];
+            const int j = S.pass_first + 2 * ((int)k - scnt[r].undo_off);
+            S.undo_list[j] = S.pts_map[u - S.vert_off];
+            S.undo_list[j + 1] = S.pts_map[v - S.vert_off];
+        }
     }
 }
 
-// undo_list[first + i] = pts_map[tmp_undo[i]]: the map in pts_map at this point is
-// the previous round's (cusimp_free.cu:869-878 runs before :1042-1045).
+// undo_list[first + i] = pts_map[tmp_undo[i]], through the previous round's map
 __global__ void k_rearrange(const int *tmp_undo, const int *pts_map, int *undo_list, int first, int count)
 {
     PAMO_GRID_STRIDE(i, count) undo_list[first + i] = pts_map[tmp_undo[i]];
@@ -1145,36 +1193,28 @@ __global__ void k_mark_invalid(const int *undo_in, int n, uint8_t *table)
     PAMO_GRID_STRIDE(i, n) table[undo_in[i]] = 1;
 }
 
-__global__ void k_face_live_flags(const int4 *tris, int m, int *fflag)
-{
-    PAMO_GRID_STRIDE(f, m) fflag[f] = tris[f].x >= 0;
-}
-
+// Compaction by the scans' positions, and the tree's leaves renumbered: leaf p's
+// face gets its compacted index, or -1 if removed.
 __global__ void k_compact(const float4 *pts, const int *occ, const int *pts_map, int n, const int4 *tris,
-                          const int *fflag, const int *fpos, int m, float4 *opts, int4 *otris, RoundCounters *cnt)
+                          const int *fpos, int m, float4 *opts, int4 *otris, int *vals, int L, RoundCounters *cnt)
 {
     long long N = n > m ? n : m;
+    N = N > L ? N : L;
     PAMO_GRID_STRIDE(i, N)
     {
         if (i < n && occ[i]) opts[pts_map[i]] = pts[i];
-        if (i < m && fflag[i]) {
-            int4 t = tris[i];
-            otris[fpos[i]] = make_int4(pts_map[t.x], pts_map[t.y], pts_map[t.z], 0);
+        if (i < m) {
+            const int4 t = tris[i];
+            if (t.x >= 0) otris[fpos[i]] = make_int4(pts_map[t.x], pts_map[t.y], pts_map[t.z], 0);
+        }
+        if (i < L) {
+            const int f = vals[i];
+            vals[i] = f >= 0 && tris[f].x >= 0 ? fpos[f] : -1;
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         cnt->n_pts_next = pts_map[n];
-        cnt->n_tris_next = fpos[m - 1 >= 0 ? m - 1 : 0] + (m > 0 ? fflag[m - 1] : 0);
-    }
-}
-
-// After compaction: leaf p's face gets its compacted index, or -1 if removed.
-__global__ void k_remap_leaves(int *vals, int L, const int *fflag, const int *fpos)
-{
-    PAMO_GRID_STRIDE(p, L)
-    {
-        const int f = vals[p];
-        vals[p] = (f >= 0 && fflag[f]) ? fpos[f] : -1;
+        cnt->n_tris_next = m > 0 ? fpos[m - 1] + (tris[m - 1].x >= 0) : 0;
     }
 }
 
@@ -1305,7 +1345,8 @@ __global__ void __launch_bounds__(kLineThreads) k_b_line_apply(const int2 *edges
 }
 
 __global__ void k_b_cand_fill(const int *collapsed, const int *line_list, const int2 *edges, const int *vslot,
-                              const RoundCounters *cnt, const SlotCounters *scnt, int *cand)
+                              const RoundCounters *cnt, const SlotCounters *scnt, int *cand,
+                              const int *first_near, const int *near_tris, uint8_t *active)
 {
     const int nm = cnt->n_main, nl = cnt->n_line;
     PAMO_GRID_STRIDE(p, (long long)nm + nl)
@@ -1320,6 +1361,11 @@ __global__ void k_b_cand_fill(const int *collapsed, const int *line_list, const 
             e = line_list[q];
             r = vslot[edges[e].x];
             k = scnt[r].n_main + q - scnt[r].line_off;
+            if (k < scnt[r].n_considered)  // its faces query the tree (the collapses marked theirs)
+                for (int side = 0; side < 2; ++side) {
+                    const int w = side ? edges[e].y : edges[e].x;
+                    for (int a = first_near[w]; a < first_near[w + 1]; ++a) active[near_tris[a]] = 1;
+                }
         }
         if (k < scnt[r].n_considered) cand[scnt[r].cand_off + k] = e;
     }
@@ -1334,34 +1380,6 @@ __global__ void k_b_undo_counts(const int *upos, const RoundCounters *cnt, SlotC
         scnt[r].undo_off = off;
         scnt[r].n_undo = c;
     }
-}
-
-// undo edges (packed) and each mesh's undo vertices (mesh-local numbers)
-__global__ void k_b_undo_scatter(const int *uflag, const int *upos, const RoundCounters *cnt, const int *cand,
-                                 const int2 *edges, const int *vslot, const SlotInfo *slots,
-                                 const SlotCounters *scnt, int *undo_edges)
-{
-    const int N = cnt->n_considered;
-    PAMO_GRID_STRIDE(p, N)
-    {
-        if (!uflag[p]) continue;
-        int k = upos[p];
-        int e = cand[p];
-        int2 ed = edges[e];
-        undo_edges[k] = e;
-        int r = vslot[ed.x];
-        const SlotInfo &S = slots[r];
-        int j = k - scnt[r].undo_off;
-        S.tmp_undo[2 * j] = ed.x - S.vert_off;
-        S.tmp_undo[2 * j + 1] = ed.y - S.vert_off;
-    }
-}
-
-// undo_list[first + j] = pts_map[tmp_undo[j]] per mesh (the previous round's map)
-__global__ void k_b_rearrange(const SlotInfo *slots)
-{
-    const SlotInfo S = slots[blockIdx.y];
-    SLOT_STRIDE(j, S.pass_count) S.undo_list[S.pass_first + j] = S.pts_map[S.tmp_undo[j]];
 }
 
 // each mesh's vertex map in its own numbers, and the copy of its undo list
@@ -1472,7 +1490,7 @@ void Stage2::release()
 {
     void *p[] = {edge_cost, pts_map, undo_list, tmp_undo, invalid_table, opts, pts, otris, tris, occ,
                  first_near, cursor, near_tris, first_edge, edges, plane, elen4, nxt, quad, vmin, eflag, collapsed,
-                 active, isect, uflag, undo_edges, fflag, pairs, scan_scratch, dev_misc, dcnt, quad64, epos};
+                 active, isect, uflag, undo_idx, fpos, qlist, pairs, scan_scratch, scan_scratch2, dev_misc, dcnt, quad64, epos};
     for (void *q : p)
         if (q) cudaFree(q);
     quad64 = nullptr;
@@ -1485,8 +1503,8 @@ void Stage2::release()
     opts = pts = nullptr; otris = tris = nullptr; occ = nullptr;
     first_near = cursor = near_tris = first_edge = nullptr; edges = nullptr; plane = quad = elen4 = nullptr;
     nxt = nullptr;
-    vmin = nullptr; eflag = collapsed = nullptr; active = isect = nullptr; uflag = undo_edges = fflag = nullptr;
-    pairs = nullptr; scan_scratch = nullptr; dev_misc = nullptr; dcnt = nullptr; hcnt = nullptr; h_scalars = nullptr;
+    vmin = nullptr; eflag = collapsed = nullptr; active = isect = nullptr; uflag = undo_idx = fpos = qlist = nullptr;
+    pairs = nullptr; scan_scratch = scan_scratch2 = nullptr; dev_misc = nullptr; dcnt = nullptr; hcnt = nullptr; h_scalars = nullptr;
     tree.release();
     tree_carried = false;
     cap_pts = cap_tris = cap_edges = cap_undo = cap_pairs = 0;
@@ -1537,9 +1555,11 @@ int Stage2::ensure(long long n, long long m)
     ALLOC(active, ct + 1);
     ALLOC(isect, ct + 1);
     ALLOC(uflag, (ce + 1) * 4);
-    ALLOC(undo_edges, (ce + 1) * 4);
-    ALLOC(fflag, (ct + 1) * 4);
+    ALLOC(undo_idx, (ce + 1) * 4);
+    ALLOC(fpos, (ct + 1) * 4);
+    ALLOC(qlist, (ct + 1) * 4);
     ALLOC(scan_scratch, scan_scratch_len * 4);
+    ALLOC(scan_scratch2, scan_scratch_len * 4);
     ALLOC(dev_misc, 256);
     ALLOC(dcnt, sizeof(RoundCounters));
 #undef ALLOC
@@ -1552,6 +1572,7 @@ int Stage2::ensure(long long n, long long m)
         return PAMO_ERR_OOM;
     }
     scan_scratch_init(scan_scratch, scan_scratch_len);
+    scan_scratch_init(scan_scratch2, scan_scratch_len);
     // state the reference reads stale starts at zero
     cudaMemset(edge_cost, 0, (ce + 1) * 4);
     cudaMemset(pts_map, 0, (cp + 1) * 4);
@@ -1590,37 +1611,27 @@ int Stage2::ensure_pairs(long long n)
         if (_e != cudaSuccess) return map_cuda_error(_e); \
     } while (0)
 
-// Selects the faces that query: the one-rings of the listed edges.
-static cudaError_t mark_active(Stage2 &S, int m, const int *list, const int *n_list, cudaStream_t s)
-{
-    cudaError_t e = cudaMemsetAsync(S.active, 0, (size_t)m, s);
-    if (e != cudaSuccess) return e;
-    launch(k_mark_active, grid_for(3LL * m), kThreads, 0, s, list, n_list, (const int2 *)S.edges,
-           (const int *)S.first_near, (const int *)S.near_tris, S.active);
-    return cudaGetLastError();
-}
-
-// Flags every face of an intersecting pair that has a selected face.  The first
+// Flags every face of an intersecting pair that has a selected face, then counts
+// the considered edges with such a face in their one-rings (n_undo).  The first
 // pass of a round selects the one-rings of all the collapses that the undo check
 // considers, a later pass only those of the edges the previous check undid: every
 // pair that intersected had a face of such a ring, so all of its one-ring was
 // selected again, and a pair of two faces outside them is as it was, apart.  (The
 // rings of an independent set's collapses are disjoint, so undoing one moves no
 // other face; after coincident-endpoint collapses, which may chain, every pass
-// selects what the first one did.)
-static cudaError_t isect_pass(Stage2 &S, int m, cudaStream_t s)
+// selects what the first one did.)  The pass's counters are zero before.
+static cudaError_t isect_pass(Stage2 &S, int m, const int *considered, cudaStream_t s)
 {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(&S.dcnt->n_pairs, 0, 3 * sizeof(int), s)) != cudaSuccess) return e;  // pairs, overflow, queries
     S.prof.begin(PH_REFIT, s);
-    if ((e = tree_refit(S.tree, S.pts, S.tris, S.active, S.fflag, &S.dcnt->n_query, S.isect, m, s)) != cudaSuccess)
+    if ((e = tree_refit(S.tree, S.pts, S.tris, S.active, S.qlist, &S.dcnt->n_query, S.isect, m, s)) != cudaSuccess)
         return e;
     S.prof.begin(PH_QUERY, s);
     if (S.n_slots > 0)
-        launch(k_query<true>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.fflag, S.dcnt,
+        launch(k_query<true>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.qlist, S.dcnt,
                S.pairs, S.cap_pairs, 2, (const int2 *)S.ranges, (const int *)S.vslot);
     else
-        launch(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.fflag, S.dcnt,
+        launch(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.qlist, S.dcnt,
                S.pairs, S.cap_pairs, S.quality ? 4 : 2, (const int2 *)nullptr, (const int *)nullptr);
     S.prof.begin(PH_PAIRS, s);
     if (S.quality)
@@ -1629,8 +1640,40 @@ static cudaError_t isect_pass(Stage2 &S, int m, cudaStream_t s)
     else
         launch(k_pairs<false>, grid_for(S.cap_pairs), kThreads, 0, s, S.pairs, S.dcnt, S.cap_pairs, S.pts, S.tris,
                S.isect, 1e-3f);
+    if (considered) {
+        S.prof.begin(PH_UNDO, s);
+        launch(k_undo_flags, grid_for(3LL * m), kThreads, 0, s, considered, S.dcnt, (const int2 *)S.edges,
+               (const int *)S.first_near, (const int *)S.near_tris, (const uint8_t *)S.isect, S.uflag);
+    }
     S.prof.end(s);
     return cudaGetLastError();
+}
+
+// isect_pass and the counters' copy; once more with a larger pair buffer if the
+// candidates did not fit.
+static int checked_pass(Stage2 &S, int m, const int *considered, cudaStream_t s)
+{
+    for (int attempt = 0;; ++attempt) {
+        S2_TRY(isect_pass(S, m, considered, s));
+        S2_TRY(cudaMemcpyAsync(S.hcnt, S.dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
+        S2_TRY(cudaStreamSynchronize(s));
+        S.prof.collect();
+        if (S.hcnt->scan_fault) return PAMO_ERR_DEVICE;
+        if (S.hcnt->pair_overflow == 0) return PAMO_OK;
+        if (attempt > 0) return PAMO_ERR_CAPACITY;
+        const int rc = S.ensure_pairs((long long)S.hcnt->n_pairs + S.hcnt->n_pairs / 2 + 1024);
+        if (rc) return rc;
+        S2_TRY(cudaMemsetAsync(&S.dcnt->n_undo, 0, 5 * sizeof(int), s));  // n_undo to n_hit
+    }
+}
+
+// positions of the flagged entries of the considered list, in its order (pos: also
+// each entry's prefix, which a batch splits by mesh)
+static cudaError_t undo_list_of(Stage2 &S, int *pos, cudaStream_t s)
+{
+    return scan_job(ScanJob{S.uflag, nullptr, pos, S.undo_idx, S.hcnt->n_considered, nullptr, S.scan_scratch,
+                            &S.dcnt->n_undo},
+                    s, &S.dcnt->scan_fault);
 }
 
 // A thread per edge follows a chain of a dozen faces (~33 us a pass at least,
@@ -1649,26 +1692,10 @@ static void launch_edge_cost(const CostArgs &A, const int *order, int m, int L, 
         launch(k_edge_cost<QUALITY>, grid_for(L, kChunkFaces), kThreads, 0, s, A, order, L, first_edge);
 }
 
-static cudaError_t undo_check(Stage2 &S, cudaStream_t s)
-{
-    S.prof.begin(PH_UNDO, s);
-    const long long NC = S.cap_edges;
-    launch(k_undo_flags, grid_for(NC), kThreads, 0, s, S.collapsed, S.dcnt, S.edges, S.first_near, S.near_tris, S.isect,
-                                                   S.uflag);
-    // positions of the flagged entries (in collapsed-list order)
-    cudaError_t e = exclusive_scan(S.uflag, S.eflag, NC, &S.dcnt->n_considered, S.scan_scratch, &S.dcnt->n_undo, s, &S.dcnt->scan_fault);
-    if (e != cudaSuccess) return e;
-    launch(k_undo_scatter, grid_for(NC), kThreads, 0, s, S.uflag, S.eflag, S.dcnt, S.collapsed, S.edges, S.undo_edges,
-                                                     S.tmp_undo);
-    S.prof.end(s);
-    return cudaGetLastError();
-}
-
 int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, const int *d_undo_in, int n_undo_in,
                   int *n_undo_out, cudaStream_t s, bool keep_bvh)
 {
     int nvu = 0, first = 0;
-    S2_TRY(cudaMemsetAsync(dcnt, 0, sizeof(RoundCounters), s));
     if (is_stuck) {
         if (n_undo_in > 0) {
             S2_TRY(cudaMemcpyAsync(tmp_undo, d_undo_in, (size_t)n_undo_in * 4, cudaMemcpyDeviceToDevice, s));
@@ -1689,12 +1716,12 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
     const uint32_t collapse_t = (uint32_t)(unsigned long long)(ct / kCostRange * 4294967296.0f);
 
     prof.begin(PH_SETUP, s);
-    launch(k_round_init, grid_for((n + 1 > m ? n + 1 : m)), kThreads, 0, s, opts, otris, pts, tris, occ, first_near,
-                                                                       cursor, vmin, n, m);
+    launch(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
+           tris, occ, first_near, cursor, vmin, first_edge, active, dcnt, n, m);
     launch(k_face_a, grid_for(m), kThreads, 0, s, pts, tris, m, first_near, first_edge, plane, elen4);
-    if (m > 0) S2_TRY(cudaMemsetAsync(first_edge + m, 0, 4, s));
-    S2_TRY(exclusive_scan(first_near, first_near, (long long)n + 1, nullptr, scan_scratch, nullptr, s, &dcnt->scan_fault));
-    S2_TRY(exclusive_scan(first_edge, first_edge, (long long)m + 1, nullptr, scan_scratch, &dcnt->n_edges, s, &dcnt->scan_fault));
+    S2_TRY(scan_jobs(ScanJob{first_near, nullptr, first_near, nullptr, n + 1LL, nullptr, scan_scratch, nullptr},
+                     ScanJob{first_edge, nullptr, first_edge, nullptr, m + 1LL, nullptr, scan_scratch2, &dcnt->n_edges},
+                     s, &dcnt->scan_fault));
     const int *d_n_edges = &dcnt->n_edges;
     launch(k_face_b, grid_for(m), kThreads, 0, s, tris, m, first_near, cursor, near_tris, first_edge, edges);
     launch(k_vertex_quadric, grid_for(n), kThreads, 0, s, first_near, near_tris, plane, tris, quad, nxt, n);
@@ -1727,38 +1754,19 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
                     collapse_t, nullptr, nullptr, nullptr, quality ? (const float4 *)epos : nullptr};
     prof.begin(PH_COLLAPSE, s);
     launch(k_collapse, grid_for(EMAX), kThreads, 0, s, cl);
-    S2_TRY(exclusive_scan(eflag, uflag, EMAX, d_n_edges, scan_scratch, &dcnt->n_main, s, &dcnt->scan_fault));
-    launch(k_scatter_flagged, grid_for(EMAX), kThreads, 0, s, eflag, uflag, d_n_edges, collapsed, 0);
+    S2_TRY(scan_job(ScanJob{eflag, nullptr, nullptr, collapsed, EMAX, d_n_edges, scan_scratch, &dcnt->n_main}, s,
+                    &dcnt->scan_fault));
     if (quality)
         launch(k_collapse_apply<true>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
-               (const int *)&dcnt->n_main);
+               (const int *)&dcnt->n_main, active);
     else
         launch(k_collapse_apply<false>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
-               (const int *)&dcnt->n_main);
+               (const int *)&dcnt->n_main, active);
     prof.begin(PH_CLEANUP, s);
-    launch(k_remove_invalid_faces, grid_for(m), kThreads, 0, s, tris, m);
-    launch(k_line_flags, grid_for(EMAX), kThreads, 0, s, edges, d_n_edges, pts, eflag, &dcnt->n_line);
-    launch(k_line_apply, 1, kLineThreads, 0, s, edges, d_n_edges, eflag, first_near, near_tris, pts, tris, occ, collapsed,
-           dcnt);
-
-    S2_TRY(mark_active(*this, m, collapsed, &dcnt->n_considered, s));
-    S2_TRY(isect_pass(*this, m, s));
-    S2_TRY(undo_check(*this, s));
-    S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-    S2_TRY(cudaStreamSynchronize(s));
-    prof.collect();
-    if (hcnt->pair_overflow > 0) {
-        // candidate buffer too small: grow and redo the pass
-        long long need = (long long)hcnt->n_pairs + hcnt->n_pairs / 2 + 1024;
-        int rc = ensure_pairs(need);
-        if (rc) return rc;
-        S2_TRY(isect_pass(*this, m, s));
-        S2_TRY(undo_check(*this, s));
-        S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-        S2_TRY(cudaStreamSynchronize(s));
-        if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
-    }
-    if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
+    launch(k_cleanup<false>, grid_for(EMAX), kLineThreads, 0, s, tris, m, (const int2 *)edges, d_n_edges, pts, eflag,
+           (const int *)first_near, (const int *)near_tris, occ, collapsed, active, dcnt);
+    int rc = checked_pass(*this, m, collapsed, s);
+    if (rc) return rc;
     last_stats[0] = hcnt->n_edges;
     last_stats[1] = hcnt->n_main;
     last_stats[2] = hcnt->n_total;
@@ -1771,28 +1779,16 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
     while (cnt_undo != 0) {
         it++;
         prof.begin(PH_UNDO, s);
-        launch(k_undo_apply, grid_for(cnt_undo), kThreads, 0, s, undo_edges, dcnt, edges, first_near, near_tris, opts,
-                                                              otris, pts, tris, occ);
-        if (nvu - first > 0)
-            launch(k_rearrange, grid_for(nvu - first), kThreads, 0, s, tmp_undo, pts_map, undo_list, first, nvu - first);
+        S2_TRY(undo_list_of(*this, nullptr, s));
+        const bool reselect = hcnt->n_line == 0;  // see isect_pass
+        if (reselect) S2_TRY(cudaMemsetAsync(active, 0, (size_t)m, s));
+        launch(k_undo_apply, grid_for(cnt_undo), kThreads, 0, s, (const int *)undo_idx, cnt_undo,
+               (const int *)collapsed, (const int2 *)edges, (const int *)first_near, (const int *)near_tris,
+               (const float4 *)opts, (const int4 *)otris, pts, tris, occ, reselect ? active : nullptr,
+               (const int *)pts_map, undo_list, first, (const SlotInfo *)nullptr, (const SlotCounters *)nullptr,
+               (const int *)nullptr, dcnt);
         first += 2 * cnt_undo;
-        if (hcnt->n_line == 0) S2_TRY(mark_active(*this, m, undo_edges, &dcnt->n_undo, s));  // the undone one-rings
-        S2_TRY(isect_pass(*this, m, s));
-        S2_TRY(undo_check(*this, s));
-        S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-        S2_TRY(cudaStreamSynchronize(s));
-        prof.collect();
-        if (hcnt->pair_overflow > 0) {
-            long long need = (long long)hcnt->n_pairs + hcnt->n_pairs / 2 + 1024;
-            int rc = ensure_pairs(need);
-            if (rc) return rc;
-            S2_TRY(isect_pass(*this, m, s));  // the same selection: `active` is as marked
-            S2_TRY(undo_check(*this, s));
-            S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-            S2_TRY(cudaStreamSynchronize(s));
-            if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
-        }
-    if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
+        if ((rc = checked_pass(*this, m, collapsed, s))) return rc;
         cnt_undo = hcnt->n_undo;
         nvu += 2 * cnt_undo;
         if (nvu > cap_undo) return PAMO_ERR_CAPACITY;
@@ -1800,9 +1796,10 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
     }
     last_stats[3] = it;
     last_stats[4] = nvu;
-    // pts_map = exclusive scan of occ[0..n]
+    // pts_map = exclusive scan of occ[0..n]; the faces' positions for compact()
     prof.begin(PH_COMPACT, s);
-    S2_TRY(exclusive_scan(occ, pts_map, (long long)n + 1, nullptr, scan_scratch, nullptr, s, &dcnt->scan_fault));
+    S2_TRY(scan_jobs(ScanJob{occ, nullptr, pts_map, nullptr, n + 1LL, nullptr, scan_scratch, nullptr},
+                     ScanJob{nullptr, tris, fpos, nullptr, m, nullptr, scan_scratch2, nullptr}, s, &dcnt->scan_fault));
     prof.end(s);
     *n_undo_out = nvu;
     return PAMO_OK;
@@ -1844,40 +1841,22 @@ int Stage2::ensure_quality(long long n_pts, long long n_edges)
 int Stage2::self_intersect_all(int n, int m, cudaStream_t s)
 {
     tree_carried = false;
-    // faces of opts/otris; every live face queries the hierarchy
-    launch(k_round_init, grid_for((n + 1 > m ? n + 1 : m)), kThreads, 0, s, opts, otris, pts, tris, occ, first_near,
-                                                                       cursor, vmin, n, m);
-    S2_TRY(cudaMemsetAsync(dcnt, 0, sizeof(RoundCounters), s));
+    // faces of opts/otris; every live face queries the tree
+    launch(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
+           tris, occ, first_near, cursor, vmin, first_edge, active, dcnt, n, m);
     S2_TRY(cudaMemsetAsync(active, 1, (size_t)m, s));
     S2_TRY(tree_build(tree, pts, tris, m, s));
-    S2_TRY(isect_pass(*this, m, s));
-    S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-    S2_TRY(cudaStreamSynchronize(s));
-    if (hcnt->pair_overflow > 0) {
-        long long need = (long long)hcnt->n_pairs + hcnt->n_pairs / 2 + 1024;
-        int rc = ensure_pairs(need);
-        if (rc) return rc;
-        S2_TRY(isect_pass(*this, m, s));
-        S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-        S2_TRY(cudaStreamSynchronize(s));
-        if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
-    }
-    if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
-    return PAMO_OK;
+    return checked_pass(*this, m, nullptr, s);
 }
 
 int Stage2::compact(int n, int m, cudaStream_t s)
 {
     prof.begin(PH_COMPACT, s);
-    launch(k_face_live_flags, grid_for(m), kThreads, 0, s, tris, m, fflag);
-    S2_TRY(exclusive_scan(fflag, uflag, m, nullptr, scan_scratch, nullptr, s, &dcnt->scan_fault));
-    launch(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, pts, occ, pts_map, n, tris, fflag, uflag, m, opts, otris,
-                                                           dcnt);
-    if (tree.leaves > 0 && tree.leaves >= m) {
-        launch(k_remap_leaves, grid_for(tree.leaves), kThreads, 0, s, tree.vals, tree.leaves, (const int *)fflag,
-               (const int *)uflag);
-        tree_carried = true;
-    }
+    const bool keep = tree.leaves > 0 && tree.leaves >= m;
+    launch(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, (const float4 *)pts, (const int *)occ,
+           (const int *)pts_map, n, (const int4 *)tris, (const int *)fpos, m, opts, otris, tree.vals,
+           keep ? tree.leaves : 0, dcnt);
+    tree_carried = keep;
     prof.end(s);
     S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
     S2_TRY(cudaStreamSynchronize(s));
@@ -1919,21 +1898,6 @@ int Stage2::ensure_batch(int K)
     return PAMO_OK;
 }
 
-static cudaError_t undo_check_batch(Stage2 &S, int K, cudaStream_t s)
-{
-    S.prof.begin(PH_UNDO, s);
-    const long long NC = S.cap_edges;
-    launch(k_undo_flags, grid_for(NC), kThreads, 0, s, S.cand, S.dcnt, S.edges, S.first_near, S.near_tris, S.isect,
-           S.uflag);
-    cudaError_t e = exclusive_scan(S.uflag, S.eflag, NC, &S.dcnt->n_considered, S.scan_scratch, &S.dcnt->n_undo, s, &S.dcnt->scan_fault);
-    if (e != cudaSuccess) return e;
-    launch(k_b_undo_counts, grid_for(K), kThreads, 0, s, S.eflag, S.dcnt, S.scnt, K);
-    launch(k_b_undo_scatter, grid_for(NC), kThreads, 0, s, S.uflag, S.eflag, S.dcnt, S.cand, S.edges, S.vslot,
-           S.slots, S.scnt, S.undo_edges);
-    S.prof.end(s);
-    return cudaGetLastError();
-}
-
 static dim3 slot_grid(int K, long long per_slot_max)
 {
     long long x = (per_slot_max + kThreads - 1) / kThreads;
@@ -1951,13 +1915,12 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     for (int r = 0; r < K; ++r) {
         SlotInfo &h = hslots[r];
         nvu[r] = first[r] = h.is_stuck ? h.n_undo_in : 0;
-        h.pass_first = h.pass_count = 0;
+        h.pass_first = 0;
         h.nvu = 0;
         max_n = h.n > max_n ? h.n : max_n;
         max_undo_in = h.n_undo_in > max_undo_in ? h.n_undo_in : max_undo_in;
         max_cap_v = h.cap_v > max_cap_v ? h.cap_v : max_cap_v;
     }
-    S2_TRY(cudaMemsetAsync(dcnt, 0, sizeof(RoundCounters), s));
     S2_TRY(cudaMemsetAsync(scnt, 0, (size_t)K * sizeof(SlotCounters), s));
     S2_TRY(cudaMemcpyAsync(slots, hslots, (size_t)K * sizeof(SlotInfo), cudaMemcpyHostToDevice, s));
     launch(k_b_pre_copy, slot_grid(K, max_undo_in > max_cap_v ? max_undo_in : max_cap_v), kThreads, 0, s,
@@ -1966,12 +1929,12 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     launch(k_b_vslot, slot_grid(K, max_n), kThreads, 0, s, (const SlotInfo *)slots, vslot);
 
     prof.begin(PH_SETUP, s);
-    launch(k_round_init, grid_for((n + 1 > m ? n + 1 : m)), kThreads, 0, s, opts, otris, pts, tris, occ, first_near,
-           cursor, vmin, n, m);
+    launch(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
+           tris, occ, first_near, cursor, vmin, first_edge, active, dcnt, n, m);
     launch(k_face_a, grid_for(m), kThreads, 0, s, pts, tris, m, first_near, first_edge, plane, elen4);
-    S2_TRY(cudaMemsetAsync(first_edge + m, 0, 4, s));
-    S2_TRY(exclusive_scan(first_near, first_near, (long long)n + 1, nullptr, scan_scratch, nullptr, s, &dcnt->scan_fault));
-    S2_TRY(exclusive_scan(first_edge, first_edge, (long long)m + 1, nullptr, scan_scratch, &dcnt->n_edges, s, &dcnt->scan_fault));
+    S2_TRY(scan_jobs(ScanJob{first_near, nullptr, first_near, nullptr, n + 1LL, nullptr, scan_scratch, nullptr},
+                     ScanJob{first_edge, nullptr, first_edge, nullptr, m + 1LL, nullptr, scan_scratch2, &dcnt->n_edges},
+                     s, &dcnt->scan_fault));
     const int *d_n_edges = &dcnt->n_edges;
     launch(k_face_b, grid_for(m), kThreads, 0, s, tris, m, first_near, cursor, near_tris, first_edge, edges);
     launch(k_vertex_quadric, grid_for(n), kThreads, 0, s, first_near, near_tris, plane, tris, quad, nxt, n);
@@ -1988,44 +1951,32 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
                     0u, slots, scnt, vslot, nullptr};
     prof.begin(PH_COLLAPSE, s);
     launch(k_collapse, grid_for(EMAX), kThreads, 0, s, cl);
-    S2_TRY(exclusive_scan(eflag, uflag, EMAX, d_n_edges, scan_scratch, &dcnt->n_main, s, &dcnt->scan_fault));
-    launch(k_scatter_flagged, grid_for(EMAX), kThreads, 0, s, eflag, uflag, d_n_edges, collapsed, 0);
+    S2_TRY(scan_job(ScanJob{eflag, nullptr, uflag, collapsed, EMAX, d_n_edges, scan_scratch, &dcnt->n_main}, s,
+                    &dcnt->scan_fault));
     launch(k_collapse_apply<false>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
-           (const int *)&dcnt->n_main);
+           (const int *)&dcnt->n_main, active);
     launch(k_b_main, grid_for(K), kThreads, 0, s, (const int *)uflag, (const RoundCounters *)dcnt, scnt, K);
     prof.begin(PH_CLEANUP, s);
-    launch(k_remove_invalid_faces, grid_for(m), kThreads, 0, s, tris, m);
-    launch(k_line_flags, grid_for(EMAX), kThreads, 0, s, edges, d_n_edges, pts, eflag, &dcnt->n_line);
+    launch(k_cleanup<true>, grid_for(EMAX), kLineThreads, 0, s, tris, m, (const int2 *)edges, d_n_edges, pts, eflag,
+           (const int *)first_near, (const int *)near_tris, occ, collapsed, active, dcnt);
     launch(k_b_line_apply, 1, kLineThreads, 0, s, edges, d_n_edges, eflag, first_near, near_tris, pts, tris, occ,
            line_list, (const int *)vslot, dcnt, scnt, K);
     launch(k_b_cand_fill, grid_for(EMAX), kThreads, 0, s, (const int *)collapsed, (const int *)line_list, edges,
-           (const int *)vslot, (const RoundCounters *)dcnt, (const SlotCounters *)scnt, cand);
-
-    // as in the single-mesh round, each undo pass queries only the one-rings undone
-    auto pass = [&](bool undo) -> int {
-        if (!undo || hcnt->n_line == 0)
-            S2_TRY(mark_active(*this, m, undo ? undo_edges : cand, undo ? &dcnt->n_undo : &dcnt->n_considered, s));
-        S2_TRY(isect_pass(*this, m, s));
-        S2_TRY(undo_check_batch(*this, K, s));
-        S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
+           (const int *)vslot, (const RoundCounters *)dcnt, (const SlotCounters *)scnt, cand, (const int *)first_near,
+           (const int *)near_tris, active);
+    // a check, and where it finds edges to undo their list and each mesh's share of it
+    auto pass = [&]() -> int {
+        int rc = checked_pass(*this, m, cand, s);
+        if (rc) return rc;
+        for (int r = 0; r < K; ++r) hscnt[r].n_undo = 0;
+        if (hcnt->n_undo == 0) return PAMO_OK;
+        S2_TRY(undo_list_of(*this, eflag, s));
+        launch(k_b_undo_counts, grid_for(K), kThreads, 0, s, (const int *)eflag, (const RoundCounters *)dcnt, scnt, K);
         S2_TRY(cudaMemcpyAsync(hscnt, scnt, (size_t)K * sizeof(SlotCounters), cudaMemcpyDeviceToHost, s));
         S2_TRY(cudaStreamSynchronize(s));
-        prof.collect();
-        if (hcnt->pair_overflow > 0) {
-            long long need = (long long)hcnt->n_pairs + hcnt->n_pairs / 2 + 1024;
-            int rc = ensure_pairs(need);
-            if (rc) return rc;
-            S2_TRY(isect_pass(*this, m, s));
-            S2_TRY(undo_check_batch(*this, K, s));
-            S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-            S2_TRY(cudaMemcpyAsync(hscnt, scnt, (size_t)K * sizeof(SlotCounters), cudaMemcpyDeviceToHost, s));
-            S2_TRY(cudaStreamSynchronize(s));
-            if (hcnt->pair_overflow > 0) return PAMO_ERR_CAPACITY;
-        }
-    if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
         return PAMO_OK;
     };
-    int rc = pass(false);
+    int rc = pass();
     if (rc) return rc;
     last_stats[0] = hcnt->n_edges;
     last_stats[1] = hcnt->n_main;
@@ -2043,18 +1994,19 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     while (any) {
         it++;
         prof.begin(PH_UNDO, s);
-        launch(k_undo_apply, grid_for(hcnt->n_undo), kThreads, 0, s, undo_edges, dcnt, edges, first_near, near_tris,
-               opts, otris, pts, tris, occ);
-        long long max_cnt = 0;
         for (int r = 0; r < K; ++r) {
             hslots[r].pass_first = first[r];
-            hslots[r].pass_count = nvu[r] - first[r];
-            max_cnt = hslots[r].pass_count > max_cnt ? hslots[r].pass_count : max_cnt;
             first[r] += 2 * cnt_undo[r];
         }
         S2_TRY(cudaMemcpyAsync(slots, hslots, (size_t)K * sizeof(SlotInfo), cudaMemcpyHostToDevice, s));
-        if (max_cnt > 0) launch(k_b_rearrange, slot_grid(K, max_cnt), kThreads, 0, s, (const SlotInfo *)slots);
-        rc = pass(true);
+        const bool reselect = hcnt->n_line == 0;  // as in the single-mesh round
+        if (reselect) S2_TRY(cudaMemsetAsync(active, 0, (size_t)m, s));
+        launch(k_undo_apply, grid_for(hcnt->n_undo), kThreads, 0, s, (const int *)undo_idx, hcnt->n_undo,
+               (const int *)cand, (const int2 *)edges, (const int *)first_near, (const int *)near_tris,
+               (const float4 *)opts, (const int4 *)otris, pts, tris, occ, reselect ? active : nullptr,
+               (const int *)nullptr, (int *)nullptr, 0, (const SlotInfo *)slots, (const SlotCounters *)scnt,
+               (const int *)vslot, dcnt);
+        rc = pass();
         if (rc) return rc;
         any = false;
         for (int r = 0; r < K; ++r) {
@@ -2068,7 +2020,8 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     last_stats[3] = it;
     // the packed vertex map, each mesh's own map and undo-list copy
     prof.begin(PH_COMPACT, s);
-    S2_TRY(exclusive_scan(occ, gmap, (long long)n + 1, nullptr, scan_scratch, nullptr, s, &dcnt->scan_fault));
+    S2_TRY(scan_jobs(ScanJob{occ, nullptr, gmap, nullptr, n + 1LL, nullptr, scan_scratch, nullptr},
+                     ScanJob{nullptr, tris, fpos, nullptr, m, nullptr, scan_scratch2, fpos + m}, s, &dcnt->scan_fault));
     long long max_nvu = 0;
     for (int r = 0; r < K; ++r) {
         hslots[r].nvu = nvu[r];
@@ -2085,12 +2038,9 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
 int Stage2::compact_batch(int n, int m, int K, cudaStream_t s)
 {
     prof.begin(PH_COMPACT, s);
-    launch(k_face_live_flags, grid_for(m), kThreads, 0, s, tris, m, fflag);
-    S2_TRY(cudaMemsetAsync(fflag + m, 0, 4, s));
-    S2_TRY(exclusive_scan(fflag, uflag, (long long)m + 1, nullptr, scan_scratch, nullptr, s, &dcnt->scan_fault));
-    launch(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, pts, occ, gmap, n, tris, fflag, uflag, m, opts, otris,
-           dcnt);
-    launch(k_b_next, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)gmap, (const int *)uflag, scnt,
+    launch(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, (const float4 *)pts, (const int *)occ, (const int *)gmap,
+           n, (const int4 *)tris, (const int *)fpos, m, opts, otris, (int *)nullptr, 0, dcnt);
+    launch(k_b_next, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)gmap, (const int *)fpos, scnt,
            K);
     prof.end(s);
     S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));

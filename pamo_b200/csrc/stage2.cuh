@@ -17,12 +17,14 @@ struct RoundCounters {
     int n_undo;          // undo edges found by the last check
     int n_pairs;         // candidate pairs found by the last query
     int pair_overflow;   // pairs dropped for lack of buffer space
-    int n_query;         // faces in this pass's query list (reset with the two above)
+    int n_query;         // faces in this pass's query list
+    int n_hit;           // whether a pair of this pass intersects (reset with the three above)
     int n_pts_next;      // compaction result
     int n_tris_next;
     int n_edges;
     int scan_fault;      // a prefix scan's wait ran out (see scan.cuh)
-    int pad[4];
+    int ticket;          // k_cleanup's finished blocks
+    int pad[2];
 };
 
 // ---------------------------------------------------------------------------
@@ -48,7 +50,7 @@ struct SlotInfo {        // uploaded by the host before each round, indexed by r
     int clear_invalid;   // clear the invalid table before marking (not stuck, list non-empty)
     uint32_t collapse_t;
     float tres;          // threshold
-    int pass_first, pass_count;  // undo pass: rearrangement window of the undo list
+    int pass_first;      // undo pass: where its vertices go in the undo list
     int nvu;             // undo-list length at the end of the round
     const float *scale;  // device scalar: the mesh's scale (max bbox extent)
     uint32_t *edge_cost; // [3 m0 + 1] edge costs (stale between rounds)
@@ -143,13 +145,14 @@ struct Stage2 {
     unsigned long long *vmin = nullptr;
     int *eflag = nullptr;
     int *collapsed = nullptr;
-    uint8_t *active = nullptr;
+    uint8_t *active = nullptr;  // faces that query the tree in this pass
     uint8_t *isect = nullptr;
     int *uflag = nullptr;
-    int *undo_edges = nullptr;
-    int *fflag = nullptr;  // face compaction flags
+    int *undo_idx = nullptr;  // undone edges, as positions in the collapsed list
+    int *fpos = nullptr;      // each face's position after compaction
+    int *qlist = nullptr;     // leaves that query the tree in this pass
     uint2 *pairs = nullptr;
-    int *scan_scratch = nullptr;
+    int *scan_scratch = nullptr, *scan_scratch2 = nullptr;  // two scans run in one launch
     long long scan_scratch_len = 0;
     int *dev_misc = nullptr;  // scalars: [0] tris_mean-bits etc.
     RoundCounters *dcnt = nullptr;
