@@ -11,14 +11,15 @@
 // (simp_cuda/safe_project/scripts/cgal_intersect/main.cpp:19-111): faces that
 // share a vertex or an edge intersect only beyond what they share.
 //
-// Both traverse the faces' LBVH (lbvh.cuh) without a stack: inner nodes keep
-// both child boxes, the parent array gives the way up, and a walker that
-// returns to a node from its first child goes on to the second.
+// Both walk the faces' packed tree (ptree.cuh), a group of eight lanes per face or
+// sample.  A call's scratch is one allocation from the device's stream-ordered
+// pool: with a dozen cudaMalloc / cudaFree pairs a call, which synchronise the
+// device, the check of a 350k-face mesh took 12 to 60 ms, of which its kernels 5.
 #include <cfloat>
 #include <vector>
 
 #include "exact.cuh"
-#include "lbvh.cuh"
+#include "ptree.cuh"
 #include "scan.cuh"
 
 namespace pamo {
@@ -36,7 +37,7 @@ enum CheckCounter {
     C_UNREFERENCED,    // vertices in no live face
     C_CANDIDATES,      // face pairs with overlapping boxes
     C_DEAD,            // faces (-1, -1, -1)
-    C_ERROR,           // traversal budget exceeded (corrupt hierarchy)
+    C_ERROR,           // always 0 (a walk of the tree ends by itself)
     C_BAD_INDEX,       // an index outside [0, n_pts) in a live face
     C_COUNT
 };
@@ -73,104 +74,116 @@ __device__ __forceinline__ void load_tri(const float4 *p, int4 t, P3 *T, int *id
     }
 }
 
-// degenerate flag per live face; counts
-__global__ void k_ck_degenerate(const float4 *p, const int4 *tris, int m, uint8_t *deg, unsigned long long *cnt)
+// whether a face is live and not degenerate (those are tested); counts
+__global__ void k_ck_degenerate(const float4 *p, const int4 *tris, int m, uint8_t *ok, unsigned long long *cnt)
 {
     PAMO_GRID_STRIDE(f, m)
     {
         const int4 t = tris[f];
-        uint8_t d = 0;
+        uint8_t good = 0;
         if (!face_dead(t)) {
             P3 T[3];
             int idx[3];
             load_tri(p, t, T, idx);
-            d = exact::tri_degenerate(T, idx) ? 1 : 0;
-            if (d) atomicAdd(&cnt[C_DEGENERATE], 1ULL);
+            good = exact::tri_degenerate(T, idx) ? 0 : 1;
+            if (!good) atomicAdd(&cnt[C_DEGENERATE], 1ULL);
         }
-        deg[f] = d;
+        ok[f] = good;
     }
 }
 
-__device__ __forceinline__ bool overlaps(float4 lo, float4 hi, float3 qlo, float3 qhi)
+__device__ __noinline__ bool pair_intersects(const float4 *p, int4 ta, int4 tb)
 {
-    return !(hi.x < qlo.x || qhi.x < lo.x || hi.y < qlo.y || qhi.y < lo.y || hi.z < qlo.z || qhi.z < lo.z);
+    P3 A[3], B[3];
+    int ia[3], ib[3];
+    load_tri(p, ta, A, ia);
+    load_tri(p, tb, B, ib);
+    return exact::faces_intersect(A, ia, B, ib);
 }
 
-// Every pair f < g of live faces with overlapping closed boxes, one thread per
-// leaf (Morton order, so a warp's faces are neighbours and walk similar paths).
-__global__ void __launch_bounds__(128) k_ck_pairs(const BvhNode *__restrict__ nodes, const int *__restrict__ parent,
-                                                  const int *__restrict__ vals, const int *scene,
-                                                  const float4 *__restrict__ p, const int4 *__restrict__ tris,
-                                                  const uint8_t *__restrict__ deg, uint8_t *flags,
-                                                  unsigned long long *cnt)
+// Every pair f < g of tested faces with overlapping closed boxes: a group of eight
+// lanes walks the tree for each f, and a warp's pairs gather in shared memory
+// until 32 of them can be tested, one a lane.  With one thread per face, testing
+// each leaf as it met it on a binary hierarchy, most lanes of a warp waited while
+// one evaluated a predicate: 5.0 ms on a 350k-face torus; the whole check of that
+// mesh takes 1.4 ms so.
+constexpr int kPairThreads = 128;
+
+__global__ void __launch_bounds__(kPairThreads) k_ck_pairs(const __grid_constant__ TreeView T,
+                                                           const int *__restrict__ qlist, const int *n_query,
+                                                           const float4 *__restrict__ p, uint8_t *flags,
+                                                           unsigned long long *cnt)
 {
-    const int L = scene[7];
-    if (L < 2) return;
-    PAMO_GRID_STRIDE(pp, L)
-    {
-        const int f = vals[pp];
-        const int4 tf = tris[f];
-        if (deg[f]) continue;
-        P3 A[3];
-        int ia[3];
-        load_tri(p, tf, A, ia);
-        const float3 qlo = make_float3(fminf((float)A[0].x, fminf((float)A[1].x, (float)A[2].x)),
-                                       fminf((float)A[0].y, fminf((float)A[1].y, (float)A[2].y)),
-                                       fminf((float)A[0].z, fminf((float)A[1].z, (float)A[2].z)));
-        const float3 qhi = make_float3(fmaxf((float)A[0].x, fmaxf((float)A[1].x, (float)A[2].x)),
-                                       fmaxf((float)A[0].y, fmaxf((float)A[1].y, (float)A[2].y)),
-                                       fmaxf((float)A[0].z, fmaxf((float)A[1].z, (float)A[2].z)));
-        unsigned long long cand = 0;
+    __shared__ int2 s_pairs[kPairThreads / 32][64];  // leaves of f and g
+    __shared__ int s_off[kTreeMaxLevels];
+#pragma unroll
+    for (int l = 0; l < kTreeMaxLevels; ++l)
+        if (threadIdx.x == l) s_off[l] = T.off[l];
+    __syncthreads();
+    int2 *buf = s_pairs[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
+    const unsigned below = (1u << lane) - 1u;
+    const int N = *n_query;
+    int held = 0;
+    unsigned long long cand = 0, found = 0;
+    auto test = [&](int n) {
         bool hit = false;
-        auto visit_leaf = [&](int leaf) {
-            const int g = vals[leaf];
-            if (g <= f || deg[g]) return;
-            ++cand;
-            P3 B[3];
-            int ib[3];
-            load_tri(p, tris[g], B, ib);
-            if (exact::faces_intersect(A, ia, B, ib)) {
-                hit = true;
-                flags[g] = 1;
-                atomicAdd(&cnt[C_PAIRS], 1ULL);
+        if (lane < n) {
+            const int4 a = T.leaf[buf[lane].x], b = T.leaf[buf[lane].y];
+            hit = pair_intersects(p, a, b);
+            if (hit) flags[a.w] = flags[b.w] = 1;
+        }
+        cand += n;
+        found += __popc(__ballot_sync(0xffffffffu, hit));
+    };
+    const long long warps = (long long)gridDim.x * (kPairThreads / 32);
+    for (long long w = ((long long)blockIdx.x * kPairThreads + threadIdx.x) >> 5; w * 4 < N; w += warps) {
+        const long long k = w * 4 + (lane >> 3);
+        const bool has = k < N;
+        const int q = has ? qlist[k] : 0;
+        const int f = T.leaf[q].w;
+        const float4 qlo = T.boxes[2 * (size_t)q], qhi = T.boxes[2 * (size_t)q + 1];
+        TreeWalk wk;
+        wk.start(T, has);
+        while (__any_sync(0xffffffffu, wk.run)) {
+            bool hit = false, emit = false;
+            const int node = 8 * wk.g + gl;
+            if (wk.run) {
+                const size_t b = 2 * ((size_t)s_off[wk.lvl] + node);
+                const float4 lo = T.boxes[b], hi = T.boxes[b + 1];
+                const bool leaf = wk.lvl == 0 && node < T.L;
+                const int g = leaf ? T.leaf[node].w : kLeafDead;
+                hit = !(hi.x < qlo.x || qhi.x < lo.x || hi.y < qlo.y || qhi.y < lo.y || hi.z < qlo.z || qhi.z < lo.z);
+                emit = hit && g > f;  // selected leaves have their face's number, the others a negative one
             }
-        };
-        // stackless walk: `from` 0 = arrived from the parent, 1 = from the left
-        // child, 2 = from the right child
-        int node = 0, from = 0;
-        long long budget = 4LL * L + 16;
-        while (true) {
-            if (--budget < 0) {
-                atomicAdd(&cnt[C_ERROR], 1ULL);
-                break;
-            }
-            const BvhNode nd = nodes[node];
-            int next = -1;
-            if (from == 0) {
-                if (overlaps(nd.llo, nd.lhi, qlo, qhi)) {
-                    const int c = __float_as_int(nd.llo.w);
-                    if (c >= 0) next = c;
-                    else visit_leaf(~c);
+            const unsigned hits = __ballot_sync(0xffffffffu, hit), em = __ballot_sync(0xffffffffu, emit);
+            if (em) {
+                if (emit) buf[held + __popc(em & below)] = make_int2(q, node);
+                held += __popc(em);
+                __syncwarp();
+                if (held >= 32) {
+                    test(32);
+                    held -= 32;
+                    const int2 rest = buf[32 + lane];
+                    __syncwarp();
+                    buf[lane] = rest;
+                    __syncwarp();
                 }
             }
-            if (next < 0 && from != 2 && overlaps(nd.rlo, nd.rhi, qlo, qhi)) {
-                const int c = __float_as_int(nd.rlo.w);
-                if (c >= 0) next = c;
-                else visit_leaf(~c);
-            }
-            if (next >= 0) {
-                node = next;
-                from = 0;
-                continue;
-            }
-            const int code = parent[node];
-            if (code < 0) break;  // back at the root
-            node = code >> 2;
-            from = (code & 1) ? 2 : 1;
+            if (wk.run) wk.advance(T, (hits >> shift) & 255u);
         }
-        if (hit) flags[f] = 1;
-        if (cand) atomicAdd(&cnt[C_CANDIDATES], cand);
     }
+    if (held > 0) test(held);
+    if (lane == 0 && cand) atomicAdd(&cnt[C_CANDIDATES], cand);
+    if (lane == 0 && found) atomicAdd(&cnt[C_PAIRS], found);
+}
+
+__global__ void k_ck_flagged(const uint8_t *flags, int m, unsigned long long *cnt)
+{
+    int n = 0;
+    PAMO_GRID_STRIDE(f, m) n += flags[f];
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&cnt[C_FACES], (unsigned long long)n);
 }
 
 __global__ void k_ck_count(const int4 *tris, int m, int *deg_v)
@@ -332,80 +345,104 @@ __device__ __forceinline__ double box_d2(float4 lo, float4 hi, D3 p)
     return dx * dx + dy * dy + dz * dz;
 }
 
-// squared distance from p to the nearest face of the hierarchy's mesh: a
-// stackless walk that enters the nearer child first and the farther one on
-// the way back if its box is still closer than the best face so far
-__device__ double nearest_d2(D3 p, const BvhNode *__restrict__ nodes, const int *__restrict__ parent,
-                             const int *__restrict__ vals, int L, const float4 *__restrict__ pts,
-                             const int4 *__restrict__ tris, unsigned long long *err)
+// Squared distance from the group's point p to the nearest face of the tree's
+// mesh.  The eight lanes test a node's children, the walk enters the nearest one
+// and leaves the others that could still hold something closer on the group's
+// stack (shared memory; at most seven a level).  All lanes of a warp call this
+// together; the result is the same in all lanes of a group.
+constexpr int kHdThreads = 128;
+constexpr int kHdStack = 64;
+
+struct HdEntry {
+    double d2;
+    int lvl, g;
+};
+
+__device__ __forceinline__ double nearest_d2(bool has, D3 p, const TreeView &T, const int *off, HdEntry *stack,
+                                             const float4 *__restrict__ pts)
 {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
     double best = DBL_MAX;
-    auto leaf = [&](int pos) {
-        const int g = vals[pos];
-        if (g < 0) return;
-        const int4 t = tris[g];
-        const double d2 = point_tri_d2(p, dat(pts[t.x]), dat(pts[t.y]), dat(pts[t.z]));
-        best = fmin(best, d2);
-    };
-    if (L == 1) {
-        leaf(0);
-        return best;
-    }
-    int node = 0, from = 0;  // from: 0 parent, 1 left child, 2 right child
-    long long budget = 4LL * L + 16;
-    while (true) {
-        if (--budget < 0) {
-            atomicAdd(err, 1ULL);
-            break;
-        }
-        const BvhNode nd = nodes[node];
-        const double dl = box_d2(nd.llo, nd.lhi, p), dr = box_d2(nd.rlo, nd.rhi, p);
-        const int near_side = dl <= dr ? 1 : 2;
-        const int cl = __float_as_int(nd.llo.w), cr = __float_as_int(nd.rlo.w);
-        int next = -1;
-        // from the parent: the nearer side, then the farther; back from the
-        // nearer side: the farther; back from the farther side: done here
-        if (from == 0 || from == near_side) {
-            for (int k = from == 0 ? 0 : 1; k < 2 && next < 0; ++k) {
-                const int side = k == 0 ? near_side : 3 - near_side;
-                if ((side == 1 ? dl : dr) >= best) continue;
-                const int c = side == 1 ? cl : cr;
-                if (c >= 0) next = c;
-                else leaf(~c);
+    int lvl = T.top, g = 0, topg = 0, sp = 0;
+    bool run = has;
+    while (__any_sync(kAll, run)) {
+        const int node = 8 * g + gl;
+        double d = DBL_MAX;
+        if (run) {
+            const size_t b = 2 * ((size_t)off[lvl] + node);
+            d = box_d2(T.boxes[b], T.boxes[b + 1], p);
+            if (lvl == 0) {
+                const int4 t = d < best && node < T.L ? T.leaf[node] : make_int4(0, 0, 0, kLeafDead);
+                d = t.w != kLeafDead ? point_tri_d2(p, dat(pts[t.x]), dat(pts[t.y]), dat(pts[t.z])) : DBL_MAX;
             }
         }
-        if (next >= 0) {
-            node = next;
-            from = 0;
-            continue;
+        double m = d;
+        int at = gl;  // the nearest of the eight (the lowest lane of equals)
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const double md = __shfl_xor_sync(kAll, m, o);
+            const int ma = __shfl_xor_sync(kAll, at, o);
+            if (md < m || (md == m && ma < at)) {
+                m = md;
+                at = ma;
+            }
         }
-        const int code = parent[node];
-        if (code < 0) break;
-        node = code >> 2;
-        from = (code & 1) ? 2 : 1;
+        const bool inner = run && lvl > 0;
+        const unsigned others = (__ballot_sync(kAll, inner && d < best && gl != at) >> shift) & 255u;
+        if (inner && d < best && gl != at) stack[sp + __popc(others & ((1u << gl) - 1u))] = HdEntry{d, lvl - 1, node};
+        __syncwarp();
+        if (run) {
+            sp += __popc(others);
+            if (inner && m < best) {
+                g = 8 * g + at;
+                --lvl;
+            } else {
+                if (lvl == 0 && m < best) best = m;
+                bool found = false;
+                while (sp > 0 && !found) {
+                    const HdEntry e = stack[--sp];
+                    found = e.d2 < best;
+                    lvl = e.lvl;
+                    g = e.g;
+                }
+                if (!found) {
+                    run = ++topg < T.top_groups;
+                    lvl = T.top;
+                    g = topg;
+                }
+            }
+        }
+        __syncwarp();
     }
     return best;
 }
 
-// One thread per sample (face f of A, barycentric grid point (i/k, j/k)):
-// distance to mesh B; the block's largest squared distance and the sum of the
-// squared distances go to this block's partials.
-__global__ void __launch_bounds__(128) k_hd_samples(const float4 *__restrict__ pa, const int4 *__restrict__ fa,
-                                                    int nfa, int k, const BvhNode *__restrict__ nodes,
-                                                    const int *__restrict__ parent, const int *__restrict__ vals,
-                                                    const int *scene, const float4 *__restrict__ pb,
-                                                    const int4 *__restrict__ fb, double *part_max, double *part_sum,
-                                                    double *part_edge, unsigned long long *err)
+// One group of eight lanes per sample (face f of A, barycentric grid point (i/k,
+// j/k)): distance to mesh B; the block's largest squared distance and the sum of
+// the squared distances go to this block's partials.
+__global__ void __launch_bounds__(kHdThreads) k_hd_samples(const float4 *__restrict__ pa, const int4 *__restrict__ fa,
+                                                           int nfa, int k, const __grid_constant__ TreeView T,
+                                                           const float4 *__restrict__ pb, double *part_max,
+                                                           double *part_sum, double *part_edge)
 {
-    const int L = scene[7];
+    __shared__ HdEntry s_stack[kHdThreads / 8][kHdStack];
+    __shared__ int s_off[kTreeMaxLevels];
+#pragma unroll
+    for (int l = 0; l < kTreeMaxLevels; ++l)
+        if (threadIdx.x == l) s_off[l] = T.off[l];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
     const int S = (k + 1) * (k + 2) / 2;
+    const long long total = (long long)nfa * S;
     double mx = 0.0, sum = 0.0, edge = 0.0;
-    PAMO_GRID_STRIDE(i, (long long)nfa * S)
-    {
-        const int f = (int)(i / S);
+    const long long warps = (long long)gridDim.x * (kHdThreads / 32);
+    for (long long w = ((long long)blockIdx.x * kHdThreads + threadIdx.x) >> 5; w * 4 < total; w += warps) {
+        const long long i = w * 4 + (lane >> 3);
+        const int f = i < total ? (int)(i / S) : 0;
         int s = (int)(i % S);
         const int4 t = fa[f];
-        if (face_dead(t) || L == 0) continue;
+        const bool has = i < total && !face_dead(t);
         // s -> (u, v) with u + v <= k, rows of u
         int u = 0;
         while (s > k - u) {
@@ -413,11 +450,17 @@ __global__ void __launch_bounds__(128) k_hd_samples(const float4 *__restrict__ p
             ++u;
         }
         const int v = s;
-        const D3 a = dat(pa[t.x]), b = dat(pa[t.y]), c = dat(pa[t.z]);
+        D3 a{}, b{}, c{};
+        if (has) {
+            a = dat(pa[t.x]);
+            b = dat(pa[t.y]);
+            c = dat(pa[t.z]);
+        }
         const double su = (double)u / k, sv = (double)v / k;
         const D3 q = {a.x + su * (b.x - a.x) + sv * (c.x - a.x), a.y + su * (b.y - a.y) + sv * (c.y - a.y),
                       a.z + su * (b.z - a.z) + sv * (c.z - a.z)};
-        const double d2 = nearest_d2(q, nodes, parent, vals, L, pb, fb, err);
+        const double d2 = nearest_d2(has, q, T, s_off, s_stack[threadIdx.x >> 3], pb);
+        if (!has || (lane & 7) != 0) continue;
         mx = fmax(mx, d2);
         sum += d2;
         if (u == 0 && v == 0) {  // the face's longest edge, once per face
@@ -425,12 +468,12 @@ __global__ void __launch_bounds__(128) k_hd_samples(const float4 *__restrict__ p
             edge = fmax(edge, fmax(ddot(e0, e0), fmax(ddot(e1, e1), ddot(e2, e2))));
         }
     }
-    __shared__ double sm[3][128];
+    __shared__ double sm[3][kHdThreads];
     sm[0][threadIdx.x] = mx;
     sm[1][threadIdx.x] = sum;
     sm[2][threadIdx.x] = edge;
     __syncthreads();
-    for (int o = 64; o > 0; o >>= 1) {
+    for (int o = kHdThreads / 2; o > 0; o >>= 1) {
         if (threadIdx.x < o) {
             sm[0][threadIdx.x] = fmax(sm[0][threadIdx.x], sm[0][threadIdx.x + o]);
             sm[1][threadIdx.x] += sm[1][threadIdx.x + o];
@@ -447,20 +490,31 @@ __global__ void __launch_bounds__(128) k_hd_samples(const float4 *__restrict__ p
 
 constexpr int kHdBlocks = kNumSMs * 8;
 
-struct DeviceBuf {
-    void *p = nullptr;
+// One stream-ordered allocation, handed out in pieces: sized by a first pass over
+// the same take() calls with no memory behind them.
+struct Scratch {
+    unsigned char *p = nullptr;
+    size_t at = 0;
     cudaStream_t s = nullptr;
-    DeviceBuf(size_t bytes, cudaStream_t st) : s(st)
-    {
-        if (bytes && cudaMallocAsync(&p, bytes, st) != cudaSuccess) p = nullptr;
-    }
-    ~DeviceBuf()
+    explicit Scratch(cudaStream_t st) : s(st) {}
+    ~Scratch()
     {
         if (p) cudaFreeAsync(p, s);
     }
-    DeviceBuf(const DeviceBuf &) = delete;
-    DeviceBuf &operator=(const DeviceBuf &) = delete;
-    template <class T> T *as() const { return static_cast<T *>(p); }
+    Scratch(const Scratch &) = delete;
+    Scratch &operator=(const Scratch &) = delete;
+    bool allocate()  // after the sizing pass
+    {
+        const size_t bytes = at;
+        at = 0;
+        return cudaMallocAsync((void **)&p, bytes ? bytes : 1, s) == cudaSuccess;
+    }
+    template <class T> T *take(size_t n)
+    {
+        T *q = p ? reinterpret_cast<T *>(p + at) : nullptr;
+        at += tree_align(n * sizeof(T));
+        return q;
+    }
 };
 
 }  // namespace
@@ -481,63 +535,64 @@ extern "C" int pamo_check_mesh(const float *d_points, const int *d_tris, int n_p
     if (cudaGetDevice(&dev) != cudaSuccess) return PAMO_ERR_NO_DEVICE;
     cudaStream_t s = (cudaStream_t)stream;
     PAMO_CUDA_TRY(retain_pool_memory());
-    DeviceBuf p4((size_t)n_pts * 16, s), t4((size_t)n_tris * 16, s), cnt(C_COUNT * 8, s), deg((size_t)n_tris, s);
-    DeviceBuf flags(d_out_flags ? 0 : (size_t)n_tris, s);
-    DeviceBuf degv(((size_t)n_pts + 1) * 4, s), first(((size_t)n_pts + 1) * 4, s), cursor((size_t)n_pts * 4, s);
-    DeviceBuf faces_of((size_t)n_tris * 3 * 4, s), scan_tmp((size_t)scan_scratch_ints((long long)n_pts + 1) * 4, s);
-    if (!p4.p || !t4.p || !cnt.p || !deg.p || !degv.p || !first.p || !cursor.p || !faces_of.p || !scan_tmp.p ||
-        (!d_out_flags && !flags.p))
-        return PAMO_ERR_OOM;
-    uint8_t *fl = d_out_flags ? d_out_flags : flags.as<uint8_t>();
-    unsigned long long *c = cnt.as<unsigned long long>();
-    PAMO_CUDA_TRY(cudaMemsetAsync(c, 0, C_COUNT * 8, s));
-    PAMO_CUDA_TRY(cudaMemsetAsync(fl, 0, (size_t)n_tris, s));
-    launch(k_ck_convert, grid_for(n_pts > n_tris ? n_pts : n_tris), kThreads, 0, s, d_points, n_pts, d_tris, n_tris,
-           p4.as<float4>(), t4.as<int4>());
-    launch(k_ck_validate, grid_for(n_tris), kThreads, 0, s, (const int4 *)t4.as<int4>(), n_tris, n_pts, c);
-    unsigned long long h_bad[C_COUNT];
-    PAMO_CUDA_TRY(cudaMemcpyAsync(h_bad, c, C_COUNT * 8, cudaMemcpyDeviceToHost, s));
-    PAMO_CUDA_TRY(cudaStreamSynchronize(s));
-    if (h_bad[C_BAD_INDEX]) return PAMO_ERR_INVALID_ARG;
-    launch(k_ck_degenerate, grid_for(n_tris), kThreads, 0, s, (const float4 *)p4.as<float4>(),
-           (const int4 *)t4.as<int4>(), n_tris, deg.as<uint8_t>(), c);
-    // self-intersections
-    Lbvh b;
-    cudaError_t e = lbvh_build(b, p4.as<float4>(), t4.as<int4>(), n_tris, s);
-    if (e == cudaSuccess) e = lbvh_refit(b, p4.as<float4>(), t4.as<int4>(), n_tris, s);
-    if (e != cudaSuccess) {
-        b.release();
-        return map_cuda_error(e);
+    const size_t n = (size_t)n_pts, m = (size_t)n_tris;
+    const long long scan_ints = scan_scratch_ints((long long)n_pts + 1);
+    Scratch mem(s);
+    float4 *p4;
+    int4 *t4;
+    unsigned long long *c;
+    uint8_t *ok, *fl;
+    int *qlist, *n_query, *degv, *first, *cursor, *faces_of, *scan_tmp;
+    unsigned char *tree_mem;
+    for (int pass = 0; pass < 2; ++pass) {
+        p4 = mem.take<float4>(n);
+        t4 = mem.take<int4>(m);
+        c = mem.take<unsigned long long>(C_COUNT + 1);
+        ok = mem.take<uint8_t>(m);
+        fl = d_out_flags ? d_out_flags : mem.take<uint8_t>(m);
+        qlist = mem.take<int>(m);
+        degv = mem.take<int>(n + 1);
+        first = mem.take<int>(n + 1);
+        cursor = mem.take<int>(n);
+        faces_of = mem.take<int>(3 * m);
+        scan_tmp = mem.take<int>((size_t)scan_ints);
+        tree_mem = mem.take<unsigned char>(PackedTree::bytes(n_tris));
+        if (pass == 0 && !mem.allocate()) return PAMO_ERR_OOM;
     }
-    launch(k_ck_pairs, grid_for(n_tris, 128), 128, 0, s, (const BvhNode *)b.nodes, (const int *)b.parent,
-           (const int *)b.vals, (const int *)b.scene, (const float4 *)p4.as<float4>(), (const int4 *)t4.as<int4>(),
-           (const uint8_t *)deg.as<uint8_t>(), fl, c);
-    // manifold checks over the vertex -> face lists
-    PAMO_CUDA_TRY(cudaMemsetAsync(degv.p, 0, ((size_t)n_pts + 1) * 4, s));
-    PAMO_CUDA_TRY(cudaMemsetAsync(cursor.p, 0, (size_t)n_pts * 4, s));
-    launch(k_ck_count, grid_for(n_tris), kThreads, 0, s, (const int4 *)t4.as<int4>(), n_tris, degv.as<int>());
-    PAMO_CUDA_TRY(scan_scratch_init(scan_tmp.as<int>(), scan_scratch_ints((long long)n_pts + 1), s));
-    PAMO_CUDA_TRY(exclusive_scan(degv.as<int>(), first.as<int>(), (long long)n_pts + 1, nullptr, scan_tmp.as<int>(),
-                                 nullptr, s));
-    launch(k_ck_fill, grid_for(n_tris), kThreads, 0, s, (const int4 *)t4.as<int4>(), n_tris,
-           (const int *)first.as<int>(), cursor.as<int>(), faces_of.as<int>());
-    launch(k_ck_edges, grid_for(3LL * n_tris), kThreads, 0, s, (const int4 *)t4.as<int4>(), n_tris,
-           (const int *)first.as<int>(), (const int *)faces_of.as<int>(), c);
-    launch(k_ck_fans, grid_for(n_pts), kThreads, 0, s, (const int4 *)t4.as<int4>(), n_pts,
-           (const int *)first.as<int>(), (const int *)faces_of.as<int>(), c);
-    // faces in intersecting pairs
+    n_query = reinterpret_cast<int *>(c + C_COUNT);
+    PAMO_CUDA_TRY(cudaMemsetAsync(c, 0, (C_COUNT + 1) * 8, s));
+    launch(k_ck_convert, grid_for(n_pts > n_tris ? n_pts : n_tris), kThreads, 0, s, d_points, n_pts, d_tris, n_tris, p4,
+           t4);
+    launch(k_ck_validate, grid_for(n_tris), kThreads, 0, s, (const int4 *)t4, n_tris, n_pts, c);
     unsigned long long h[C_COUNT];
-    e = cudaMemcpyAsync(h, c, C_COUNT * 8, cudaMemcpyDeviceToHost, s);
-    std::vector<uint8_t> hf((size_t)n_tris);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hf.data(), fl, (size_t)n_tris, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    b.release();
-    if (e != cudaSuccess) return map_cuda_error(e);
-    long long nf = 0;
-    for (uint8_t x : hf) nf += x;
+    PAMO_CUDA_TRY(cudaMemcpyAsync(h, c, C_COUNT * 8, cudaMemcpyDeviceToHost, s));
+    PAMO_CUDA_TRY(cudaStreamSynchronize(s));
+    if (h[C_BAD_INDEX]) return PAMO_ERR_INVALID_ARG;
+    launch(k_ck_degenerate, grid_for(n_tris), kThreads, 0, s, (const float4 *)p4, (const int4 *)t4, n_tris, ok, c);
+    // self-intersections (the refit clears the flags)
+    PackedTree tree;  // its arrays lie in this call's scratch: nothing to release
+    PAMO_CUDA_TRY(tree.place(tree_mem, n_tris, s));
+    PAMO_CUDA_TRY(tree_build(tree, p4, t4, n_tris, s));
+    PAMO_CUDA_TRY(tree_refit(tree, p4, t4, ok, qlist, n_query, fl, n_tris, s));
+    launch(k_ck_pairs, grid_for(8LL * n_tris, kPairThreads), kPairThreads, 0, s, tree.view(), (const int *)qlist,
+           (const int *)n_query, (const float4 *)p4, fl, c);
+    launch(k_ck_flagged, grid_for(n_tris), kThreads, 0, s, (const uint8_t *)fl, n_tris, c);
+    // manifold checks over the vertex -> face lists
+    PAMO_CUDA_TRY(cudaMemsetAsync(degv, 0, (n + 1) * 4, s));
+    PAMO_CUDA_TRY(cudaMemsetAsync(cursor, 0, n * 4, s));
+    launch(k_ck_count, grid_for(n_tris), kThreads, 0, s, (const int4 *)t4, n_tris, degv);
+    PAMO_CUDA_TRY(scan_scratch_init(scan_tmp, scan_ints, s));
+    PAMO_CUDA_TRY(exclusive_scan(degv, first, (long long)n_pts + 1, nullptr, scan_tmp, nullptr, s));
+    launch(k_ck_fill, grid_for(n_tris), kThreads, 0, s, (const int4 *)t4, n_tris, (const int *)first, cursor, faces_of);
+    launch(k_ck_edges, grid_for(3LL * n_tris), kThreads, 0, s, (const int4 *)t4, n_tris, (const int *)first,
+           (const int *)faces_of, c);
+    launch(k_ck_fans, grid_for(n_pts), kThreads, 0, s, (const int4 *)t4, n_pts, (const int *)first,
+           (const int *)faces_of, c);
+    PAMO_CUDA_TRY(cudaGetLastError());
+    PAMO_CUDA_TRY(cudaMemcpyAsync(h, c, C_COUNT * 8, cudaMemcpyDeviceToHost, s));
+    PAMO_CUDA_TRY(cudaStreamSynchronize(s));
     for (int i = 0; i < C_COUNT; ++i) h_out[i] = (long long)h[i];
-    h_out[C_FACES] = nf;
-    return h[C_ERROR] ? PAMO_ERR_DEVICE : PAMO_OK;
+    return PAMO_OK;
 }
 
 extern "C" int pamo_mesh_distance(const float *d_pa, const int *d_fa, int na, int nfa, const float *d_pb,
@@ -552,47 +607,44 @@ extern "C" int pamo_mesh_distance(const float *d_pa, const int *d_fa, int na, in
     if (cudaGetDevice(&dev) != cudaSuccess) return PAMO_ERR_NO_DEVICE;
     cudaStream_t s = (cudaStream_t)stream;
     PAMO_CUDA_TRY(retain_pool_memory());
-    DeviceBuf pa4((size_t)na * 16, s), fa4((size_t)nfa * 16, s), pb4((size_t)nb * 16, s), fb4((size_t)nfb * 16, s);
-    DeviceBuf part(3 * kHdBlocks * 8, s), err(8, s), bad(C_COUNT * 8, s);
-    if (!pa4.p || !fa4.p || !pb4.p || !fb4.p || !part.p || !err.p || !bad.p) return PAMO_ERR_OOM;
-    launch(k_ck_convert, grid_for(na > nfa ? na : nfa), kThreads, 0, s, d_pa, na, d_fa, nfa, pa4.as<float4>(),
-           fa4.as<int4>());
-    launch(k_ck_convert, grid_for(nb > nfb ? nb : nfb), kThreads, 0, s, d_pb, nb, d_fb, nfb, pb4.as<float4>(),
-           fb4.as<int4>());
-    PAMO_CUDA_TRY(cudaMemsetAsync(bad.p, 0, C_COUNT * 8, s));
-    PAMO_CUDA_TRY(cudaMemsetAsync(err.p, 0, 8, s));
-    launch(k_ck_validate, grid_for(nfa), kThreads, 0, s, (const int4 *)fa4.as<int4>(), nfa, na,
-           bad.as<unsigned long long>());
-    unsigned long long ba[C_COUNT];
-    PAMO_CUDA_TRY(cudaMemcpyAsync(ba, bad.p, C_COUNT * 8, cudaMemcpyDeviceToHost, s));
-    PAMO_CUDA_TRY(cudaStreamSynchronize(s));
-    if (ba[C_BAD_INDEX] || ba[C_DEAD] == (unsigned long long)nfa) return PAMO_ERR_INVALID_ARG;
-    const long long live_a = (long long)nfa - (long long)ba[C_DEAD];  // dead faces of A add no samples
-    PAMO_CUDA_TRY(cudaMemsetAsync(bad.p, 0, C_COUNT * 8, s));
-    launch(k_ck_validate, grid_for(nfb), kThreads, 0, s, (const int4 *)fb4.as<int4>(), nfb, nb,
-           bad.as<unsigned long long>());
-    PAMO_CUDA_TRY(cudaMemcpyAsync(ba, bad.p, C_COUNT * 8, cudaMemcpyDeviceToHost, s));
-    PAMO_CUDA_TRY(cudaStreamSynchronize(s));
-    if (ba[C_BAD_INDEX] || ba[C_DEAD] == (unsigned long long)nfb) return PAMO_ERR_INVALID_ARG;
-    Lbvh b;
-    cudaError_t e = lbvh_build(b, pb4.as<float4>(), fb4.as<int4>(), nfb, s);
-    if (e == cudaSuccess) e = lbvh_refit(b, pb4.as<float4>(), fb4.as<int4>(), nfb, s);
-    if (e != cudaSuccess) {
-        b.release();
-        return map_cuda_error(e);
+    Scratch mem(s);
+    float4 *pa4, *pb4;
+    int4 *fa4, *fb4;
+    double *pm;
+    unsigned long long *bad;
+    unsigned char *tree_mem;
+    for (int pass = 0; pass < 2; ++pass) {
+        pa4 = mem.take<float4>((size_t)na);
+        fa4 = mem.take<int4>((size_t)nfa);
+        pb4 = mem.take<float4>((size_t)nb);
+        fb4 = mem.take<int4>((size_t)nfb);
+        pm = mem.take<double>(3 * kHdBlocks);
+        bad = mem.take<unsigned long long>(2 * C_COUNT);
+        tree_mem = mem.take<unsigned char>(PackedTree::bytes(nfb));
+        if (pass == 0 && !mem.allocate()) return PAMO_ERR_OOM;
     }
-    double *pm = part.as<double>(), *ps = pm + kHdBlocks, *pe = ps + kHdBlocks;
-    launch(k_hd_samples, kHdBlocks, 128, 0, s, (const float4 *)pa4.as<float4>(), (const int4 *)fa4.as<int4>(), nfa,
-           subdiv, (const BvhNode *)b.nodes, (const int *)b.parent, (const int *)b.vals, (const int *)b.scene,
-           (const float4 *)pb4.as<float4>(), (const int4 *)fb4.as<int4>(), pm, ps, pe, err.as<unsigned long long>());
+    double *ps = pm + kHdBlocks, *pe = ps + kHdBlocks;
+    launch(k_ck_convert, grid_for(na > nfa ? na : nfa), kThreads, 0, s, d_pa, na, d_fa, nfa, pa4, fa4);
+    launch(k_ck_convert, grid_for(nb > nfb ? nb : nfb), kThreads, 0, s, d_pb, nb, d_fb, nfb, pb4, fb4);
+    PAMO_CUDA_TRY(cudaMemsetAsync(bad, 0, 2 * C_COUNT * 8, s));
+    launch(k_ck_validate, grid_for(nfa), kThreads, 0, s, (const int4 *)fa4, nfa, na, bad);
+    launch(k_ck_validate, grid_for(nfb), kThreads, 0, s, (const int4 *)fb4, nfb, nb, bad + C_COUNT);
+    unsigned long long hb[2 * C_COUNT];
+    PAMO_CUDA_TRY(cudaMemcpyAsync(hb, bad, sizeof(hb), cudaMemcpyDeviceToHost, s));
+    PAMO_CUDA_TRY(cudaStreamSynchronize(s));
+    if (hb[C_BAD_INDEX] || hb[C_DEAD] == (unsigned long long)nfa) return PAMO_ERR_INVALID_ARG;
+    if (hb[C_COUNT + C_BAD_INDEX] || hb[C_COUNT + C_DEAD] == (unsigned long long)nfb) return PAMO_ERR_INVALID_ARG;
+    const long long live_a = (long long)nfa - (long long)hb[C_DEAD];  // dead faces of A add no samples
+    PackedTree tree;  // its arrays lie in this call's scratch: nothing to release
+    PAMO_CUDA_TRY(tree.place(tree_mem, nfb, s));
+    PAMO_CUDA_TRY(tree_build(tree, pb4, fb4, nfb, s));
+    PAMO_CUDA_TRY(tree_refit(tree, pb4, fb4, nullptr, nullptr, nullptr, nullptr, nfb, s));
+    launch(k_hd_samples, kHdBlocks, kHdThreads, 0, s, (const float4 *)pa4, (const int4 *)fa4, nfa, subdiv, tree.view(),
+           (const float4 *)pb4, pm, ps, pe);
+    PAMO_CUDA_TRY(cudaGetLastError());
     std::vector<double> h(3 * kHdBlocks);
-    unsigned long long herr = 0;
-    e = cudaMemcpyAsync(h.data(), pm, 3 * kHdBlocks * 8, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err.p, 8, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    b.release();
-    if (e != cudaSuccess) return map_cuda_error(e);
-    if (herr) return PAMO_ERR_DEVICE;
+    PAMO_CUDA_TRY(cudaMemcpyAsync(h.data(), pm, 3 * kHdBlocks * 8, cudaMemcpyDeviceToHost, s));
+    PAMO_CUDA_TRY(cudaStreamSynchronize(s));
     double mx = 0.0, sum = 0.0, edge = 0.0;
     for (int i = 0; i < kHdBlocks; ++i) {  // fixed order: the result does not depend on scheduling
         mx = fmax(mx, h[i]);

@@ -3,7 +3,6 @@
 // allocate device memory (see include/pamo_b200.h).
 #include <cstring>
 
-#include "lbvh.cuh"
 #include "ptree.cuh"
 #include "scan.cuh"
 #include "stage2.cuh"
@@ -14,29 +13,18 @@ namespace {
 constexpr int kMaxFaces = 32768;   // limit of this entry point
 constexpr int kMaxVerts = 65536;
 constexpr int kPairsPerFace = 24;  // sizes the pair buffer: 24 * kMaxFaces candidate pairs in total
-constexpr int kTiles = (kMaxFaces + kLbvhSortTile - 1) / kLbvhSortTile;  // the Morton sort's tiles
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // byte offsets inside the scratch array
 constexpr size_t kOffPts = 0;
 constexpr size_t kOffTris = kOffPts + align256(sizeof(float4) * kMaxVerts);
-constexpr size_t kOffKeys = kOffTris + align256(sizeof(int4) * kMaxFaces);
-constexpr size_t kOffKeys2 = kOffKeys + align256(4 * (size_t)kMaxFaces);
-constexpr size_t kOffVals = kOffKeys2 + align256(4 * (size_t)kMaxFaces);
-constexpr size_t kOffVals2 = kOffVals + align256(4 * (size_t)kMaxFaces);
-constexpr size_t kOffHist = kOffVals2 + align256(4 * (size_t)kMaxFaces);
-constexpr size_t kOffHistScratch = kOffHist + align256(4 * (256 * (size_t)kTiles + 64));
-constexpr size_t kOffBoxes = kOffHistScratch + align256(4 * (size_t)scan_scratch_ints(256LL * kTiles));
-constexpr size_t kOffLeaf = kOffBoxes + align256(2 * sizeof(float4) * (size_t)tree_nodes(kMaxFaces));
-constexpr size_t kOffQuery = kOffLeaf + align256(sizeof(int4) * (size_t)kMaxFaces);
-constexpr size_t kOffScene = kOffQuery + align256(4 * (size_t)kMaxFaces);
-constexpr size_t kOffPairs = kOffScene + align256(64);
+constexpr size_t kOffTree = kOffTris + align256(sizeof(int4) * kMaxFaces);
+constexpr size_t kOffQuery = kOffTree + align256(PackedTree::bytes(kMaxFaces));
+constexpr size_t kOffPairs = kOffQuery + align256(4 * (size_t)kMaxFaces);
 constexpr size_t kOffCounters = kOffPairs + align256(sizeof(uint2) * kPairsPerFace * (size_t)kMaxFaces);
 constexpr size_t kOffBad = kOffCounters + align256(sizeof(RoundCounters));
 constexpr size_t kScratchBytes = kOffBad + 256;  // about 10 MB
-static_assert(kOffHistScratch - kOffHist >= 4 * (256 * (size_t)kTiles), "radix histogram area");
-static_assert(kOffPairs - kOffScene >= 64, "scene area");
 
 // Held by every GPU that loads the library, until the process exits.
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
@@ -104,16 +92,7 @@ extern "C" int pamo_self_intersect_noalloc(const float *d_points, const int *d_t
     RoundCounters *cnt = reinterpret_cast<RoundCounters *>(base + kOffCounters);
     int *qlist = reinterpret_cast<int *>(base + kOffQuery);
     PackedTree b;  // views into the scratch array; never released (nothing was allocated)
-    b.cap = kMaxFaces;
-    b.keys = reinterpret_cast<uint32_t *>(base + kOffKeys);
-    b.keys2 = reinterpret_cast<uint32_t *>(base + kOffKeys2);
-    b.vals = reinterpret_cast<int *>(base + kOffVals);
-    b.vals2 = reinterpret_cast<int *>(base + kOffVals2);
-    b.hist = reinterpret_cast<int *>(base + kOffHist);
-    b.hist_scratch = reinterpret_cast<int *>(base + kOffHistScratch);
-    b.boxes = reinterpret_cast<float4 *>(base + kOffBoxes);
-    b.leaf = reinterpret_cast<int4 *>(base + kOffLeaf);
-    b.scene = reinterpret_cast<int *>(base + kOffScene);
+    if (b.place(base + kOffTree, kMaxFaces, s) != cudaSuccess) return PAMO_ERR_DEVICE;
 
     // the array keeps the previous call's contents: reset what must start at zero
     launch(k_na_convert, grid_for(n_pts > n_tris ? n_pts : n_tris), kThreads, 0, s, d_points, n_pts, d_tris, n_tris, p4,

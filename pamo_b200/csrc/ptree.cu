@@ -140,48 +140,45 @@ __global__ void __launch_bounds__(kTreeTile) k_tree_refit(const __grid_constant_
 
 }  // namespace
 
+cudaError_t PackedTree::place(void *memory, long long n, cudaStream_t s)
+{
+    unsigned char *at = static_cast<unsigned char *>(memory);
+    auto take = [&](size_t b) {
+        void *p = at;
+        at += tree_align(b);
+        return p;
+    };
+    keys = static_cast<uint32_t *>(take(4 * (size_t)n));
+    keys2 = static_cast<uint32_t *>(take(4 * (size_t)n));
+    vals = static_cast<int *>(take(4 * (size_t)n));
+    vals2 = static_cast<int *>(take(4 * (size_t)n));
+    hist = static_cast<int *>(take(4 * (size_t)tree_hist(n)));
+    hist_scratch = static_cast<int *>(take(4 * (size_t)scan_scratch_ints(tree_hist(n))));
+    boxes = static_cast<float4 *>(take(2 * sizeof(float4) * (size_t)tree_nodes(n)));
+    leaf = static_cast<int4 *>(take(sizeof(int4) * (size_t)n));
+    scene = static_cast<int *>(take(64));
+    cap = n;
+    leaves = 0;
+    return scan_scratch_init(hist_scratch, scan_scratch_ints(tree_hist(n)), s);
+}
+
 cudaError_t PackedTree::ensure(long long n)
 {
     if (n <= cap && keys) return cudaSuccess;
     release();
     const long long c = n > 16 ? n : 16;
-    const long long tiles = (c + kLbvhSortTile - 1) / kLbvhSortTile;
-    cudaError_t e;
-#define ALLOC(p, bytes)                                          \
-    if ((e = cudaMalloc((void **)&p, (bytes))) != cudaSuccess) { \
-        release();                                               \
-        return e;                                                \
-    }
-    ALLOC(keys, c * 4);
-    ALLOC(keys2, c * 4);
-    ALLOC(vals, c * 4);
-    ALLOC(vals2, c * 4);
-    ALLOC(hist, 256 * tiles * 4 + 64);
-    ALLOC(hist_scratch, scan_scratch_ints(256 * tiles) * 4);
-    ALLOC(boxes, tree_nodes(c) * 2 * sizeof(float4));
-    ALLOC(leaf, c * sizeof(int4));
-    ALLOC(scene, 64);
-#undef ALLOC
-    if ((e = scan_scratch_init(hist_scratch, scan_scratch_ints(256 * tiles))) != cudaSuccess ||
-        (e = cudaMemset(scene, 0, 64)) != cudaSuccess) {
-        release();
+    cudaError_t e = cudaMalloc(&mem, bytes(c));
+    if (e != cudaSuccess) {
+        mem = nullptr;
         return e;
     }
-    cap = c;
-    return cudaSuccess;
+    return place(mem, c, 0);
 }
 
 void PackedTree::release()
 {
-    void *p[] = {keys, keys2, vals, vals2, hist, hist_scratch, boxes, leaf, scene};
-    for (void *q : p)
-        if (q) cudaFree(q);
-    keys = keys2 = nullptr;
-    vals = vals2 = hist = hist_scratch = scene = nullptr;
-    boxes = nullptr;
-    leaf = nullptr;
-    cap = 0;
-    leaves = 0;
+    if (mem) cudaFree(mem);
+    *this = PackedTree{};
 }
 
 TreeView PackedTree::view() const

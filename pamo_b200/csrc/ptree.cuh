@@ -17,6 +17,8 @@
 #pragma once
 
 #include "common.cuh"
+#include "lbvh.cuh"
+#include "scan.cuh"
 
 namespace pamo {
 
@@ -46,7 +48,8 @@ constexpr long long tree_nodes(long long n)  // box slots for n leaves, the leve
 }
 
 struct PackedTree {
-    long long cap = 0;  // faces
+    long long cap = 0;    // faces
+    void *mem = nullptr;  // owned by ensure()
     uint32_t *keys = nullptr, *keys2 = nullptr;
     int *vals = nullptr, *vals2 = nullptr;  // face of each leaf (and the sort's other buffer)
     int *hist = nullptr, *hist_scratch = nullptr;
@@ -56,9 +59,22 @@ struct PackedTree {
     int leaves = 0;        // of the last build
 
     cudaError_t ensure(long long n_faces);
+    // the arrays in the caller's memory (bytes(n) of it, 256-byte aligned) instead
+    cudaError_t place(void *memory, long long n_faces, cudaStream_t s);
+    static constexpr size_t bytes(long long n);
     void release();
     TreeView view() const;
 };
+
+constexpr size_t tree_align(size_t x) { return (x + 255) & ~size_t(255); }
+constexpr long long tree_hist(long long n) { return 256 * ((n + kLbvhSortTile - 1) / kLbvhSortTile); }
+
+constexpr size_t PackedTree::bytes(long long n)
+{
+    return 4 * tree_align(4 * (size_t)n) + tree_align(4 * (size_t)tree_hist(n)) +
+           tree_align(4 * (size_t)scan_scratch_ints(tree_hist(n))) +
+           tree_align(2 * sizeof(float4) * (size_t)tree_nodes(n)) + tree_align(sizeof(int4) * (size_t)n) + 256;
+}
 
 // Orders the faces [0, m) of the round input.  For a batch of meshes, vslot
 // gives each vertex's mesh rank (< n_ranks): a mesh's leaves are then one run,
