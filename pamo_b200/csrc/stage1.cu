@@ -12,14 +12,16 @@
 //      float32, as preprocess_mesh does with numpy (:60-72);
 //   2. unsigned distance (double) from every grid sample ((i + 0.5) / R, ...)
 //      within `band` of a triangle to the nearest triangle, else `band`: one
-//      warp per triangle walks the samples of its box grown by `band` and
+//      warp per triangle walks the samples of its box grown by two voxels and
 //      lowers the sample's squared distance with a 64-bit atomic minimum (the
-//      bits of a non-negative double order like the value);
+//      bits of a non-negative double order like the value).  Two voxels of the
+//      band's three are enough for the same result: see kReach;
 //   3. sign by flood fill: samples farther than half a voxel from every
 //      triangle are free, free samples 6-connected to the grid boundary are
-//      outside; tiles of 8^3 samples propagate "outside" in shared memory
-//      until they settle, and launches repeat until no sample changes
-//      (bounded); the field is +-distance - 0.9/R;
+//      outside; the field is +-distance - 0.9/R.  From here on the grid is bits,
+//      a word per 32 samples of a row: which samples are free, outside, inside
+//      (negative).  Tiles of 8 x 8 rows propagate "outside" in shared memory until
+//      they settle, and launches repeat until no word changes (bounded);
 //   4. dual marching cubes: a sample is inside where the field is negative.
 //      Per cell, the crossed edges pair up on each cube face (an ambiguous face
 //      cuts off each outside corner, a rule both cells sharing the face agree
@@ -27,7 +29,9 @@
 //      one vertex at the mean of its edges' crossing points.  Every crossed
 //      grid edge gives one quad through its four cells' patch vertices, wound
 //      with the normal towards the outside.  Vertices are numbered by cell and
-//      patch, quads by axis and lower sample, through prefix scans;
+//      patch, quads by axis and lower sample, through prefix scans over the
+//      words' counts; a place within a word is a population count.  Distances
+//      (their square roots) are only taken at crossed edges;
 //   5. each quad is split into (0,1,3),(1,2,3) or (0,1,2),(0,2,3), whichever
 //      has the smaller largest corner cosine (double), first-kind quads first
 //      (:95-118); vertices are mapped back to the centred frame in double and
@@ -230,7 +234,18 @@ __device__ double point_tri_d2(D3 p, D3 a, D3 b, D3 c)
     return ddot(d, d);
 }
 
-// One warp per triangle over the samples of its box grown by `band`.  Before
+// How far from a triangle a sample's distance matters, in voxels.  The distance is
+// used where an edge is crossed: between an inside sample A (negative) and a
+// neighbour B outside at 0.9 voxels or more.  A is outside within 0.9 voxels, or
+// near (within 0.5), or free but not reached -- which no neighbour of an outside
+// sample is.  Distances of neighbours differ by at most a voxel, so B's is below
+// 1.9, and both ends lie within 2.  Any value of 2 or more in a farther sample
+// gives the same bits: free, and not within 0.9.  Against the band's 3 voxels a
+// small triangle's box has a third of the samples: 2.7 -> 1.6 ms for 500,000 faces
+// at R = 256, 8.8 -> 4.9 ms for 2,000,000.
+constexpr double kReach = 2.0;
+
+// One warp per triangle over the samples of its box grown by `reach`.  Before
 // the full closest-point computation a sample is skipped when a lower bound of
 // its distance to the triangle -- the distance to the triangle's bounding box,
 // and to its plane -- already reaches the sample's current value (the bounds
@@ -243,13 +258,13 @@ __device__ __forceinline__ double s1_coord(int i, int R, double inv_r)
     return inv_r > 0.0 ? (i + 0.5) * inv_r : (i + 0.5) / R;
 }
 
-__global__ void __launch_bounds__(256, 3) k_s1_udist(const float *tris, int m, int R, double inv_r, double band,
+__global__ void __launch_bounds__(256, 3) k_s1_udist(const float *tris, int m, int R, double inv_r, double reach,
                                                   unsigned long long *field)
 {
     const int lane = threadIdx.x & 31;
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const double band2 = band * band;
+    const double reach2 = reach * reach;
     for (long long t = warp0; t < m; t += nw) {
         const float *T = tris + 9 * t;
         const D3 a = {T[0], T[1], T[2]}, b = {T[3], T[4], T[5]}, c = {T[6], T[7], T[8]};
@@ -257,8 +272,8 @@ __global__ void __launch_bounds__(256, 3) k_s1_udist(const float *tris, int m, i
         const double mn[3] = {fmin(a.x, fmin(b.x, c.x)), fmin(a.y, fmin(b.y, c.y)), fmin(a.z, fmin(b.z, c.z))};
         const double mx[3] = {fmax(a.x, fmax(b.x, c.x)), fmax(a.y, fmax(b.y, c.y)), fmax(a.z, fmax(b.z, c.z))};
         for (int k = 0; k < 3; ++k) {
-            // samples (i + 0.5) / R within [mn - band, mx + band]
-            int l = (int)floor((mn[k] - band) * R - 0.5), h = (int)ceil((mx[k] + band) * R - 0.5);
+            // samples (i + 0.5) / R within [mn - reach, mx + reach]
+            int l = (int)floor((mn[k] - reach) * R - 0.5), h = (int)ceil((mx[k] + reach) * R - 0.5);
             l = max(l, 0);
             h = min(h, R - 1);
             lo[k] = l;
@@ -296,7 +311,7 @@ __global__ void __launch_bounds__(256, 3) k_s1_udist(const float *tris, int m, i
             const double by = fmax(fmax(mn[1] - p.y, 0.0), p.y - mx[1]);
             const double bz = fmax(fmax(mn[2] - p.z, 0.0), p.z - mx[2]);
             const double box2 = bx * bx + by * by + bz * bz;
-            if (box2 >= band2 * (1.0 + 1e-9)) continue;  // the value stays band^2 or lower
+            if (box2 >= reach2 * (1.0 + 1e-9)) continue;  // the value stays reach^2 or more
             unsigned long long *dst = field + gidx(ix, iy, iz, R);
             const double cur = __longlong_as_double((long long)*dst);
             if (box2 > cur * (1.0 + 1e-9)) continue;
@@ -314,173 +329,320 @@ __global__ void k_s1_fill(unsigned long long *a, long long n, unsigned long long
     PAMO_GRID_STRIDE(i, n) a[i] = v;
 }
 
-// squared distance -> unsigned distance (double), free / near / boundary state
-__global__ void k_s1_state(unsigned long long *field, long long n3, int R, double band, uint8_t *state)
+// ------------------------------------------------------------ the grid as bits
+// Word w of row (y, z) holds samples 32 w .. 32 w + 31 of the row.
+struct Bits {
+    int R, W;  // samples and words per row
+    uint32_t *free_, *low, *out, *in;  // free; distance - 0.9/R negative; outside; inside
+};
+
+__device__ __forceinline__ long long row_word(const Bits &B, int y, int z) { return ((long long)z * B.R + y) * B.W; }
+
+// the row's samples that exist in word w
+__device__ __forceinline__ uint32_t valid_bits(int n, int w)
 {
-    PAMO_GRID_STRIDE(i, n3)
-    {
-        const double ud = sqrt(__longlong_as_double((long long)field[i]));
-        field[i] = (unsigned long long)__double_as_longlong(ud);
-        const bool free_ = ud > 0.5 / R;
-        const int x = (int)(i % R), y = (int)((i / R) % R), z = (int)(i / ((long long)R * R));
-        const bool border = x == 0 || y == 0 || z == 0 || x == R - 1 || y == R - 1 || z == R - 1;
-        state[i] = free_ ? (border ? 2 : 1) : 0;
-    }
+    const int left = n - 32 * w;
+    return left >= 32 ? 0xFFFFFFFFu : left <= 0 ? 0u : (1u << left) - 1u;
 }
 
-// ----------------------------------------------------------- 3. flood fill
-constexpr int kTile = 8;
-constexpr int kHalo = kTile + 2;
-
-// One block per 8^3 tile (one thread per sample): free samples next to an
-// outside sample become outside, repeated in shared memory until the tile
-// settles (at most 3 * 8^3 sweeps); a change is reported in dev[4].  Only
-// tiles marked in `dirty_in` (changed, or next to a tile that changed, in the
-// previous launch; all tiles in the first) do the work; a tile that changes
-// marks itself and its six neighbours in `dirty_out`.
-__global__ void __launch_bounds__(kTile * kTile * kTile) k_s1_flood(uint8_t *state, int R, int *dev,
-                                                                   const uint8_t *dirty_in, uint8_t *dirty_out)
+// Free and within-0.9 bits from the squared distances, and the flood's start: the
+// free samples on the grid's boundary.  Most samples hold the fill value, whose
+// bits are known, so few take a square root.
+__global__ void __launch_bounds__(kThreads) k_s1_bits(const unsigned long long *__restrict__ field, Bits B,
+                                                      unsigned long long fill)
 {
-    __shared__ uint8_t s[kHalo][kHalo][kHalo];
-    __shared__ int changed, any_change;
-    const int tpr = (R + kTile - 1) / kTile;
-    if (!dirty_in[blockIdx.x]) return;
-    const int bx = blockIdx.x % tpr, by = (blockIdx.x / tpr) % tpr, bz = blockIdx.x / (tpr * tpr);
-    const int tx = threadIdx.x % kTile, ty = (threadIdx.x / kTile) % kTile, tz = threadIdx.x / (kTile * kTile);
-    // the tile with its one-sample halo (outside the grid: near, never spreads)
-    for (int i = threadIdx.x; i < kHalo * kHalo * kHalo; i += blockDim.x) {
-        const int hx = i % kHalo, hy = (i / kHalo) % kHalo, hz = i / (kHalo * kHalo);
-        const int gx = bx * kTile + hx - 1, gy = by * kTile + hy - 1, gz = bz * kTile + hz - 1;
-        uint8_t v = 0;
-        if (gx >= 0 && gy >= 0 && gz >= 0 && gx < R && gy < R && gz < R) v = state[gidx(gx, gy, gz, R)];
-        s[hz][hy][hx] = v;
-    }
-    if (threadIdx.x == 0) any_change = 0;
-    const int gx = bx * kTile + tx, gy = by * kTile + ty, gz = bz * kTile + tz;
-    const bool in_grid = gx < R && gy < R && gz < R;
-    const int x = tx + 1, y = ty + 1, z = tz + 1;
-    bool any = false;
-    __syncthreads();
-    for (int sweep = 0; sweep < 3 * kTile * kTile * kTile; ++sweep) {
-        if (threadIdx.x == 0) changed = 0;
-        __syncthreads();
-        if (in_grid && s[z][y][x] == 1 &&
-            (s[z][y][x - 1] == 2 || s[z][y][x + 1] == 2 || s[z][y - 1][x] == 2 || s[z][y + 1][x] == 2 ||
-             s[z - 1][y][x] == 2 || s[z + 1][y][x] == 2)) {
-            s[z][y][x] = 2;
-            changed = 1;
-            any = true;
+    constexpr int kBatch = 4;  // words a warp has in flight
+    const int R = B.R, lane = threadIdx.x & 31;
+    const long long words = (long long)R * R * B.W;
+    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long q = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kBatch; q < words;
+         q += warps * kBatch) {
+        unsigned long long v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const long long row = (q + k) / B.W;
+            const int x = (int)((q + k) % B.W) * 32 + lane;
+            v[k] = q + k < words && x < R ? field[row * R + x] : fill;
         }
-        __syncthreads();
-        if (!changed) break;
-    }
-    if (any) {
-        state[gidx(gx, gy, gz, R)] = 2;
-        any_change = 1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && any_change) {
-        atomicExch(&dev[4], 1);
-        dirty_out[blockIdx.x] = 1;
-        if (bx > 0) dirty_out[blockIdx.x - 1] = 1;
-        if (bx + 1 < tpr) dirty_out[blockIdx.x + 1] = 1;
-        if (by > 0) dirty_out[blockIdx.x - tpr] = 1;
-        if (by + 1 < tpr) dirty_out[blockIdx.x + tpr] = 1;
-        if (bz > 0) dirty_out[blockIdx.x - tpr * tpr] = 1;
-        if (bz + 1 < tpr) dirty_out[blockIdx.x + tpr * tpr] = 1;
-    }
-}
-
-__global__ void k_s1_field(unsigned long long *field, const uint8_t *state, long long n3, int R)
-{
-    PAMO_GRID_STRIDE(i, n3)
-    {
-        const double ud = __longlong_as_double((long long)field[i]);
-        const double v = (state[i] == 2 ? ud : -ud) - 0.9 / R;
-        field[i] = (unsigned long long)__double_as_longlong(v);
-    }
-}
-
-// ------------------------------------------------------- 4. dual marching cubes
-__device__ __forceinline__ double fval(const unsigned long long *field, int x, int y, int z, int R)
-{
-    return __longlong_as_double((long long)field[gidx(x, y, z, R)]);
-}
-
-__device__ __forceinline__ int cell_case(const unsigned long long *field, int x, int y, int z, int R)
-{
-    int cs = 0;
-    for (int c = 0; c < 8; ++c) cs |= (fval(field, x + (c & 1), y + ((c >> 1) & 1), z + ((c >> 2) & 1), R) < 0.0) << c;
-    return cs;
-}
-
-__global__ void k_s1_cells(const unsigned long long *field, int R, int *cell_cnt)
-{
-    const int C = R - 1;
-    PAMO_GRID_STRIDE(i, (long long)C * C * C)
-    {
-        const int x = (int)(i % C), y = (int)((i / C) % C), z = (int)(i / ((long long)C * C));
-        cell_cnt[i] = c_npatch[cell_case(field, x, y, z, R)];
-    }
-}
-
-// the patch vertices of each cell: the mean of its edges' crossing points (edge
-// order), in sample-index coordinates, mapped to the centred frame
-__global__ void k_s1_verts(const unsigned long long *field, int R, const int *cell_first, double band, double margin,
-                           double tmax, const int *dev, float *verts)
-{
-    const int C = R - 1;
-    double lo[3];
-    for (int k = 0; k < 3; ++k) lo[k] = (double)ordered_to_float(dev[k]);
-    PAMO_GRID_STRIDE(i, (long long)C * C * C)
-    {
-        const int first = cell_first[i], np = cell_first[i + 1] - first;
-        if (np == 0) continue;
-        const int x = (int)(i % C), y = (int)((i / C) % C), z = (int)(i / ((long long)C * C));
-        const int cs = cell_case(field, x, y, z, R);
-        double sx[4] = {0, 0, 0, 0}, sy[4] = {0, 0, 0, 0}, sz[4] = {0, 0, 0, 0};
-        int cnt[4] = {0, 0, 0, 0};
-        for (int e = 0; e < 12; ++e) {
-            const int p = c_patch[cs][e];
-            if (p < 0) continue;
-            int a, b;
-            edge_corners(e, a, b);
-            const int ax = x + (a & 1), ay = y + ((a >> 1) & 1), az = z + ((a >> 2) & 1);
-            const int bx = x + (b & 1), by = y + ((b >> 1) & 1), bz = z + ((b >> 2) & 1);
-            const double da = fval(field, ax, ay, az, R), db = fval(field, bx, by, bz, R);
-            const double t = da / (da - db);
-            sx[p] += ax + t * (double)(bx - ax);
-            sy[p] += ay + t * (double)(by - ay);
-            sz[p] += az + t * (double)(bz - az);
-            cnt[p]++;
-        }
-        for (int p = 0; p < np; ++p) {
-            const double v[3] = {sx[p] / cnt[p], sy[p] / cnt[p], sz[p] / cnt[p]};
-            for (int k = 0; k < 3; ++k) {
-                const double xn = (v[k] + 0.5) / R;
-                verts[3LL * (first + p) + k] = (float)((xn * margin - band) * tmax + lo[k]);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            if (q + k >= words) break;
+            const long long row = (q + k) / B.W;
+            const int w = (int)((q + k) % B.W), x = w * 32 + lane;
+            bool fr = true, lo = false;
+            if (v[k] != fill) {
+                const double ud = sqrt(__longlong_as_double((long long)v[k]));
+                fr = ud > 0.5 / R;
+                lo = ud - 0.9 / R < 0.0;
+            }
+            const uint32_t f = __ballot_sync(0xffffffffu, fr && x < R), l = __ballot_sync(0xffffffffu, lo && x < R);
+            if (lane == 0) {
+                const int y = (int)(row % R), z = (int)(row / R);
+                uint32_t border = 0;
+                if (y == 0 || z == 0 || y == R - 1 || z == R - 1) border = 0xFFFFFFFFu;
+                if (w == 0) border |= 1u;
+                if (w == (R - 1) >> 5) border |= 1u << ((R - 1) & 31);
+                B.free_[q + k] = f;
+                B.low[q + k] = l;
+                B.out[q + k] = f & border;
             }
         }
     }
 }
 
-// crossed grid edges whose four cells exist (every crossed edge, given the
-// grid's outer layer is outside): 1 per axis-major edge slot
-__global__ void k_s1_edges(const unsigned long long *field, int R, int *edge_cnt)
+// ----------------------------------------------------------- 3. flood fill
+constexpr int kTile = 8;
+constexpr int kMaxWords = 32;  // R <= 1024
+
+// the bits of o spread along the runs of f they lie in
+__device__ __forceinline__ uint32_t spread(uint32_t o, uint32_t f)
 {
-    const long long n3 = (long long)R * R * R;
-    PAMO_GRID_STRIDE(i, 3 * n3)
+    uint32_t up = f, down = f;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        o |= (up & (o << k)) | (down & (o >> k));
+        up &= up << k;
+        down &= down >> k;
+    }
+    return o;
+}
+
+// One block per tile of 8 x 8 whole rows: free samples next to an outside sample
+// become outside, repeated in shared memory until the tile settles (each sweep
+// but the last adds a bit, so it does); a change is reported in dev[4].  Only
+// tiles marked in `dirty_in` (changed, or next to a tile that changed, in the
+// previous launch; all tiles in the first) do the work; a tile that changes marks
+// itself and its four neighbours in `dirty_out`.  Rows start outside at both
+// ends, so a few launches settle the grid.  With a byte per sample in 8^3 tiles a
+// launch took 66 us at R = 256; this one takes 5.
+__global__ void __launch_bounds__(kThreads) k_s1_flood(Bits B, int *dev, const uint8_t *dirty_in, uint8_t *dirty_out)
+{
+    __shared__ uint32_t o[(kTile + 2) * (kTile + 2)][kMaxWords];
+    const int R = B.R, W = B.W, tpr = (R + kTile - 1) / kTile;
+    if (!dirty_in[blockIdx.x]) return;
+    const int by = blockIdx.x % tpr, bz = blockIdx.x / tpr;
+    for (int i = threadIdx.x; i < (kTile + 2) * (kTile + 2) * W; i += blockDim.x) {
+        const int r = i / W, w = i % W;
+        const int y = by * kTile + r % (kTile + 2) - 1, z = bz * kTile + r / (kTile + 2) - 1;
+        o[r][w] = y >= 0 && z >= 0 && y < R && z < R ? B.out[row_word(B, y, z) + w] : 0;
+    }
+    __syncthreads();
+    bool any = false;
+    for (int sweep = 0; sweep <= 32 * kTile * kTile * W; ++sweep) {
+        int changed = 0;
+        for (int i = threadIdx.x; i < kTile * kTile * W; i += blockDim.x) {
+            const int w = i % W, ty = i / W % kTile, tz = i / W / kTile;
+            const int y = by * kTile + ty, z = bz * kTile + tz, r = (tz + 1) * (kTile + 2) + ty + 1;
+            if (y >= R || z >= R) continue;
+            const uint32_t f = B.free_[row_word(B, y, z) + w], was = o[r][w];
+            uint32_t next = o[r - 1][w] | o[r + 1][w] | o[r - kTile - 2][w] | o[r + kTile + 2][w];
+            if (w > 0) next |= o[r][w - 1] >> 31;
+            if (w + 1 < W) next |= o[r][w + 1] << 31;
+            const uint32_t now = spread(was | (next & f), f);
+            if (now != was) {
+                o[r][w] = now;
+                changed = 1;
+            }
+        }
+        changed = __syncthreads_or(changed);
+        if (!changed) break;
+        any = true;
+    }
+    if (!any) return;
+    for (int i = threadIdx.x; i < kTile * kTile * W; i += blockDim.x) {
+        const int w = i % W, ty = i / W % kTile, tz = i / W / kTile;
+        const int y = by * kTile + ty, z = bz * kTile + tz;
+        if (y < R && z < R) B.out[row_word(B, y, z) + w] = o[(tz + 1) * (kTile + 2) + ty + 1][w];
+    }
+    if (threadIdx.x == 0) {
+        atomicExch(&dev[4], 1);
+        dirty_out[blockIdx.x] = 1;
+        if (by > 0) dirty_out[blockIdx.x - 1] = 1;
+        if (by + 1 < tpr) dirty_out[blockIdx.x + 1] = 1;
+        if (bz > 0) dirty_out[blockIdx.x - tpr] = 1;
+        if (bz + 1 < tpr) dirty_out[blockIdx.x + tpr] = 1;
+    }
+}
+
+// inside: the field (outside ? d : -d) - 0.9/R is negative
+__global__ void k_s1_inside(Bits B)
+{
+    PAMO_GRID_STRIDE(i, (long long)B.R * B.R * B.W)
+        B.in[i] = (~B.out[i] | B.low[i]) & valid_bits(B.R, (int)(i % B.W));
+}
+
+// ------------------------------------------------------- 4. dual marching cubes
+__device__ __forceinline__ bool bit_at(const uint32_t *b, const Bits &B, int x, int y, int z)
+{
+    return b[row_word(B, y, z) + (x >> 5)] >> (x & 31) & 1u;
+}
+
+// the field at a sample
+__device__ __forceinline__ double fval(const unsigned long long *field, const Bits &B, int x, int y, int z)
+{
+    const double ud = sqrt(__longlong_as_double((long long)field[gidx(x, y, z, B.R)]));
+    return (bit_at(B.out, B, x, y, z) ? ud : -ud) - 0.9 / B.R;
+}
+
+__device__ __forceinline__ int cell_case(const Bits &B, int x, int y, int z)
+{
+    int cs = 0;
+    for (int c = 0; c < 8; ++c) cs |= (int)bit_at(B.in, B, x + (c & 1), y + ((c >> 1) & 1), z + ((c >> 2) & 1)) << c;
+    return cs;
+}
+
+// Word w of row (y, z) of the (R - 1)^3 cells: which cells have at least one, two,
+// three, four patches, and the number of patches before the word (first).
+struct Cells {
+    int C, W;
+    uint32_t *has[4];
+    int *first;
+};
+
+__device__ __forceinline__ long long cell_word(const Cells &K, int x, int y, int z)
+{
+    return ((long long)z * K.C + y) * K.W + (x >> 5);
+}
+
+// the number of the cell's first patch
+__device__ __forceinline__ int cell_first(const Cells &K, int x, int y, int z)
+{
+    const long long i = cell_word(K, x, y, z);
+    const uint32_t below = (1u << (x & 31)) - 1u;
+    int n = K.first[i];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) n += __popc(K.has[k][i] & below);
+    return n;
+}
+
+__global__ void k_s1_cells(Bits B, Cells K)
+{
+    PAMO_GRID_STRIDE(i, (long long)K.C * K.C * K.W)
     {
-        const int ax = (int)(i / n3);
-        const long long g = i % n3;
-        const int x = (int)(g % R), y = (int)((g / R) % R), z = (int)(g / ((long long)R * R));
-        int c = 0;
-        const int x2 = x + (ax == 0), y2 = y + (ax == 1), z2 = z + (ax == 2);
+        const int w = (int)(i % K.W), y = (int)(i / K.W % K.C), z = (int)(i / ((long long)K.W * K.C));
+        uint32_t any = 0, all = 0xFFFFFFFFu;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const long long q = row_word(B, y + (r & 1), z + (r >> 1)) + w;
+            const uint32_t a = B.in[q], b = w + 1 < B.W ? B.in[q + 1] : 0u;
+            const uint32_t s = (a >> 1) | (b << 31);
+            any |= a | s;
+            all &= a & s;
+        }
+        uint32_t has[4] = {0, 0, 0, 0};
+        int n = 0;
+        for (uint32_t todo = any & ~all & valid_bits(K.C, w); todo; todo &= todo - 1) {
+            const int b = __ffs(todo) - 1;
+            const int np = c_npatch[cell_case(B, 32 * w + b, y, z)];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (np > k) has[k] |= 1u << b;
+            n += np;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) K.has[k][i] = has[k];
+        K.first[i] = n;  // counts: scanned in place
+    }
+}
+
+// The numbered patches and quads as lists, so that the kernels that compute them
+// have one of each in every thread: patch k's cell and which of its patches (4 cell
+// + patch), quad q's word and bit (32 word + bit).  Warps that looked for set bits
+// among their words instead held ten lanes busy and a surface's words fell to few
+// of them (k_s1_verts and k_s1_quads 0.75 ms together at R = 256).
+__global__ void k_s1_lists(Cells K, const uint32_t *edge_mask, const int *edge_first, long long edge_words,
+                           uint32_t *patches, uint32_t *quads)
+{
+    const long long cwords = (long long)K.C * K.C * K.W;
+    PAMO_GRID_STRIDE(i, cwords + edge_words)
+    {
+        if (i < cwords) {
+            int n = K.first[i];
+            const uint32_t h0 = K.has[0][i];
+            if (!h0) continue;
+            const uint32_t h1 = K.has[1][i], h2 = K.has[2][i], h3 = K.has[3][i];
+            const uint32_t cell0 = (uint32_t)(i / K.W * K.C + (i % K.W) * 32);
+            for (uint32_t todo = h0; todo; todo &= todo - 1) {
+                const int b = __ffs(todo) - 1;
+                const int np = 1 + (h1 >> b & 1) + (h2 >> b & 1) + (h3 >> b & 1);
+                for (int p = 0; p < np; ++p) patches[n++] = 4 * (cell0 + b) + p;
+            }
+        } else {
+            const long long j = i - cwords;
+            int n = edge_first[j];
+            for (uint32_t todo = edge_mask[j]; todo; todo &= todo - 1)
+                quads[n++] = (uint32_t)(32 * j) + (__ffs(todo) - 1);
+        }
+    }
+}
+
+// the patch vertices: the mean of a patch's edges' crossing points (edge order),
+// in sample-index coordinates, mapped to the centred frame
+__global__ void __launch_bounds__(kThreads) k_s1_verts(const unsigned long long *field, Bits B,
+                                                       const uint32_t *patches, int nv, double band, double margin,
+                                                       double tmax, const int *dev, float *verts)
+{
+    const int R = B.R, C = R - 1;
+    double lo[3];
+    for (int k = 0; k < 3; ++k) lo[k] = (double)ordered_to_float(dev[k]);
+    PAMO_GRID_STRIDE(i, nv)
+    {
+        const uint32_t code = patches[i], cell = code >> 2;
+        const int p = (int)(code & 3u);
+        const int x = (int)(cell % (uint32_t)C), y = (int)(cell / (uint32_t)C % (uint32_t)C),
+                  z = (int)(cell / ((uint32_t)C * (uint32_t)C));
+        const int cs = cell_case(B, x, y, z);
+        double d[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) d[c] = fval(field, B, x + (c & 1), y + ((c >> 1) & 1), z + ((c >> 2) & 1));
+        double sx = 0, sy = 0, sz = 0;
+        int cnt = 0;
+#pragma unroll
+        for (int e = 0; e < 12; ++e) {
+            if (c_patch[cs][e] != p) continue;
+            int a, b;
+            edge_corners(e, a, b);
+            const int ax = x + (a & 1), ay = y + ((a >> 1) & 1), az = z + ((a >> 2) & 1);
+            const int bx = x + (b & 1), by = y + ((b >> 1) & 1), bz = z + ((b >> 2) & 1);
+            const double t = d[a] / (d[a] - d[b]);
+            sx += ax + t * (double)(bx - ax);
+            sy += ay + t * (double)(by - ay);
+            sz += az + t * (double)(bz - az);
+            cnt++;
+        }
+        const double v[3] = {sx / cnt, sy / cnt, sz / cnt};
+        for (int k = 0; k < 3; ++k) {
+            const double xn = (v[k] + 0.5) / R;
+            verts[3LL * i + k] = (float)((xn * margin - band) * tmax + lo[k]);
+        }
+    }
+}
+
+// Crossed grid edges whose four cells exist (every crossed edge, given the grid's
+// outer layer is outside), by axis and lower sample: a mask per word of samples
+// and its count (scanned in place).
+__global__ void k_s1_edges(Bits B, uint32_t *mask, int *first)
+{
+    const int R = B.R;
+    const long long words = (long long)R * R * B.W;
+    PAMO_GRID_STRIDE(i, 3 * words)
+    {
+        const int ax = (int)(i / words);
+        const long long g = i % words;
+        const int w = (int)(g % B.W), y = (int)(g / B.W % R), z = (int)(g / ((long long)B.W * R));
         // the four cells need the two other coordinates in [1, R - 2]
-        const bool room = x2 < R && y2 < R && z2 < R && (ax == 0 || (x >= 1 && x <= R - 2)) &&
-                          (ax == 1 || (y >= 1 && y <= R - 2)) && (ax == 2 || (z >= 1 && z <= R - 2));
-        if (room) c = (fval(field, x, y, z, R) < 0.0) != (fval(field, x2, y2, z2, R) < 0.0);
-        edge_cnt[i] = c;
+        const bool room = (ax == 1 ? y + 1 < R : y >= 1 && y <= R - 2) && (ax == 2 ? z + 1 < R : z >= 1 && z <= R - 2);
+        uint32_t m = 0;
+        if (room) {
+            const uint32_t a = B.in[g];
+            uint32_t b;
+            if (ax == 0) b = (a >> 1) | (w + 1 < B.W ? B.in[g + 1] << 31 : 0u);
+            else b = B.in[g + (ax == 1 ? (long long)B.W : (long long)B.W * R)];
+            m = (a ^ b) & valid_bits(R - 1, w);  // x <= R - 2
+            if (ax != 0 && w == 0) m &= ~1u;
+        }
+        mask[i] = m;
+        first[i] = __popc(m);
     }
 }
 
@@ -503,35 +665,32 @@ __device__ __forceinline__ double max_cos(const float *v, int i0, int i1, int i2
 // one quad per crossed edge, through the patch vertices of its four cells
 // (counterclockwise seen from the +axis side when the lower sample is inside),
 // and whether it splits the first way
-__global__ void k_s1_quads(const unsigned long long *field, int R, const int *edge_first, const int *cell_first,
-                           const float *verts, int4 *quads, int *q_first)
+__global__ void __launch_bounds__(kThreads) k_s1_quads(Bits B, Cells K, const uint32_t *list, int nq,
+                                                       const float *verts, int4 *quads, int *q_first)
 {
-    const long long n3 = (long long)R * R * R;
-    const int C = R - 1;
-    PAMO_GRID_STRIDE(i, 3 * n3)
+    const int R = B.R;
+    const uint32_t words = (uint32_t)((long long)R * R * B.W);
+    PAMO_GRID_STRIDE(q, nq)
     {
-        const int q = edge_first[i];
-        if (edge_first[i + 1] == q) continue;
-        const int ax = (int)(i / n3);
-        const long long g = i % n3;
-        const int x = (int)(g % R), y = (int)((g / R) % R), z = (int)(g / ((long long)R * R));
+        const uint32_t word = list[q] >> 5;
+        const int ax = (int)(word / words);
+        const uint32_t g = word % words;
+        const int x = (int)(g % B.W * 32 + (list[q] & 31u)), y = (int)(g / B.W % R), z = (int)(g / ((uint32_t)B.W * R));
         // the other two axes in cyclic order (b, c) with b x c = the edge's axis
         const int bax = (ax + 1) % 3, cax = (ax + 2) % 3;
-        const int ob[4] = {0, -1, -1, 0}, oc[4] = {0, 0, -1, -1};
         int vs[4];
+#pragma unroll
         for (int k = 0; k < 4; ++k) {
-            int cc[3] = {x, y, z};
-            cc[bax] += ob[k];
-            cc[cax] += oc[k];
+            const int ob = k == 1 || k == 2 ? -1 : 0, oc = k >= 2 ? -1 : 0;
+            const int cx = x + (bax == 0 ? ob : 0) + (cax == 0 ? oc : 0);
+            const int cy = y + (bax == 1 ? ob : 0) + (cax == 1 ? oc : 0);
+            const int cz = z + (bax == 2 ? ob : 0) + (cax == 2 ? oc : 0);
             // the edge's corners inside this cell
-            const int l[3] = {x - cc[0], y - cc[1], z - cc[2]};
-            const int ca = l[0] + 2 * l[1] + 4 * l[2];
+            const int ca = (x - cx) + 2 * (y - cy) + 4 * (z - cz);
             const int e = ax * 4 + (ax == 0 ? (ca >> 1) : (ax == 1 ? ((ca & 1) | ((ca >> 1) & 2)) : (ca & 3)));
-            const long long cell = ((long long)cc[2] * C + cc[1]) * C + cc[0];
-            const int cs = cell_case(field, cc[0], cc[1], cc[2], R);
-            vs[k] = cell_first[cell] + c_patch[cs][e];
+            vs[k] = cell_first(K, cx, cy, cz) + c_patch[cell_case(B, cx, cy, cz)][e];
         }
-        const bool lower_inside = fval(field, x, y, z, R) < 0.0;
+        const bool lower_inside = bit_at(B.in, B, x, y, z);
         const int4 qd = lower_inside ? make_int4(vs[0], vs[1], vs[2], vs[3]) : make_int4(vs[3], vs[2], vs[1], vs[0]);
         quads[q] = qd;
         const double a1 = fmax(max_cos(verts, qd.x, qd.y, qd.w), max_cos(verts, qd.y, qd.z, qd.w));
@@ -540,8 +699,9 @@ __global__ void k_s1_quads(const unsigned long long *field, int R, const int *ed
     }
 }
 
-__global__ void k_s1_faces(const int4 *quads, const int *flag, const int *pos, int nq, int n1, int *faces)
+__global__ void k_s1_faces(const int4 *quads, const int *flag, const int *pos, int nq, const int *n_first, int *faces)
 {
+    const int n1 = *n_first;
     PAMO_GRID_STRIDE(q, nq)
     {
         const int4 d = quads[q];
@@ -579,46 +739,52 @@ static_assert(kEdgeCorners[5][0] == 1 && kEdgeCorners[5][1] == 3 && kEdgeCorners
 
 void Stage1::release()
 {
-    void *p[] = {tris, field, state, cell_cnt, edge_cnt, scan_cells, scan_edges, scan_quads, quads, q_first, verts,
-                 faces, dev, mean_dev, tile_dirty};
+    void *p[] = {tris, field, bits, cell_bits, cell_first, edge_bits, edge_first, scan_cells, scan_edges, scan_quads,
+                 quads, q_first, q_pos, verts, faces, dev, mean_dev, tile_dirty,
+                 patch_list, quad_list};
     for (void *x : p)
         if (x) cudaFree(x);
     if (h_dev) cudaFreeHost(h_dev);
     tris = nullptr;
     field = nullptr;
-    state = nullptr;
-    cell_cnt = edge_cnt = scan_cells = scan_edges = scan_quads = nullptr;
+    bits = cell_bits = edge_bits = patch_list = quad_list = nullptr;
+    cell_first = edge_first = scan_cells = scan_edges = scan_quads = nullptr;
     quads = nullptr;
-    q_first = nullptr;
+    q_first = q_pos = nullptr;
     verts = nullptr;
     faces = nullptr;
     dev = h_dev = nullptr;
     mean_dev = nullptr;
     tile_dirty = nullptr;
-    cap_tris = cap_grid = cap_cells = cap_edges = cap_verts = cap_quads = cap_tiles = 0;
+    cap_tris = cap_grid = cap_words = cap_verts = cap_quads = cap_tiles = 0;
 }
 
 int Stage1::ensure(long long m, int R_)
 {
-    const long long n3 = (long long)R_ * R_ * R_, c3 = (long long)(R_ - 1) * (R_ - 1) * (R_ - 1);
-    const long long tpr = (R_ + kTile - 1) / kTile, nt = tpr * tpr * tpr;
-    if (m <= cap_tris && n3 <= cap_grid && nt <= cap_tiles && dev) return PAMO_OK;
-    const long long ctl = nt > cap_tiles ? nt : cap_tiles;
+    const long long n3 = (long long)R_ * R_ * R_;
+    const long long tpr = (R_ + kTile - 1) / kTile, nt = tpr * tpr;
+    const long long nw = (long long)R_ * R_ * ((R_ + 31) / 32);  // words of the grid; the cells have fewer
+    if (m <= cap_tris && n3 <= cap_grid && nt <= cap_tiles && nw <= cap_words && dev) return PAMO_OK;
+    const long long ctl = nt > cap_tiles ? nt : cap_tiles, cw = nw > cap_words ? nw : cap_words;
     const long long cm = m > cap_tris ? m : cap_tris, cg = n3 > cap_grid ? n3 : cap_grid;
-    const long long cc = c3 > cap_cells ? c3 : cap_cells;
-    void *keep_v = verts, *keep_f = faces, *keep_q = quads, *keep_qf = q_first, *keep_sq = scan_quads;
+    void *keep_v = verts, *keep_f = faces, *keep_q = quads, *keep_qf = q_first, *keep_qp = q_pos, *keep_sq = scan_quads;
+    void *keep_pl = patch_list, *keep_ql = quad_list;
     const long long kv = cap_verts, kq = cap_quads;
     verts = nullptr;
     faces = nullptr;
     quads = nullptr;
-    q_first = nullptr;
+    q_first = q_pos = nullptr;
     scan_quads = nullptr;
+    patch_list = quad_list = nullptr;
     release();
     verts = (float *)keep_v;
     faces = (int *)keep_f;
     quads = (int4 *)keep_q;
     q_first = (int *)keep_qf;
+    q_pos = (int *)keep_qp;
     scan_quads = (int *)keep_sq;
+    patch_list = (uint32_t *)keep_pl;
+    quad_list = (uint32_t *)keep_ql;
     cap_verts = kv;
     cap_quads = kq;
 #define S1A(ptr, bytes)                                                    \
@@ -628,12 +794,14 @@ int Stage1::ensure(long long m, int R_)
     }
     S1A(tris, 9 * 4 * (cm + 1));
     S1A(field, 8 * cg);
-    S1A(state, cg);
+    S1A(bits, 4 * 4 * cw);
     S1A(tile_dirty, 2 * ctl);
-    S1A(cell_cnt, 4 * (cc + 1));
-    S1A(edge_cnt, 4 * (3 * cg + 1));
-    S1A(scan_cells, 4 * scan_scratch_ints(cc + 1));
-    S1A(scan_edges, 4 * scan_scratch_ints(3 * cg + 1));
+    S1A(cell_bits, 4 * 4 * cw);
+    S1A(cell_first, 4 * cw);
+    S1A(edge_bits, 3 * 4 * cw);
+    S1A(edge_first, 3 * 4 * cw);
+    S1A(scan_cells, 4 * scan_scratch_ints(cw));
+    S1A(scan_edges, 4 * scan_scratch_ints(3 * cw));
     S1A(dev, 64);
     S1A(mean_dev, 16);
 #undef S1A
@@ -641,16 +809,15 @@ int Stage1::ensure(long long m, int R_)
         release();
         return PAMO_ERR_OOM;
     }
-    if (scan_scratch_init(scan_cells, scan_scratch_ints(cc + 1)) != cudaSuccess ||
-        scan_scratch_init(scan_edges, scan_scratch_ints(3 * cg + 1)) != cudaSuccess) {
+    if (scan_scratch_init(scan_cells, scan_scratch_ints(cw)) != cudaSuccess ||
+        scan_scratch_init(scan_edges, scan_scratch_ints(3 * cw)) != cudaSuccess) {
         release();
         return PAMO_ERR_OOM;
     }
     cap_tris = cm;
     cap_grid = cg;
     cap_tiles = ctl;
-    cap_cells = cc;
-    cap_edges = 3 * cg;
+    cap_words = cw;
     return PAMO_OK;
 }
 
@@ -658,28 +825,35 @@ int Stage1::ensure_out(long long nv, long long nq)
 {
     if (nv > cap_verts || !verts) {
         if (verts) cudaFree(verts);
+        if (patch_list) cudaFree(patch_list);
         verts = nullptr;
+        patch_list = nullptr;
         cap_verts = 0;
         const long long c = nv + nv / 8 + 64;
-        if (cudaMalloc((void **)&verts, (size_t)c * 12) != cudaSuccess) return PAMO_ERR_OOM;
+        if (cudaMalloc((void **)&verts, (size_t)c * 12) != cudaSuccess ||
+            cudaMalloc((void **)&patch_list, (size_t)c * 4) != cudaSuccess)
+            return PAMO_ERR_OOM;
         cap_verts = c;
     }
     if (nq > cap_quads || !quads) {
-        void *p[] = {quads, q_first, faces, scan_quads};
+        void *p[] = {quads, q_first, q_pos, faces, scan_quads, quad_list};
         for (void *x : p)
             if (x) cudaFree(x);
         quads = nullptr;
-        q_first = nullptr;
+        q_first = q_pos = nullptr;
         faces = nullptr;
         scan_quads = nullptr;
+        quad_list = nullptr;
         cap_quads = 0;
         const long long c = nq + nq / 8 + 64;
         if (cudaMalloc((void **)&quads, (size_t)c * 16) != cudaSuccess ||
-            cudaMalloc((void **)&q_first, (size_t)(c + 1) * 4) != cudaSuccess ||
+            cudaMalloc((void **)&q_first, (size_t)c * 4) != cudaSuccess ||
+            cudaMalloc((void **)&q_pos, (size_t)c * 4) != cudaSuccess ||
+            cudaMalloc((void **)&quad_list, (size_t)c * 4) != cudaSuccess ||
             cudaMalloc((void **)&faces, (size_t)c * 24) != cudaSuccess ||
-            cudaMalloc((void **)&scan_quads, (size_t)scan_scratch_ints(c + 1) * 4) != cudaSuccess)
+            cudaMalloc((void **)&scan_quads, (size_t)scan_scratch_ints(c) * 4) != cudaSuccess)
             return PAMO_ERR_OOM;
-        if (scan_scratch_init(scan_quads, scan_scratch_ints(c + 1)) != cudaSuccess) return PAMO_ERR_OOM;
+        if (scan_scratch_init(scan_quads, scan_scratch_ints(c)) != cudaSuccess) return PAMO_ERR_OOM;
         cap_quads = c;
     }
     return PAMO_OK;
@@ -703,7 +877,7 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
     S1_TRY(cudaMemcpyToSymbolAsync(c_patch, h_patch, sizeof(h_patch), 0, cudaMemcpyHostToDevice, s));
     S1_TRY(cudaMemcpyToSymbolAsync(c_npatch, h_npatch, sizeof(h_npatch), 0, cudaMemcpyHostToDevice, s));
     const double band = 3.0 / R, margin = band * 2 + 1;
-    const long long n3 = (long long)R * R * R, c3 = (long long)(R - 1) * (R - 1) * (R - 1);
+    const long long n3 = (long long)R * R * R;
     // 1. normalise
     if (S.prof) S.prof->begin(PH_S1_PREP, s);
     launch(k_s1_dev_init, 1, 32, 0, s, S.dev);
@@ -713,31 +887,31 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
            (float)band, (float)margin, S.tris);
     // 2. unsigned distance: squared distances start at band^2 (bits of a double)
     if (S.prof) S.prof->begin(PH_S1_DIST, s);
-    {
-        const double b2 = band * band;
-        unsigned long long bits;
-        memcpy(&bits, &b2, 8);
-        // fill by a kernel: cudaMemset only sets bytes
-        launch(k_s1_fill, grid_for(n3), kThreads, 0, s, S.field, n3, bits);
-    }
+    const double b2 = band * band;
+    unsigned long long fill;
+    memcpy(&fill, &b2, 8);
+    launch(k_s1_fill, grid_for(n3), kThreads, 0, s, S.field, n3, fill);  // cudaMemset only sets bytes
     const double inv_r = (R & (R - 1)) == 0 ? 1.0 / R : 0.0;
-    launch(k_s1_udist, grid_for(32LL * m), 256, 0, s, (const float *)S.tris, m, R, inv_r, band, S.field);
-    launch(k_s1_state, grid_for(n3), kThreads, 0, s, S.field, n3, R, band, S.state);
+    launch(k_s1_udist, grid_for(32LL * m), 256, 0, s, (const float *)S.tris, m, R, inv_r, kReach / R, S.field);
+    const int W = (R + 31) / 32, C = R - 1;
+    const long long words = (long long)R * R * W;
+    const Bits bits{R, W, S.bits, S.bits + words, S.bits + 2 * words, S.bits + 3 * words};
+    launch(k_s1_bits, grid_for(8 * words), kThreads, 0, s, (const unsigned long long *)S.field, bits, fill);
     // 3. flood fill from the boundary, until nothing changes
     if (S.prof) S.prof->begin(PH_S1_FLOOD, s);
     const int tpr = (R + kTile - 1) / kTile;
-    const int tiles = tpr * tpr * tpr;
+    const int tiles = tpr * tpr;
     // two dirty-tile flag sets used in turn: every tile is dirty at first
     uint8_t *dirty[2] = {S.tile_dirty, S.tile_dirty + tiles};
     S1_TRY(cudaMemsetAsync(dirty[0], 1, (size_t)tiles, s));
     S1_TRY(cudaMemsetAsync(dirty[1], 0, (size_t)tiles, s));
     int cur = 0;
     bool settled = false;
-    for (int round = 0; round < 4 * R + 64 && !settled; round += 8) {
-        S1_TRY(cudaMemsetAsync(S.dev + 4, 0, 4, s));
-        for (int k = 0; k < 8; ++k) {
-            launch(k_s1_flood, tiles, kTile * kTile * kTile, 0, s, S.state, R, S.dev, (const uint8_t *)dirty[cur],
-                   dirty[cur ^ 1]);
+    // a change crosses at least a row a launch: R^2 rows bound the launches
+    for (long long round = 0; round < (long long)R * R + 64 && !settled; round += 6) {
+        for (int k = 0; k < 6; ++k) {
+            if (k == 5) S1_TRY(cudaMemsetAsync(S.dev + 4, 0, 4, s));  // settled: nothing changed in the last launch
+            launch(k_s1_flood, tiles, kThreads, 0, s, bits, S.dev, (const uint8_t *)dirty[cur], dirty[cur ^ 1]);
             S1_TRY(cudaMemsetAsync(dirty[cur], 0, (size_t)tiles, s));
             cur ^= 1;
         }
@@ -746,19 +920,20 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
         if (S.prof) S.prof->collect();
         settled = S.h_dev[4] == 0;
     }
-    if (!settled) return PAMO_ERR_DEVICE;  // cannot happen within 4 R sweeps of tiles
-    launch(k_s1_field, grid_for(n3), kThreads, 0, s, S.field, (const uint8_t *)S.state, n3, R);
-    // 4. dual marching cubes: patch vertices
+    if (!settled) return PAMO_ERR_DEVICE;  // cannot happen within that many launches
+    launch(k_s1_inside, grid_for(words), kThreads, 0, s, bits);
+    // 4. dual marching cubes: patch and quad numbers, then the patch vertices
     if (S.prof) S.prof->begin(PH_S1_DMC, s);
-    launch(k_s1_cells, grid_for(c3), kThreads, 0, s, (const unsigned long long *)S.field, R, S.cell_cnt);
-    S1_TRY(cudaMemsetAsync(S.cell_cnt + c3, 0, 4, s));
-    S1_TRY(exclusive_scan(S.cell_cnt, S.cell_cnt, c3 + 1, nullptr, S.scan_cells, nullptr, s, S.dev + 6));
-    launch(k_s1_edges, grid_for(3 * n3), kThreads, 0, s, (const unsigned long long *)S.field, R, S.edge_cnt);
-    S1_TRY(cudaMemsetAsync(S.edge_cnt + 3 * n3, 0, 4, s));
-    S1_TRY(exclusive_scan(S.edge_cnt, S.edge_cnt, 3 * n3 + 1, nullptr, S.scan_edges, nullptr, s, S.dev + 6));
-    S1_TRY(cudaMemcpyAsync(S.h_dev + 8, S.cell_cnt + c3, 4, cudaMemcpyDeviceToHost, s));
-    S1_TRY(cudaMemcpyAsync(S.h_dev + 9, S.edge_cnt + 3 * n3, 4, cudaMemcpyDeviceToHost, s));
-    S1_TRY(cudaMemcpyAsync(S.h_dev + 6, S.dev + 6, 4, cudaMemcpyDeviceToHost, s));
+    const long long cwords = (long long)C * C * ((C + 31) / 32);
+    const Cells cells{C, (C + 31) / 32,
+                      {S.cell_bits, S.cell_bits + cwords, S.cell_bits + 2 * cwords, S.cell_bits + 3 * cwords},
+                      S.cell_first};
+    launch(k_s1_cells, grid_for(cwords), kThreads, 0, s, bits, cells);
+    launch(k_s1_edges, grid_for(3 * words), kThreads, 0, s, bits, S.edge_bits, S.edge_first);
+    S1_TRY(scan_jobs(ScanJob{S.cell_first, nullptr, S.cell_first, nullptr, cwords, nullptr, S.scan_cells, S.dev + 8},
+                     ScanJob{S.edge_first, nullptr, S.edge_first, nullptr, 3 * words, nullptr, S.scan_edges, S.dev + 9},
+                     s, S.dev + 6));
+    S1_TRY(cudaMemcpyAsync(S.h_dev, S.dev, 64, cudaMemcpyDeviceToHost, s));
     S1_TRY(cudaStreamSynchronize(s));
     if (S.h_dev[6]) return PAMO_ERR_DEVICE;  // a scan's wait ran out
     const long long nv = S.h_dev[8], nq = S.h_dev[9];
@@ -770,21 +945,19 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
         const int mx_bits = S.h_dev[3];
         if (mx_bits >= 0) memcpy(&tmax, &mx_bits, 4);
     }
-    launch(k_s1_verts, grid_for(c3), kThreads, 0, s, (const unsigned long long *)S.field, R, (const int *)S.cell_cnt,
-           band, margin, (double)tmax, (const int *)S.dev, S.verts);
+    launch(k_s1_lists, grid_for(cwords + 3 * words), kThreads, 0, s, cells, (const uint32_t *)S.edge_bits,
+           (const int *)S.edge_first, 3 * words, S.patch_list, S.quad_list);
+    launch(k_s1_verts, grid_for(nv), kThreads, 0, s, (const unsigned long long *)S.field, bits,
+           (const uint32_t *)S.patch_list, (int)nv, band, margin, (double)tmax, (const int *)S.dev, S.verts);
     // quads and their split
-    launch(k_s1_quads, grid_for(3 * n3), kThreads, 0, s, (const unsigned long long *)S.field, R,
-           (const int *)S.edge_cnt, (const int *)S.cell_cnt, (const float *)S.verts, S.quads, S.q_first);
-    S1_TRY(cudaMemsetAsync(S.q_first + nq, 0, 4, s));
-    int *qpos = S.edge_cnt;  // the edge slots are no longer needed: the flags' prefix
-    S1_TRY(exclusive_scan(S.q_first, qpos, nq + 1, nullptr, S.scan_quads, nullptr, s, S.dev + 6));
-    S1_TRY(cudaMemcpyAsync(S.h_dev + 10, qpos + nq, 4, cudaMemcpyDeviceToHost, s));
+    launch(k_s1_quads, grid_for(nq), kThreads, 0, s, bits, cells, (const uint32_t *)S.quad_list, (int)nq,
+           (const float *)S.verts, S.quads, S.q_first);
+    S1_TRY(scan_job(ScanJob{S.q_first, nullptr, S.q_pos, nullptr, nq, nullptr, S.scan_quads, S.dev + 10}, s, S.dev + 6));
+    launch(k_s1_faces, grid_for(nq), kThreads, 0, s, (const int4 *)S.quads, (const int *)S.q_first,
+           (const int *)S.q_pos, (int)nq, (const int *)(S.dev + 10), S.faces);
     S1_TRY(cudaMemcpyAsync(S.h_dev + 6, S.dev + 6, 4, cudaMemcpyDeviceToHost, s));
     S1_TRY(cudaStreamSynchronize(s));
     if (S.h_dev[6]) return PAMO_ERR_DEVICE;
-    const int n1 = S.h_dev[10];
-    launch(k_s1_faces, grid_for(nq), kThreads, 0, s, (const int4 *)S.quads, (const int *)S.q_first, (const int *)qpos,
-           (int)nq, n1, S.faces);
     if (S.prof) S.prof->end(s);
     S1_TRY(cudaGetLastError());
     S.n_verts = (int)nv;
