@@ -27,6 +27,7 @@ __device__ __forceinline__ void face_box(const float4 *pts, int4 t, float3 &lo, 
 
 __global__ void k_scene_init(int *scene)
 {
+    chain_wait();
     int i = threadIdx.x;
     if (i < 3) scene[i] = 0x7FFFFFFF;
     else if (i < 6) scene[i] = (int)0x80000000;
@@ -36,6 +37,7 @@ __global__ void k_scene_init(int *scene)
 // scene box and dead-face count over the round-start faces
 __global__ void __launch_bounds__(kThreads) k_scene_bounds(const float4 *pts, const int4 *tris, int m, int *scene)
 {
+    chain_wait();
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     int dead = 0;
     PAMO_GRID_STRIDE(f, m)
@@ -72,6 +74,7 @@ __global__ void __launch_bounds__(kThreads) k_scene_bounds(const float4 *pts, co
 __global__ void __launch_bounds__(kThreads) k_morton(const float4 *pts, const int4 *tris, int m, const int *scene,
                                                      uint32_t *keys, int *vals, const int *vslot, int bits)
 {
+    chain_wait();
     const float res = (float)(1 << bits);
     float slo[3], ext[3];
 #pragma unroll
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(kThreads) k_morton(const float4 *pts, const in
 __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const uint32_t *keys, int n, int shift, int tiles,
                                                              int *hist)
 {
+    chain_wait();
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -124,6 +128,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint32_t *
                                                                 int shift, int tiles, const int *hist_scanned,
                                                                 uint32_t *keys_out, int *vals_out)
 {
+    chain_wait();
     __shared__ int wc[kSortThreads / 32][256];
     __shared__ int base_off[256];
     base_off[threadIdx.x] = hist_scanned[threadIdx.x * tiles + blockIdx.x];
@@ -338,24 +343,24 @@ cudaError_t morton_order(const float4 *pts, const int4 *tris, int m, int *scene,
                          int *vals, int *vals2, int *hist, int *hist_scratch, const int *vslot, int n_ranks,
                          int &rank_shift, cudaStream_t s)
 {
-    launch(k_scene_init, 1, 32, 0, s, scene);
+    launch_chained(k_scene_init, 1, 32, 0, s, scene);
     if (m == 0) return cudaGetLastError();
-    launch(k_scene_bounds, grid_for(m), kThreads, 0, s, pts, tris, m, scene);
+    launch_chained(k_scene_bounds, grid_for(m), kThreads, 0, s, pts, tris, m, scene);
     // Morton bits per axis: 10, or fewer to leave room for the rank (keys of live
     // faces stay below 2^31, under the key of removed faces)
     int rank_bits = 0;
     while (vslot && (1 << rank_bits) < n_ranks) ++rank_bits;
     const int bits = vslot ? (31 - rank_bits) / 3 : 10;
     rank_shift = 3 * bits;
-    launch(k_morton, grid_for(m), kThreads, 0, s, pts, tris, m, (const int *)scene, keys, vals, vslot, bits);
+    launch_chained(k_morton, grid_for(m), kThreads, 0, s, pts, tris, m, (const int *)scene, keys, vals, vslot, bits);
     const int tiles = (m + kSortTile - 1) / kSortTile;
     uint32_t *k_in = keys, *k_out = keys2;
     int *v_in = vals, *v_out = vals2;
     for (int shift = 0; shift < 32; shift += 8) {
-        launch(k_radix_hist, tiles, kSortThreads, 0, s, k_in, m, shift, tiles, hist);
+        launch_chained(k_radix_hist, tiles, kSortThreads, 0, s, k_in, m, shift, tiles, hist);
         cudaError_t e = exclusive_scan(hist, hist, (long long)256 * tiles, nullptr, hist_scratch, nullptr, s);
         if (e != cudaSuccess) return e;
-        launch(k_radix_scatter, tiles, kSortThreads, 0, s, k_in, v_in, m, shift, tiles, hist, k_out, v_out);
+        launch_chained(k_radix_scatter, tiles, kSortThreads, 0, s, k_in, v_in, m, shift, tiles, hist, k_out, v_out);
         uint32_t *tk = k_in; k_in = k_out; k_out = tk;
         int *tv = v_in; v_in = v_out; v_out = tv;
     }

@@ -11,6 +11,7 @@ namespace {
 // at its ends.  Removed faces sort last (their key has a rank no mesh has).
 __global__ void k_tree_ranges(const uint32_t *keys, int m, int shift, int n_ranks, int2 *ranges)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(i, m)
     {
         const uint32_t r = keys[i] >> shift;
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(kTreeTile) k_tree_refit(const __grid_constant_
                                                           const uint8_t *__restrict__ sel, int *qlist, int *n_query,
                                                           uint8_t *flags, int m, int *ticket)
 {
+    chain_wait();
     __shared__ Box s1[64], s2[8];
     __shared__ int s_cnt[kTreeTile / 32], s_first;
     __shared__ bool s_last;
@@ -217,7 +219,7 @@ cudaError_t tree_build(PackedTree &t, const float4 *pts, const int4 *tris, int m
         return e;
     if (ranges) {
         if ((e = cudaMemsetAsync(ranges, 0, (size_t)n_ranks * sizeof(int2), s)) != cudaSuccess) return e;
-        if (m > 0) launch(k_tree_ranges, grid_for(m), kThreads, 0, s, (const uint32_t *)t.keys, m, shift, n_ranks, ranges);
+        if (m > 0) launch_chained(k_tree_ranges, grid_for(m), kThreads, 0, s, (const uint32_t *)t.keys, m, shift, n_ranks, ranges);
     }
     return cudaGetLastError();
 }
@@ -226,7 +228,7 @@ cudaError_t tree_refit(PackedTree &t, const float4 *pts, const int4 *tris, const
                        int *n_query, uint8_t *flags, int m, cudaStream_t s)
 {
     if (t.leaves <= 0) return cudaSuccess;
-    launch(k_tree_refit, (t.leaves + kTreeTile - 1) / kTreeTile, kTreeTile, 0, s, t.view(), pts, tris, sel, qlist,
+    launch_chained(k_tree_refit, (t.leaves + kTreeTile - 1) / kTreeTile, kTreeTile, 0, s, t.view(), pts, tris, sel, qlist,
            n_query, flags, m, t.scene + 10);
     return cudaGetLastError();
 }

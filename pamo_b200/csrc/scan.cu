@@ -20,6 +20,7 @@ constexpr int kSingleItems = 16;
 
 __global__ void __launch_bounds__(kSingleThreads) k_scan_single(const __grid_constant__ ScanPair P)
 {
+    chain_wait();
     const ScanJob &J = P.j[blockIdx.x];
     const long long n = J.d_n ? (long long)*J.d_n : J.n;
     const long long base = (long long)threadIdx.x * kSingleItems;
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const __grid_con
                                                                 int *fault, unsigned epoch, long long spin_limit,
                                                                 long long absent_tile)
 {
+    chain_wait();
     __shared__ int tile[kScanTile];
     __shared__ long long s_t;
     __shared__ int s_prefix;
@@ -210,11 +212,11 @@ cudaError_t scan_pair(const ScanPair &P, int n_jobs, cudaStream_t s, int *fault,
         single = single && P.j[k].n <= (long long)kSingleThreads * kSingleItems;
     }
     if (single) {
-        launch(k_scan_single, n_jobs, kSingleThreads, 0, s, P);
+        launch_chained(k_scan_single, n_jobs, kSingleThreads, 0, s, P);
         return cudaGetLastError();
     }
     const unsigned epoch = (epochs.fetch_add(1, std::memory_order_relaxed) + 1) & 0x3FFFFFFFu;
-    launch(k_scan_lookback, (unsigned)(tiles[0] + tiles[1]), kScanThreads, 0, s, P, (int)tiles[0], fault, epoch,
+    launch_chained(k_scan_lookback, (unsigned)(tiles[0] + tiles[1]), kScanThreads, 0, s, P, (int)tiles[0], fault, epoch,
            spin_limit, absent_tile);
     return cudaGetLastError();
 }

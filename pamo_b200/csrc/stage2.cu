@@ -59,6 +59,7 @@ __global__ void k_round_init(const float4 *__restrict__ opts, const int4 *__rest
                              int4 *tris, int *occ, int *deg, int *cursor, unsigned long long *vmin, int *first_edge,
                              uint8_t *active, RoundCounters *cnt, int n, int m)
 {
+    chain_wait();
     constexpr int kCounters = (int)(sizeof(RoundCounters) / sizeof(int));
     const long long N = n + 1 > kCounters ? n + 1 : kCounters;
     PAMO_GRID_STRIDE(i, N > m + 1 ? N : m + 1)
@@ -86,6 +87,7 @@ __global__ void k_round_init(const float4 *__restrict__ opts, const int4 *__rest
 __global__ void k_face_a(const float4 *__restrict__ pts, const int4 *__restrict__ tris, int m, int *deg,
                          int *ecount, float4 *plane, float4 *elen)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(f, m)
     {
         int4 t = tris[f];
@@ -111,6 +113,7 @@ __global__ void k_face_a(const float4 *__restrict__ pts, const int4 *__restrict_
 __global__ void k_face_b(const int4 *__restrict__ tris, int m, const int *__restrict__ first_near, int *cursor,
                          int *near_tris, const int *__restrict__ first_edge, int2 *edges)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(f, m)
     {
         int4 t = tris[f];
@@ -142,6 +145,7 @@ __global__ void __launch_bounds__(kThreads) k_vertex_quadric(const int *__restri
                                                              const int4 *__restrict__ tris, float *quad, int *nxt,
                                                              int n)
 {
+    chain_wait();
     __shared__ int s_face[kThreads / 8][kRing];
     __shared__ float4 s_plane[kThreads / 8][kRing];
     const int lane = threadIdx.x & 31, gl = lane & 7;
@@ -202,6 +206,7 @@ __global__ void __launch_bounds__(kThreads) k_vertex_quadric(const int *__restri
 __global__ void k_vertex_quadric64(const int *__restrict__ first_near, const int *__restrict__ near_tris,
                                    const float4 *__restrict__ pts, const int4 *__restrict__ tris, double *q64, int n)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(v, n)
     {
         double q[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -481,6 +486,7 @@ template <bool QUALITY>
 __global__ void __launch_bounds__(kThreads) k_edge_cost(CostArgs A, const int *order, int L,
                                                         const int *first_edge)
 {
+    chain_wait();
     __shared__ int s_list[kChunkEdges];
     for (long long base = (long long)blockIdx.x * kChunkFaces; base < L; base += (long long)gridDim.x * kChunkFaces) {
         const int total = chunk_edges(order, first_edge, L, base, s_list);
@@ -678,6 +684,7 @@ constexpr int kGroupLeaves = 8;  // few, so that a small mesh has a warp for eve
 template <bool QUALITY>
 __global__ void __launch_bounds__(kThreads, 4) k_edge_cost_group(CostArgs A, const int *order, int L, const int *first_edge)
 {
+    chain_wait();
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ int s_list[kThreads / 32][3 * kGroupLeaves];
     __shared__ float4 s_terms[kThreads];
@@ -770,6 +777,7 @@ struct CollapseArgs {
 // changes nothing.
 __global__ void __launch_bounds__(kThreads) k_collapse(CollapseArgs A)
 {
+    chain_wait();
     constexpr unsigned kAll = 0xffffffffu;
     const int E = *A.n_edges;
     const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
@@ -841,6 +849,7 @@ template <bool QUALITY>
 __global__ void __launch_bounds__(kThreads) k_collapse_apply(CollapseArgs A, const int *list, const int *n_list,
                                                              uint8_t *active)
 {
+    chain_wait();
     constexpr unsigned kAll = 0xffffffffu;
     const int N = *n_list;
     const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
@@ -958,6 +967,7 @@ __global__ void __launch_bounds__(kLineThreads) k_cleanup(int4 *tris, int m, con
                                                           const int *near_tris, int *occ, int *collapsed,
                                                           uint8_t *active, RoundCounters *cnt)
 {
+    chain_wait();
     const int E = *n_edges;
     __shared__ bool s_last;
     int local = 0;
@@ -1038,6 +1048,7 @@ __global__ void __launch_bounds__(kQueryThreads) k_query(const __grid_constant__
                                                          int skip_shared, const int2 *__restrict__ ranges,
                                                          const int *__restrict__ vslot)
 {
+    chain_wait();
     __shared__ uint2 s_pairs[kQueryThreads / 32][64];
     __shared__ int s_off[kTreeMaxLevels];  // indexed by a lane's own level
 #pragma unroll
@@ -1124,6 +1135,7 @@ __global__ void __launch_bounds__(kThreads) k_pairs(const uint2 *pairs, RoundCou
                                                     long long cap_pairs, const float4 *__restrict__ pts,
                                                     const int4 *__restrict__ tris, uint8_t *isect, float eps)
 {
+    chain_wait();
     long long N = cnt->n_pairs < cap_pairs ? cnt->n_pairs : cap_pairs;
     PAMO_GRID_STRIDE(k, N)
     {
@@ -1163,6 +1175,7 @@ __global__ void __launch_bounds__(kThreads) k_pairs(const uint2 *pairs, RoundCou
 __global__ void k_undo_flags(const int *collapsed, RoundCounters *cnt, const int2 *edges,
                              const int *first_near, const int *near_tris, const uint8_t *isect, int *uflag)
 {
+    chain_wait();
     if (!cnt->n_hit) return;  // no pair intersects (n_undo is 0)
     const int N = cnt->n_considered;
     int local = 0;
@@ -1190,6 +1203,7 @@ __global__ void k_undo_apply(const int *undo_idx, int N, const int *collapsed, c
                              int first, const SlotInfo *slots, const SlotCounters *scnt, const int *vslot,
                              RoundCounters *cnt)
 {
+    chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0)
         cnt->n_pairs = cnt->pair_overflow = cnt->n_query = cnt->n_hit = cnt->n_undo = 0;
     PAMO_GRID_STRIDE(k, N)
@@ -1236,6 +1250,7 @@ __global__ void k_mark_invalid(const int *undo_in, int n, uint8_t *table)
 __global__ void k_compact(const float4 *pts, const int *occ, const int *pts_map, int n, const int4 *tris,
                           const int *fpos, int m, float4 *opts, int4 *otris, int *vals, int L, RoundCounters *cnt)
 {
+    chain_wait();
     long long N = n > m ? n : m;
     N = N > L ? N : L;
     PAMO_GRID_STRIDE(i, N)
@@ -1287,6 +1302,7 @@ __global__ void k_validate_range(const int *v, int count, int hi, int *bad)
 // vertex map; not stuck with a non-empty list: the invalid table is cleared.
 __global__ void k_b_pre_copy(const SlotInfo *slots)
 {
+    chain_wait();
     const SlotInfo S = slots[blockIdx.y];
     if (S.is_stuck) {
         SLOT_STRIDE(j, S.n_undo_in)
@@ -1302,12 +1318,14 @@ __global__ void k_b_pre_copy(const SlotInfo *slots)
 
 __global__ void k_b_pre_mark(const SlotInfo *slots)
 {
+    chain_wait();
     const SlotInfo S = slots[blockIdx.y];
     SLOT_STRIDE(j, S.n_undo_in) S.invalid[S.undo_prev[j]] = 1;
 }
 
 __global__ void k_b_vslot(const SlotInfo *slots, int *vslot)
 {
+    chain_wait();
     const SlotInfo S = slots[blockIdx.y];
     SLOT_STRIDE(j, S.n) vslot[S.vert_off + j] = (int)blockIdx.y;
 }
@@ -1315,6 +1333,7 @@ __global__ void k_b_vslot(const SlotInfo *slots, int *vslot)
 // first packed edge and edge count of each mesh (first_edge has m + 1 entries)
 __global__ void k_b_edge_off(const SlotInfo *slots, const int *first_edge, SlotCounters *scnt, int K)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(r, K)
     {
         const SlotInfo &S = slots[r];
@@ -1335,6 +1354,7 @@ __device__ __forceinline__ void seg_of_scan(const int *pos, int total, int n_all
 
 __global__ void k_b_main(const int *pos, const RoundCounters *cnt, SlotCounters *scnt, int K)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(r, K)
     {
         int off, c;
@@ -1354,6 +1374,7 @@ __global__ void __launch_bounds__(kLineThreads) k_b_line_apply(const int2 *edges
                                                                int *line_list, const int *vslot, RoundCounters *cnt,
                                                                SlotCounters *scnt, int K)
 {
+    chain_wait();
     const int E = *n_edges;
     for (int r = threadIdx.x; r < K; r += blockDim.x) scnt[r].n_line = 0;
     __syncthreads();
@@ -1386,6 +1407,7 @@ __global__ void k_b_cand_fill(const int *collapsed, const int *line_list, const 
                               const RoundCounters *cnt, const SlotCounters *scnt, int *cand,
                               const int *first_near, const int *near_tris, uint8_t *active)
 {
+    chain_wait();
     const int nm = cnt->n_main, nl = cnt->n_line;
     PAMO_GRID_STRIDE(p, (long long)nm + nl)
     {
@@ -1411,6 +1433,7 @@ __global__ void k_b_cand_fill(const int *collapsed, const int *line_list, const 
 
 __global__ void k_b_undo_counts(const int *upos, const RoundCounters *cnt, SlotCounters *scnt, int K)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(r, K)
     {
         int off, c;
@@ -1423,6 +1446,7 @@ __global__ void k_b_undo_counts(const int *upos, const RoundCounters *cnt, SlotC
 // each mesh's vertex map in its own numbers, and the copy of its undo list
 __global__ void k_b_local_map(const SlotInfo *slots, const int *gmap)
 {
+    chain_wait();
     const SlotInfo S = slots[blockIdx.y];
     const int base = gmap[S.vert_off];
     SLOT_STRIDE(j, (long long)S.n + 1) S.pts_map[j] = gmap[S.vert_off + j] - base;
@@ -1431,6 +1455,7 @@ __global__ void k_b_local_map(const SlotInfo *slots, const int *gmap)
 
 __global__ void k_b_next(const SlotInfo *slots, const int *gmap, const int *fpos, SlotCounters *scnt, int K)
 {
+    chain_wait();
     PAMO_GRID_STRIDE(r, K)
     {
         const SlotInfo &S = slots[r];
@@ -1666,21 +1691,22 @@ static cudaError_t isect_pass(Stage2 &S, int m, const int *considered, cudaStrea
         return e;
     S.prof.begin(PH_QUERY, s);
     if (S.n_slots > 0)
-        launch(k_query<true>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.qlist, S.dcnt,
+        launch_chained(k_query<true>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.qlist, S.dcnt,
                S.pairs, S.cap_pairs, 2, (const int2 *)S.ranges, (const int *)S.vslot);
     else
-        launch(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.qlist, S.dcnt,
+        launch_chained(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, S.tree.view(), (const int *)S.qlist, S.dcnt,
                S.pairs, S.cap_pairs, S.quality ? 4 : 2, (const int2 *)nullptr, (const int *)nullptr);
     S.prof.begin(PH_PAIRS, s);
+    const int pair_grid = grid_for(S.cap_pairs < 8LL * m ? S.cap_pairs : 8LL * m);  // about the pairs there are
     if (S.quality)
-        launch(k_pairs<true>, grid_for(S.cap_pairs), kThreads, 0, s, S.pairs, S.dcnt, S.cap_pairs, S.pts, S.tris,
+        launch_chained(k_pairs<true>, pair_grid, kThreads, 0, s, S.pairs, S.dcnt, S.cap_pairs, S.pts, S.tris,
                S.isect, 1e-3f);
     else
-        launch(k_pairs<false>, grid_for(S.cap_pairs), kThreads, 0, s, S.pairs, S.dcnt, S.cap_pairs, S.pts, S.tris,
+        launch_chained(k_pairs<false>, pair_grid, kThreads, 0, s, S.pairs, S.dcnt, S.cap_pairs, S.pts, S.tris,
                S.isect, 1e-3f);
     if (considered) {
         S.prof.begin(PH_UNDO, s);
-        launch(k_undo_flags, grid_for(3LL * m), kThreads, 0, s, considered, S.dcnt, (const int2 *)S.edges,
+        launch_chained(k_undo_flags, grid_for(3LL * m), kThreads, 0, s, considered, S.dcnt, (const int2 *)S.edges,
                (const int *)S.first_near, (const int *)S.near_tris, (const uint8_t *)S.isect, S.uflag);
     }
     S.prof.end(s);
@@ -1724,10 +1750,10 @@ template <bool QUALITY>
 static void launch_edge_cost(const CostArgs &A, const int *order, int m, int L, const int *first_edge, cudaStream_t s)
 {
     if (m <= (QUALITY ? 50000 : 100000))
-        launch(k_edge_cost_group<QUALITY>, grid_for(L, kThreads / 32 * kGroupLeaves), kThreads, 0, s, A, order, L,
+        launch_chained(k_edge_cost_group<QUALITY>, grid_for(L, kThreads / 32 * kGroupLeaves), kThreads, 0, s, A, order, L,
                first_edge);
     else
-        launch(k_edge_cost<QUALITY>, grid_for(L, kChunkFaces), kThreads, 0, s, A, order, L, first_edge);
+        launch_chained(k_edge_cost<QUALITY>, grid_for(L, kChunkFaces), kThreads, 0, s, A, order, L, first_edge);
 }
 
 int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, const int *d_undo_in, int n_undo_in,
@@ -1754,20 +1780,20 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
     const uint32_t collapse_t = (uint32_t)(unsigned long long)(ct / kCostRange * 4294967296.0f);
 
     prof.begin(PH_SETUP, s);
-    launch(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
+    launch_chained(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
            tris, occ, first_near, cursor, vmin, first_edge, active, dcnt, n, m);
-    launch(k_face_a, grid_for(m), kThreads, 0, s, pts, tris, m, first_near, first_edge, plane, elen4);
+    launch_chained(k_face_a, grid_for(m), kThreads, 0, s, pts, tris, m, first_near, first_edge, plane, elen4);
     S2_TRY(scan_jobs(ScanJob{first_near, nullptr, first_near, nullptr, n + 1LL, nullptr, scan_scratch, nullptr},
                      ScanJob{first_edge, nullptr, first_edge, nullptr, m + 1LL, nullptr, scan_scratch2, &dcnt->n_edges},
                      s, &dcnt->scan_fault));
     const int *d_n_edges = &dcnt->n_edges;
-    launch(k_face_b, grid_for(m), kThreads, 0, s, tris, m, first_near, cursor, near_tris, first_edge, edges);
-    launch(k_vertex_quadric, grid_for(8LL * n), kThreads, 0, s, (const int *)first_near, near_tris, (const float4 *)plane,
+    launch_chained(k_face_b, grid_for(m), kThreads, 0, s, tris, m, first_near, cursor, near_tris, first_edge, edges);
+    launch_chained(k_vertex_quadric, grid_for(8LL * n), kThreads, 0, s, (const int *)first_near, near_tris, (const float4 *)plane,
            (const int4 *)tris, reinterpret_cast<float *>(quad), nxt, n);
     if (quality) {
         int rc = ensure_quality(n, 3LL * m);
         if (rc) return rc;
-        launch(k_vertex_quadric64, grid_for(n), kThreads, 0, s, (const int *)first_near, (const int *)near_tris,
+        launch_chained(k_vertex_quadric64, grid_for(n), kThreads, 0, s, (const int *)first_near, (const int *)near_tris,
                (const float4 *)pts, (const int4 *)tris, quad64, n);
     }
     // The tree only needs an order of the round input's faces: sort them, or keep
@@ -1792,17 +1818,17 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
     CollapseArgs cl{edges, d_n_edges, edge_cost, vmin, first_near, near_tris, opts, otris, pts, tris, occ, eflag,
                     collapse_t, nullptr, nullptr, nullptr, quality ? (const float4 *)epos : nullptr};
     prof.begin(PH_COLLAPSE, s);
-    launch(k_collapse, grid_for(EMAX), kThreads, 0, s, cl);
+    launch_chained(k_collapse, grid_for(EMAX), kThreads, 0, s, cl);
     S2_TRY(scan_job(ScanJob{eflag, nullptr, nullptr, collapsed, EMAX, d_n_edges, scan_scratch, &dcnt->n_main}, s,
                     &dcnt->scan_fault));
     if (quality)
-        launch(k_collapse_apply<true>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
+        launch_chained(k_collapse_apply<true>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
                (const int *)&dcnt->n_main, active);
     else
-        launch(k_collapse_apply<false>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
+        launch_chained(k_collapse_apply<false>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
                (const int *)&dcnt->n_main, active);
     prof.begin(PH_CLEANUP, s);
-    launch(k_cleanup<false>, grid_for(EMAX), kLineThreads, 0, s, tris, m, (const int2 *)edges, d_n_edges, pts, eflag,
+    launch_chained(k_cleanup<false>, grid_for(EMAX), kLineThreads, 0, s, tris, m, (const int2 *)edges, d_n_edges, pts, eflag,
            (const int *)first_near, (const int *)near_tris, occ, collapsed, active, dcnt);
     int rc = checked_pass(*this, m, collapsed, s);
     if (rc) return rc;
@@ -1821,7 +1847,7 @@ int Stage2::round(int n, int m, float scale, float threshold, bool is_stuck, con
         S2_TRY(undo_list_of(*this, nullptr, s));
         const bool reselect = hcnt->n_line == 0;  // see isect_pass
         if (reselect) S2_TRY(cudaMemsetAsync(active, 0, (size_t)m, s));
-        launch(k_undo_apply, grid_for(cnt_undo), kThreads, 0, s, (const int *)undo_idx, cnt_undo,
+        launch_chained(k_undo_apply, grid_for(cnt_undo), kThreads, 0, s, (const int *)undo_idx, cnt_undo,
                (const int *)collapsed, (const int2 *)edges, (const int *)first_near, (const int *)near_tris,
                (const float4 *)opts, (const int4 *)otris, pts, tris, occ, reselect ? active : nullptr,
                (const int *)pts_map, undo_list, first, (const SlotInfo *)nullptr, (const SlotCounters *)nullptr,
@@ -1850,9 +1876,9 @@ cudaError_t query_and_test_pairs(PackedTree &tree, const float4 *pts, const int4
 {
     cudaError_t e = tree_refit(tree, pts, tris, nullptr, qlist, &cnt->n_query, isect, m, s);
     if (e != cudaSuccess) return e;
-    launch(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, tree.view(), (const int *)qlist, cnt, pairs,
+    launch_chained(k_query<false>, grid_for(8LL * m), kQueryThreads, 0, s, tree.view(), (const int *)qlist, cnt, pairs,
            cap_pairs, 2, (const int2 *)nullptr, (const int *)nullptr);
-    launch(k_pairs<false>, grid_for(cap_pairs), kThreads, 0, s, pairs, cnt, cap_pairs, pts, tris, isect, 1e-3f);
+    launch_chained(k_pairs<false>, grid_for(cap_pairs), kThreads, 0, s, pairs, cnt, cap_pairs, pts, tris, isect, 1e-3f);
     return cudaGetLastError();
 }
 
@@ -1881,7 +1907,7 @@ int Stage2::self_intersect_all(int n, int m, cudaStream_t s)
 {
     tree_carried = false;
     // faces of opts/otris; every live face queries the tree
-    launch(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
+    launch_chained(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
            tris, occ, first_near, cursor, vmin, first_edge, active, dcnt, n, m);
     S2_TRY(cudaMemsetAsync(active, 1, (size_t)m, s));
     S2_TRY(tree_build(tree, pts, tris, m, s));
@@ -1892,7 +1918,7 @@ int Stage2::compact(int n, int m, cudaStream_t s)
 {
     prof.begin(PH_COMPACT, s);
     const bool keep = tree.leaves > 0 && tree.leaves >= m;
-    launch(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, (const float4 *)pts, (const int *)occ,
+    launch_chained(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, (const float4 *)pts, (const int *)occ,
            (const int *)pts_map, n, (const int4 *)tris, (const int *)fpos, m, opts, otris, tree.vals,
            keep ? tree.leaves : 0, dcnt);
     tree_carried = keep;
@@ -1962,23 +1988,23 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     }
     S2_TRY(cudaMemsetAsync(scnt, 0, (size_t)K * sizeof(SlotCounters), s));
     S2_TRY(cudaMemcpyAsync(slots, hslots, (size_t)K * sizeof(SlotInfo), cudaMemcpyHostToDevice, s));
-    launch(k_b_pre_copy, slot_grid(K, max_undo_in > max_cap_v ? max_undo_in : max_cap_v), kThreads, 0, s,
+    launch_chained(k_b_pre_copy, slot_grid(K, max_undo_in > max_cap_v ? max_undo_in : max_cap_v), kThreads, 0, s,
            (const SlotInfo *)slots);
-    launch(k_b_pre_mark, slot_grid(K, max_undo_in), kThreads, 0, s, (const SlotInfo *)slots);
-    launch(k_b_vslot, slot_grid(K, max_n), kThreads, 0, s, (const SlotInfo *)slots, vslot);
+    launch_chained(k_b_pre_mark, slot_grid(K, max_undo_in), kThreads, 0, s, (const SlotInfo *)slots);
+    launch_chained(k_b_vslot, slot_grid(K, max_n), kThreads, 0, s, (const SlotInfo *)slots, vslot);
 
     prof.begin(PH_SETUP, s);
-    launch(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
+    launch_chained(k_round_init, grid_for((n > m ? n : m) + 1LL), kThreads, 0, s, (const float4 *)opts, (const int4 *)otris, pts,
            tris, occ, first_near, cursor, vmin, first_edge, active, dcnt, n, m);
-    launch(k_face_a, grid_for(m), kThreads, 0, s, pts, tris, m, first_near, first_edge, plane, elen4);
+    launch_chained(k_face_a, grid_for(m), kThreads, 0, s, pts, tris, m, first_near, first_edge, plane, elen4);
     S2_TRY(scan_jobs(ScanJob{first_near, nullptr, first_near, nullptr, n + 1LL, nullptr, scan_scratch, nullptr},
                      ScanJob{first_edge, nullptr, first_edge, nullptr, m + 1LL, nullptr, scan_scratch2, &dcnt->n_edges},
                      s, &dcnt->scan_fault));
     const int *d_n_edges = &dcnt->n_edges;
-    launch(k_face_b, grid_for(m), kThreads, 0, s, tris, m, first_near, cursor, near_tris, first_edge, edges);
-    launch(k_vertex_quadric, grid_for(8LL * n), kThreads, 0, s, (const int *)first_near, near_tris, (const float4 *)plane,
+    launch_chained(k_face_b, grid_for(m), kThreads, 0, s, tris, m, first_near, cursor, near_tris, first_edge, edges);
+    launch_chained(k_vertex_quadric, grid_for(8LL * n), kThreads, 0, s, (const int *)first_near, near_tris, (const float4 *)plane,
            (const int4 *)tris, reinterpret_cast<float *>(quad), nxt, n);
-    launch(k_b_edge_off, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)first_edge, scnt, K);
+    launch_chained(k_b_edge_off, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)first_edge, scnt, K);
     prof.begin(PH_LBVH_BUILD, s);
     S2_TRY(tree_build(tree, pts, tris, m, s, vslot, K, ranges));
 
@@ -1990,18 +2016,18 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
     CollapseArgs cl{edges, d_n_edges, nullptr, vmin, first_near, near_tris, opts, otris, pts, tris, occ, eflag,
                     0u, slots, scnt, vslot, nullptr};
     prof.begin(PH_COLLAPSE, s);
-    launch(k_collapse, grid_for(EMAX), kThreads, 0, s, cl);
+    launch_chained(k_collapse, grid_for(EMAX), kThreads, 0, s, cl);
     S2_TRY(scan_job(ScanJob{eflag, nullptr, uflag, collapsed, EMAX, d_n_edges, scan_scratch, &dcnt->n_main}, s,
                     &dcnt->scan_fault));
-    launch(k_collapse_apply<false>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
+    launch_chained(k_collapse_apply<false>, grid_for(EMAX), kThreads, 0, s, cl, (const int *)collapsed,
            (const int *)&dcnt->n_main, active);
-    launch(k_b_main, grid_for(K), kThreads, 0, s, (const int *)uflag, (const RoundCounters *)dcnt, scnt, K);
+    launch_chained(k_b_main, grid_for(K), kThreads, 0, s, (const int *)uflag, (const RoundCounters *)dcnt, scnt, K);
     prof.begin(PH_CLEANUP, s);
-    launch(k_cleanup<true>, grid_for(EMAX), kLineThreads, 0, s, tris, m, (const int2 *)edges, d_n_edges, pts, eflag,
+    launch_chained(k_cleanup<true>, grid_for(EMAX), kLineThreads, 0, s, tris, m, (const int2 *)edges, d_n_edges, pts, eflag,
            (const int *)first_near, (const int *)near_tris, occ, collapsed, active, dcnt);
-    launch(k_b_line_apply, 1, kLineThreads, 0, s, edges, d_n_edges, eflag, first_near, near_tris, pts, tris, occ,
+    launch_chained(k_b_line_apply, 1, kLineThreads, 0, s, edges, d_n_edges, eflag, first_near, near_tris, pts, tris, occ,
            line_list, (const int *)vslot, dcnt, scnt, K);
-    launch(k_b_cand_fill, grid_for(EMAX), kThreads, 0, s, (const int *)collapsed, (const int *)line_list, edges,
+    launch_chained(k_b_cand_fill, grid_for(EMAX), kThreads, 0, s, (const int *)collapsed, (const int *)line_list, edges,
            (const int *)vslot, (const RoundCounters *)dcnt, (const SlotCounters *)scnt, cand, (const int *)first_near,
            (const int *)near_tris, active);
     // a check, and where it finds edges to undo their list and each mesh's share of it
@@ -2011,7 +2037,7 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
         for (int r = 0; r < K; ++r) hscnt[r].n_undo = 0;
         if (hcnt->n_undo == 0) return PAMO_OK;
         S2_TRY(undo_list_of(*this, eflag, s));
-        launch(k_b_undo_counts, grid_for(K), kThreads, 0, s, (const int *)eflag, (const RoundCounters *)dcnt, scnt, K);
+        launch_chained(k_b_undo_counts, grid_for(K), kThreads, 0, s, (const int *)eflag, (const RoundCounters *)dcnt, scnt, K);
         S2_TRY(cudaMemcpyAsync(hscnt, scnt, (size_t)K * sizeof(SlotCounters), cudaMemcpyDeviceToHost, s));
         S2_TRY(cudaStreamSynchronize(s));
         return PAMO_OK;
@@ -2041,7 +2067,7 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
         S2_TRY(cudaMemcpyAsync(slots, hslots, (size_t)K * sizeof(SlotInfo), cudaMemcpyHostToDevice, s));
         const bool reselect = hcnt->n_line == 0;  // as in the single-mesh round
         if (reselect) S2_TRY(cudaMemsetAsync(active, 0, (size_t)m, s));
-        launch(k_undo_apply, grid_for(hcnt->n_undo), kThreads, 0, s, (const int *)undo_idx, hcnt->n_undo,
+        launch_chained(k_undo_apply, grid_for(hcnt->n_undo), kThreads, 0, s, (const int *)undo_idx, hcnt->n_undo,
                (const int *)cand, (const int2 *)edges, (const int *)first_near, (const int *)near_tris,
                (const float4 *)opts, (const int4 *)otris, pts, tris, occ, reselect ? active : nullptr,
                (const int *)nullptr, (int *)nullptr, 0, (const SlotInfo *)slots, (const SlotCounters *)scnt,
@@ -2069,7 +2095,7 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
         nvu_out[r] = nvu[r];
     }
     S2_TRY(cudaMemcpyAsync(slots, hslots, (size_t)K * sizeof(SlotInfo), cudaMemcpyHostToDevice, s));
-    launch(k_b_local_map, slot_grid(K, (max_n + 1 > max_nvu ? max_n + 1 : max_nvu)), kThreads, 0, s,
+    launch_chained(k_b_local_map, slot_grid(K, (max_n + 1 > max_nvu ? max_n + 1 : max_nvu)), kThreads, 0, s,
            (const SlotInfo *)slots, (const int *)gmap);
     prof.end(s);
     return PAMO_OK;
@@ -2078,9 +2104,9 @@ int Stage2::round_batch(int n, int m, int K, int *nvu_out, cudaStream_t s)
 int Stage2::compact_batch(int n, int m, int K, cudaStream_t s)
 {
     prof.begin(PH_COMPACT, s);
-    launch(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, (const float4 *)pts, (const int *)occ, (const int *)gmap,
+    launch_chained(k_compact, grid_for(n > m ? n : m), kThreads, 0, s, (const float4 *)pts, (const int *)occ, (const int *)gmap,
            n, (const int4 *)tris, (const int *)fpos, m, opts, otris, (int *)nullptr, 0, dcnt);
-    launch(k_b_next, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)gmap, (const int *)fpos, scnt,
+    launch_chained(k_b_next, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)gmap, (const int *)fpos, scnt,
            K);
     prof.end(s);
     S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
