@@ -1190,20 +1190,31 @@ __global__ void k_b_extract(const float4 *opts, const int4 *otris, int voff, int
 }
 
 struct Move {
-    int src_v, dst_v, n, src_f, dst_f, m;
+    int src_v, dst_v, n, src_f, dst_f, m;  // m < 0: the mesh left
+    int rank;                              // before the move
 };
 
-// kept meshes moved down to close the gaps of retired ones (into the other buffer)
-__global__ void k_b_repack(const Move *moves, const float4 *src_p, const int4 *src_t, float4 *dst_p, int4 *dst_t)
+// kept meshes moved down to close the gaps of retired ones (into the other buffer),
+// their leaves renumbered, their runs of leaves under their new ranks; a retired
+// mesh's leaves become empty
+__global__ void k_b_repack(const Move *moves, const float4 *src_p, const int4 *src_t, float4 *dst_p, int4 *dst_t,
+                           const int2 *ranges, int2 *ranges_next, int *vals)
 {
     const Move mv = moves[blockIdx.y];
     const int shift = mv.src_v - mv.dst_v;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (mv.n > mv.m ? mv.n : mv.m);
+    const int2 run = ranges[mv.rank];
+    if (mv.m >= 0 && blockIdx.x == 0 && threadIdx.x == 0) ranges_next[blockIdx.y] = run;
+    const int len = run.y - run.x, most = mv.n > mv.m ? mv.n : mv.m;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (most > len ? most : len);
          i += (long long)blockDim.x * gridDim.x) {
         if (i < mv.n) dst_p[mv.dst_v + i] = src_p[mv.src_v + i];
         if (i < mv.m) {
             int4 t = src_t[mv.src_f + i];
             dst_t[mv.dst_f + i] = make_int4(t.x - shift, t.y - shift, t.z - shift, 0);
+        }
+        if (i < len) {
+            const int f = vals[run.x + i];
+            if (f >= 0) vals[run.x + i] = mv.m >= 0 ? f - (mv.src_f - mv.dst_f) : -1;
         }
     }
 }
@@ -1434,6 +1445,7 @@ int pamo_batch_destroy(pamo_batch *b)
     if (b->S.slots) cudaFree(b->S.slots);
     if (b->S.scnt) cudaFree(b->S.scnt);
     if (b->S.ranges) cudaFree(b->S.ranges);
+    if (b->S.ranges_next) cudaFree(b->S.ranges_next);
     if (b->S.vslot) cudaFree(b->S.vslot);
     if (b->S.gmap) cudaFree(b->S.gmap);
     if (b->S.line_list) cudaFree(b->S.line_list);
@@ -1523,6 +1535,7 @@ int pamo_batch_step(pamo_batch *b, int *out_running, int *out_pending)
             continue;
         }
         int rc = batch_admit(b, j);
+        S.tree_carried = false;  // the new mesh's faces are not in the order
         b->pending.erase(b->pending.begin() + k);
         if (rc) {
             batch_fail(b, j, rc);
@@ -1562,12 +1575,14 @@ int pamo_batch_step(pamo_batch *b, int *out_running, int *out_pending)
             }
             b->running.clear();
             b->n_packed = b->m_packed = 0;
+            S.tree_carried = false;
             return rc;
         }
         b->rounds_run++;
         // PaMO.run's loop per mesh (simp_cuda/pamo/__init__.py:169-185)
         std::vector<BatchJob *> keep;
         int n_moves = 0, dst_v = 0, dst_f = 0;
+        std::vector<Move> left;
         bool moved = false;
         for (int r = 0; r < K; ++r) {
             BatchJob *j = b->running[r];
@@ -1595,17 +1610,20 @@ int pamo_batch_step(pamo_batch *b, int *out_running, int *out_pending)
                 if (frc) batch_fail(b, j, frc);
                 b->done_ids.push_back(j->id);
                 moved = true;
+                left.push_back(Move{0, 0, 0, 0, 0, -1, r});
                 continue;
             }
             if (j->vert_off != dst_v || j->face_off != dst_f) moved = true;
-            b->h_moves[n_moves++] = Move{j->vert_off, dst_v, j->n, j->face_off, dst_f, j->m};
+            b->h_moves[n_moves++] = Move{j->vert_off, dst_v, j->n, j->face_off, dst_f, j->m, r};
             j->vert_off = dst_v;
             j->face_off = dst_f;
             dst_v += j->n;
             dst_f += j->m;
             keep.push_back(j);
         }
+        if (n_moves == 0) S.tree_carried = false;
         if (moved && n_moves > 0) {
+            for (const Move &l : left) b->h_moves[n_moves++] = l;  // at most max_meshes entries in all
             int max_len = 0;
             for (int k = 0; k < n_moves; ++k) {
                 int l = b->h_moves[k].n > b->h_moves[k].m ? b->h_moves[k].n : b->h_moves[k].m;
@@ -1615,7 +1633,9 @@ int pamo_batch_step(pamo_batch *b, int *out_running, int *out_pending)
             long long gx = (max_len + kThreads - 1) / kThreads;
             gx = gx < 1 ? 1 : (gx > 64 ? 64 : gx);
             launch(k_b_repack, dim3((unsigned)gx, (unsigned)n_moves), kThreads, 0, s, (const Move *)b->d_moves,
-                   (const float4 *)S.opts, (const int4 *)S.otris, S.pts, S.tris);
+                   (const float4 *)S.opts, (const int4 *)S.otris, S.pts, S.tris, (const int2 *)S.ranges, S.ranges_next,
+                   S.tree.vals);
+            std::swap(S.ranges, S.ranges_next);
             std::swap(S.opts, S.pts);
             std::swap(S.otris, S.tris);
             CU_RET(cudaGetLastError());

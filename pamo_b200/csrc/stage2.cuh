@@ -170,7 +170,8 @@ struct Stage2 {
     SlotCounters *scnt = nullptr;    // device [cap_slots]
     SlotCounters *hscnt = nullptr;   // pinned host copy
     int *vslot = nullptr;            // device [cap_pts + 1]: rank of each packed vertex
-    int2 *ranges = nullptr;          // device [cap_slots]: each rank's run of leaves in the hierarchy
+    int2 *ranges = nullptr;          // device [cap_slots]: each rank's run of leaves in the tree
+    int2 *ranges_next = nullptr;     // and for the ranks after meshes left
     int *line_list = nullptr;        // device [cap_edges + 1]
     int *cand = nullptr;             // device [cap_edges + 1]: per-mesh undo-candidate windows
     int *gmap = nullptr;             // device [cap_pts + 1]: packed vertex map
