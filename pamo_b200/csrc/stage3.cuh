@@ -55,9 +55,9 @@ struct Stage3 {
     // contact blocks
     int4 *bidx = nullptr;
     int *bkind = nullptr, *bsub = nullptr;
-    float *bd = nullptr, *bb2 = nullptr;
-    float4 *bg = nullptr;  // 4 gradient vectors per block
-    int *bact = nullptr;   // blocks with d < d_hat (the CG operator's contact terms)
+    float *bd = nullptr;
+    int4 *aidx = nullptr;  // blocks with d < d_hat (the CG operator's contact terms), packed:
+    float4 *ag = nullptr;  // vertices, and gradients as 4 arrays of cap_b
     int2 *cand_pt = nullptr, *cand_ee = nullptr;  // detection: pairs whose boxes overlap
     long long cap_c = 0;
     float4 *q_gather = nullptr;  // positions when the candidates were gathered
