@@ -349,7 +349,10 @@ __device__ __forceinline__ double box_d2(float4 lo, float4 hi, D3 p)
 // mesh.  The eight lanes test a node's children, the walk enters the nearest one
 // and leaves the others that could still hold something closer on the group's
 // stack (shared memory; at most seven a level).  All lanes of a warp call this
-// together; the result is the same in all lanes of a group.
+// together; the result is the same in all lanes of a group.  That rests on the
+// lanes' distances being ordered: a face with a NaN or infinite corner gives NaN,
+// which would stay in its lane's minimum and part the lanes' walks, so a leaf's
+// distance is never more than DBL_MAX (box_d2 gives no NaN: fmax drops it).
 constexpr int kHdThreads = 128;
 constexpr int kHdStack = 64;
 
@@ -375,6 +378,7 @@ __device__ __forceinline__ double nearest_d2(bool has, D3 p, const TreeView &T, 
             if (lvl == 0) {
                 const int4 t = d < best && node < T.L ? T.leaf[node] : make_int4(0, 0, 0, kLeafDead);
                 d = t.w != kLeafDead ? point_tri_d2(p, dat(pts[t.x]), dat(pts[t.y]), dat(pts[t.z])) : DBL_MAX;
+                d = fmin(d, DBL_MAX);
             }
         }
         double m = d;
