@@ -148,11 +148,10 @@ __global__ void __launch_bounds__(kPairThreads) k_ck_pairs(const __grid_constant
         while (__any_sync(0xffffffffu, wk.run)) {
             bool hit = false, emit = false;
             const int node = 8 * wk.g + gl;
-            if (wk.run) {
+            if (wk.run && T.holds(wk.lvl, node)) {
                 const size_t b = 2 * ((size_t)s_off[wk.lvl] + node);
                 const float4 lo = T.boxes[b], hi = T.boxes[b + 1];
-                const bool leaf = wk.lvl == 0 && node < T.L;
-                const int g = leaf ? T.leaf[node].w : kLeafDead;
+                const int g = wk.lvl == 0 ? T.leaf[node].w : kLeafDead;
                 hit = !(hi.x < qlo.x || qhi.x < lo.x || hi.y < qlo.y || qhi.y < lo.y || hi.z < qlo.z || qhi.z < lo.z);
                 emit = hit && g > f;  // selected leaves have their face's number, the others a negative one
             }
@@ -372,11 +371,11 @@ __device__ __forceinline__ double nearest_d2(bool has, D3 p, const TreeView &T, 
     while (__any_sync(kAll, run)) {
         const int node = 8 * g + gl;
         double d = DBL_MAX;
-        if (run) {
+        if (run && T.holds(lvl, node)) {
             const size_t b = 2 * ((size_t)off[lvl] + node);
             d = box_d2(T.boxes[b], T.boxes[b + 1], p);
             if (lvl == 0) {
-                const int4 t = d < best && node < T.L ? T.leaf[node] : make_int4(0, 0, 0, kLeafDead);
+                const int4 t = d < best ? T.leaf[node] : make_int4(0, 0, 0, kLeafDead);
                 d = t.w != kLeafDead ? point_tri_d2(p, dat(pts[t.x]), dat(pts[t.y]), dat(pts[t.z])) : DBL_MAX;
                 d = fmin(d, DBL_MAX);
             }

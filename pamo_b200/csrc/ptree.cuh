@@ -34,6 +34,11 @@ struct TreeView {
     int top_groups; // groups of eight nodes there (one unless top == kTreeMaxLevels - 1)
     int off[kTreeMaxLevels];
     int count[kTreeMaxLevels];  // nodes that cover a leaf or its tile's padding
+
+    // Whether node i of level l covers a leaf.  Every walk asks: the nodes of the
+    // levels' padding are empty, but a query box that is NaN or infinite on all
+    // axes is apart from none, and the children of padding lie outside the tree.
+    __device__ __forceinline__ bool holds(int l, int i) const { return i <= (L - 1) >> (3 * l); }
 };
 
 // leaf_code: the face of a leaf, and whether it is selected (queries, and not

@@ -1084,11 +1084,11 @@ __global__ void __launch_bounds__(kQueryThreads) k_query(const __grid_constant__
         while (__any_sync(0xffffffffu, wk.run)) {
             bool hit = false, emit = false;
             int other = 0;
-            if (wk.run) {
-                const int node = 8 * wk.g + gl;
+            const int node = 8 * wk.g + gl;
+            if (wk.run && T.holds(wk.lvl, node)) {
                 const size_t b = 2 * ((size_t)s_off[wk.lvl] + node);
                 const float4 lo = T.boxes[b], hi = T.boxes[b + 1];
-                const bool leaf = wk.lvl == 0 && node < T.L;
+                const bool leaf = wk.lvl == 0;
                 const int4 r = leaf ? T.leaf[node] : make_int4(-1, -1, -1, kLeafDead);
                 hit = box_overlap(lo, hi, qlo, qhi);
                 if (BATCH) {

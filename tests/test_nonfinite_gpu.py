@@ -63,3 +63,53 @@ def test_distance_of_non_finite_mesh_matches_plain_search(torch_cuda, m, n_bad, 
     # FP64 on both sides, some dozen roundings of values below 10
     assert abs(got["max"] - d.max()) < 1e-12
     assert abs(got["mean_sq"] - (d**2).mean()) < 1e-12
+
+
+def _boundless(V, F, kind):
+    """Face 0's box made NaN, or all of space, on every axis."""
+    V = V.copy()
+    V[F[0]] = np.nan if kind == "nan" else np.array([[-np.inf] * 3, [np.inf] * 3, [0] * 3], np.float32)
+    return V
+
+
+def _overlaps(V, F):
+    """Pairs f < g whose boxes are not apart."""
+    P = V[F]
+    lo, hi = P.min(1), P.max(1)
+    n = 0
+    for f in range(len(F)):
+        apart = (hi[f + 1:] < lo[f]) | (hi[f] < lo[f + 1:])
+        n += int((~apart.any(1)).sum())
+    return n
+
+
+# the ends of a group, a tile and a level, where padding starts
+@pytest.mark.parametrize("kind", ["nan", "inf"])
+@pytest.mark.parametrize("m", [1, 2, 8, 9, 63, 65, 512, 513, 4095, 4097, 33000])
+def test_face_apart_from_nothing_meets_every_face_once(torch_cuda, m, kind):
+    import pamo_b200
+    from pamo_b200 import metrics
+
+    V, F = _soup(np.random.default_rng(m), m)
+    V = _boundless(V, F, kind)
+    want = _overlaps(V, F)
+    assert want >= m - 1
+    ctx = pamo_b200.Context(0)
+    _, got = pamo_b200.self_intersect(ctx, torch_cuda.from_numpy(V).cuda(), torch_cuda.from_numpy(F).cuda())
+    assert got == want
+    res = metrics.check_mesh(V, F)
+    assert res["degenerate_faces"] in (0, 1)  # such a face may count as degenerate, and is then not tested
+    assert res["candidate_pairs"] == want - (m - 1) * res["degenerate_faces"]
+
+
+@pytest.mark.parametrize("m", [1, 9, 513, 4097, 33000])
+def test_sample_without_coordinates_is_at_no_distance(torch_cuda, m):
+    from pamo_b200 import metrics
+
+    rng = np.random.default_rng(m)
+    V, F = _soup(rng, m)
+    A, FA = _soup(rng, 5)
+    A[FA[2]] = np.nan
+    got = metrics.mesh_distance(A, FA, V, F, subdiv=2)
+    assert got["samples"] == 30
+    assert got["max"] == np.sqrt(np.finfo(np.float64).max)
