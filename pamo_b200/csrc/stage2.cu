@@ -870,11 +870,14 @@ __global__ void __launch_bounds__(kThreads) k_collapse_apply(CollapseArgs A, con
             if constexpr (QUALITY) mid = v3(A.epos[e]);  // the position the edge cost chose
             else mid = vmid(v3(A.opts[u]), v3(A.opts[v]));
         }
-        // the one-rings after the collapse, from the round input (no other winner touches them)
+        // the one-rings after the collapse, from the round input (no other winner touches
+        // them).  A ring lists a face once for each corner there: one that holds v twice
+        // goes, as its second turn finds the u that the first one left.
         auto moved = [&](int i, int &f) {
             f = A.near_tris[(i < du ? ua : va) + i];
             int4 t = A.otris[f];
-            if (face_has(t, i < du ? v : u)) t = make_int4(-1, -1, -1, 0);
+            const int at_v = (t.x == v) + (t.y == v) + (t.z == v);
+            if (face_has(t, i < du ? v : u) || at_v > 1) t = make_int4(-1, -1, -1, 0);
             else if (t.x == v) t.x = u;
             else if (t.y == v) t.y = u;
             else if (t.z == v) t.z = u;
