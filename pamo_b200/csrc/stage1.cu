@@ -907,8 +907,9 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
     S1_TRY(cudaMemsetAsync(dirty[1], 0, (size_t)tiles, s));
     int cur = 0;
     bool settled = false;
-    // a change crosses at least a row a launch: R^2 rows bound the launches
-    for (long long round = 0; round < (long long)R * R + 64 && !settled; round += 6) {
+    // A launch that changes anything sets a bit, so n3 + 1 launches settle any grid; a
+    // surface takes a few, a path that winds between two tiles one per crossing.
+    for (long long round = 0; round <= n3 && !settled; round += 6) {
         for (int k = 0; k < 6; ++k) {
             if (k == 5) S1_TRY(cudaMemsetAsync(S.dev + 4, 0, 4, s));  // settled: nothing changed in the last launch
             launch(k_s1_flood, tiles, kThreads, 0, s, bits, S.dev, (const uint8_t *)dirty[cur], dirty[cur ^ 1]);
@@ -920,7 +921,7 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
         if (S.prof) S.prof->collect();
         settled = S.h_dev[4] == 0;
     }
-    if (!settled) return PAMO_ERR_DEVICE;  // cannot happen within that many launches
+    if (!settled) return PAMO_ERR_DEVICE;  // cannot happen: see above
     launch(k_s1_inside, grid_for(words), kThreads, 0, s, bits);
     // 4. dual marching cubes: patch and quad numbers, then the patch vertices
     if (S.prof) S.prof->begin(PH_S1_DMC, s);
