@@ -232,6 +232,53 @@ __device__ __forceinline__ T classified_distance(int block_kind, int t, const Ve
     }
 }
 
+// A lower bound of the distance between a block's two primitives (x[0] and x[1..3], or
+// x[0..1] and x[2..3]): the gap of their projections on an axis, less its rounding.
+// The axis is the one that the class's closest points lie on, so the gap is the
+// distance where the class is right, and a bound whatever the class: a classified
+// distance is none, as the class can turn on a rounding (pt_classify takes the nearest
+// corner of a triangle below an area).
+__device__ __forceinline__ float axis_gap(int block_kind, int t, const F3 *x)
+{
+    if (t < 0) return 0.f;
+    const TypeInfo ti = type_info(block_kind, t);
+    F3 w;
+    if (ti.kind == 0) {
+        w = x[ti.i0] - x[ti.i1];
+    } else if (ti.kind == 1) {
+        const F3 e = x[ti.i2] - x[ti.i1], p = x[ti.i0] - x[ti.i1];
+        w = p - (dot(p, e) / dot(e, e)) * e;
+    } else if (ti.kind == 2) {
+        w = cross(x[2] - x[1], x[3] - x[1]);
+    } else {
+        w = cross(x[1] - x[0], x[3] - x[2]);
+    }
+    const F3 y1 = x[1] - x[0], y2 = x[2] - x[0], y3 = x[3] - x[0];
+    const float l = len(w), s1 = dot(w, y1), s2 = dot(w, y2), s3 = dot(w, y3);
+    if (!(l > 1e-15f)) return 0.f;  // no axis
+    float alo = 0.f, ahi = 0.f, blo = fmin(s2, s3), bhi = fmax(s2, s3);
+    if (block_kind == KIND_PT) {
+        blo = fmin(blo, s1);
+        bhi = fmax(bhi, s1);
+    } else {
+        alo = fmin(alo, s1);
+        ahi = fmax(ahi, s1);
+    }
+    // some ten roundings of 6e-8 in the projections, relative to the block's size
+    return fmax(blo - ahi, alo - bhi) / l - 1e-6f * (len(y1) + len(y2) + len(y3));
+}
+
+// The CCD ends a block at its first step, slack (d - thick) / lv, if that is beyond 1.
+// lv is the sum of two lengths of a vertex's step less the four's mean, each at most
+// 3/2 of the largest step of a vertex.  A block whose primitives are farther apart
+// than this ends there (without iterations none does; the margins cover the roundings
+// of the step and of this sum).
+__device__ __forceinline__ float ccd_far(float step_bound, float slack, float thick, int max_iters)
+{
+    if (!(slack > 0.f) || max_iters <= 0) return 3e38f;
+    return (3.f * 1.00001f * step_bound / slack + thick) * 1.00001f + 1e-12f;
+}
+
 // distance and its gradient w.r.t. the four block vertices
 __device__ inline float distance_grad(int block_kind, int t, const F3 *x, F3 *g)
 {

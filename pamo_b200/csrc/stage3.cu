@@ -1628,25 +1628,27 @@ __global__ void k_clamp(float4 *p, const float4 *q_prev, const float4 *q_det, in
 
 // Additive CCD (Li et al. 2021) per block, in FP64 (ccd_kernels.py:8-110).
 __global__ void __launch_bounds__(128) k_accd(const float4 *q, const float4 *pv, const int4 *bidx, const int *bkind,
-                                              const float *bd, const int *iscal, long long cap_b, float slack,
+                                              const int *bsub, const int *iscal, long long cap_b, float slack,
                                               float thick, int max_iters, float ee_thres, const float *step_bound,
                                               float *ccd_step)
 {
     const long long nb = min((long long)iscal[I_NB], cap_b);
-    // A first step beyond 1 (below) needs slack (d - thickness) > lv, and lv, the sum
-    // of two lengths of a vertex's step less the four's mean, is at most four times
-    // the largest step.  So a block whose distance at the iterate, from detection, is
-    // beyond `far` is skipped unread (the margins cover the fp32 distance and step).
-    const float far = max_iters > 0 ? 4.f * *step_bound * 1.00001f / slack + thick + 1e-5f : INFINITY;
+    // A block whose primitives are farther apart than this (by their projections on the
+    // axis of the class that detection found at this iterate) ends at its first step.
+    // On 733,000 blocks a pass takes 33 us so, and 50 with the FP64 bound below alone;
+    // detection's distance in place of the gap took 17, but is no bound (axis_gap).
+    const float far = ccd_far(*step_bound, slack, thick, max_iters);
     PAMO_GRID_STRIDE(b, nb)
     {
-        if (bd[b] * 0.99999f > far) continue;
         int4 i = bidx[b];
         int kind = bkind[b];
         int idx[4] = {i.x, i.y, i.z, i.w};
+        F3 xf[4];
+        for (int a = 0; a < 4; ++a) xf[a] = ld(q, idx[a]);
+        if (axis_gap(kind, bsub[b], xf) > far) continue;
         D3 x[4], v[4];
         for (int a = 0; a < 4; ++a) {
-            x[a] = d3(q[idx[a]]);
+            x[a] = {xf[a].x, xf[a].y, xf[a].z};
             v[a] = d3(pv[idx[a]]);
         }
         D3 avg = 0.25 * (v[0] + v[1] + v[2] + v[3]);
@@ -2266,7 +2268,7 @@ int Stage3::newton_body(cudaStream_t s)
     launch(k_clamp, grid_for(np), kThreads, 0, s, p, (const float4 *)q_prev, (const float4 *)q_det, np,
            cfg.contact_detection_radius, fscal + 1);
     launch(k_accd, grid_for(cap_b, 128), 128, 0, s, (const float4 *)q, (const float4 *)p,
-           (const int4 *)bidx, (const int *)bkind, (const float *)bd, (const int *)iscal, cap_b, cfg.ccd_slackness,
+           (const int4 *)bidx, (const int *)bkind, (const int *)bsub, (const int *)iscal, cap_b, cfg.ccd_slackness,
            cfg.ccd_thickness, cfg.ccd_max_iters, cfg.ee_classify_thres, (const float *)(fscal + 1), fscal);
     // line search (system.py:393-409)
     if (prof) prof->begin(PH_S3_LINE, s);
