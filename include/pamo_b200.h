@@ -361,7 +361,8 @@ int pamo_safe_project_trace(pamo_ctx *ctx, double *h_out, int cap_rows, int *out
 /*
  * Test of the library's bounded device waits (no counterpart in the
  * reference).  which = 0: a prefix scan (the single-pass look-back of every
- * stage-2 round) in which one tile never publishes; which = 1: the persistent
+ * stage-2 round) in which one tile never publishes, its fault put before a
+ * batch's compaction, which must report it; which = 1: the persistent
  * CG solve of stage 3 in which one block never publishes its partial sums.
  * The waiting blocks give up after `spin_limit` polls (at most 2^24), record
  * the fault and return; the call then reports what a real run reports for

@@ -986,6 +986,8 @@ int pamo_safe_project_trace(pamo_ctx *ctx, double *h_out, int cap_rows, int *out
     return PAMO_OK;
 }
 
+static int batch_with_scan_fault(int device, const int *d_fault, cudaStream_t s);
+
 int pamo_debug_wait_timeout(pamo_ctx *ctx, int which, long long spin_limit, void *stream)
 {
     if (!ctx || (which != 0 && which != 1) || spin_limit < 0 || spin_limit > (1LL << 24)) return PAMO_ERR_INVALID_ARG;
@@ -993,7 +995,8 @@ int pamo_debug_wait_timeout(pamo_ctx *ctx, int which, long long spin_limit, void
     cudaStream_t s = (cudaStream_t)stream;
     if (which == 0) {
         // a 32-tile scan whose tile 3 never publishes: the tiles after it wait
-        // on it, give up after spin_limit polls and record the fault
+        // on it, give up after spin_limit polls and record the fault, which must end
+        // a round: a batch's compaction, the last to read it, is asked to
         const long long n = 32LL * pamo::kScanTile;
         const long long sc = pamo::scan_scratch_ints(n);
         int *buf = nullptr;
@@ -1004,9 +1007,9 @@ int pamo_debug_wait_timeout(pamo_ctx *ctx, int which, long long spin_limit, void
         if (e == cudaSuccess) e = pamo::exclusive_scan_waits(in, out, n, nullptr, scratch, nullptr, s, fault, spin_limit, 3);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h_fault, fault, 4, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        const int rc = e == cudaSuccess && h_fault ? batch_with_scan_fault(ctx->device, fault, s) : PAMO_OK;
         cudaFree(buf);
-        if (e != cudaSuccess) return map_cuda_error(e);
-        return h_fault ? PAMO_ERR_DEVICE : PAMO_OK;
+        return e != cudaSuccess ? map_cuda_error(e) : rc;
     }
     // the persistent CG with block 1 never publishing its partial sums: every
     // block's wait on that slot gives up, the solve returns with the error
@@ -1457,6 +1460,24 @@ int pamo_batch_destroy(pamo_batch *b)
     if (b->pool) cudaMemPoolDestroy(b->pool);
     delete b;
     return PAMO_OK;
+}
+
+// What a batch's compaction reports when a scan of its round recorded *d_fault (the
+// pamo_debug_wait_timeout test): one mesh of no vertices and no faces.
+static int batch_with_scan_fault(int device, const int *d_fault, cudaStream_t s)
+{
+    pamo_batch *b = nullptr;
+    int rc = pamo_batch_create(device, 4, 4, 1, 0, s, &b);
+    if (rc) return rc;
+    Stage2 &S = b->S;
+    cudaError_t e = cudaMemsetAsync(S.dcnt, 0, sizeof(RoundCounters), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S.slots, 0, sizeof(SlotInfo), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S.gmap, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S.fpos, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&S.dcnt->scan_fault, d_fault, sizeof(int), cudaMemcpyDeviceToDevice, s);
+    rc = e == cudaSuccess ? S.compact_batch(0, 0, 1, s) : map_cuda_error(e);
+    pamo_batch_destroy(b);
+    return rc;
 }
 
 int pamo_batch_submit(pamo_batch *b, const float *points, const int *tris, int n_pts, int n_tris, int on_host,

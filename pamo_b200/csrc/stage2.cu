@@ -1716,19 +1716,27 @@ static cudaError_t isect_pass(Stage2 &S, int m, const int *considered, cudaStrea
     return cudaGetLastError();
 }
 
+// The counters, and with them whatever was copied to the host before, once the
+// stream is done; a fault that a scan recorded since the last time ends the round.
+int Stage2::read_counters(cudaStream_t s)
+{
+    S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
+    S2_TRY(cudaStreamSynchronize(s));
+    prof.collect();
+    return hcnt->scan_fault ? PAMO_ERR_DEVICE : PAMO_OK;
+}
+
 // isect_pass and the counters' copy; once more with a larger pair buffer if the
 // candidates did not fit.
 static int checked_pass(Stage2 &S, int m, const int *considered, cudaStream_t s)
 {
     for (int attempt = 0;; ++attempt) {
         S2_TRY(isect_pass(S, m, considered, s));
-        S2_TRY(cudaMemcpyAsync(S.hcnt, S.dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-        S2_TRY(cudaStreamSynchronize(s));
-        S.prof.collect();
-        if (S.hcnt->scan_fault) return PAMO_ERR_DEVICE;
+        int rc = S.read_counters(s);
+        if (rc) return rc;
         if (S.hcnt->pair_overflow == 0) return PAMO_OK;
         if (attempt > 0) return PAMO_ERR_CAPACITY;
-        const int rc = S.ensure_pairs((long long)S.hcnt->n_pairs + S.hcnt->n_pairs / 2 + 1024);
+        rc = S.ensure_pairs((long long)S.hcnt->n_pairs + S.hcnt->n_pairs / 2 + 1024);
         if (rc) return rc;
         S2_TRY(cudaMemsetAsync(&S.dcnt->n_undo, 0, 5 * sizeof(int), s));  // n_undo to n_hit
     }
@@ -1926,11 +1934,7 @@ int Stage2::compact(int n, int m, cudaStream_t s)
            keep ? tree.leaves : 0, dcnt);
     tree_carried = keep;
     prof.end(s);
-    S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
-    S2_TRY(cudaStreamSynchronize(s));
-    prof.collect();
-    if (hcnt->scan_fault) return PAMO_ERR_DEVICE;
-    return PAMO_OK;
+    return read_counters(s);
 }
 
 }  // namespace pamo
@@ -2119,11 +2123,8 @@ int Stage2::compact_batch(int n, int m, int K, cudaStream_t s)
     launch_chained(k_b_next, grid_for(K), kThreads, 0, s, (const SlotInfo *)slots, (const int *)gmap, (const int *)fpos, scnt,
            K);
     prof.end(s);
-    S2_TRY(cudaMemcpyAsync(hcnt, dcnt, sizeof(RoundCounters), cudaMemcpyDeviceToHost, s));
     S2_TRY(cudaMemcpyAsync(hscnt, scnt, (size_t)K * sizeof(SlotCounters), cudaMemcpyDeviceToHost, s));
-    S2_TRY(cudaStreamSynchronize(s));
-    prof.collect();
-    return PAMO_OK;
+    return read_counters(s);
 }
 
 }  // namespace pamo

@@ -196,6 +196,7 @@ struct Stage2 {
     // -1,-1,-1) and undo entries outside [0, undo_hi]; nothing else runs on bad input.
     int validate(const int *d_tris_aos3, int n, int m, const int *d_undo, int n_undo, int undo_hi, cudaStream_t s);
     int ensure_pairs(long long n);
+    int read_counters(cudaStream_t s);  // into hcnt; PAMO_ERR_DEVICE if a scan recorded a fault
     void release();
 
     // One round on opts/otris (already holding the input; init shuffle applied
