@@ -214,12 +214,6 @@ __global__ void __launch_bounds__(kThreads) k_karras(const uint32_t *keys, const
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_leaf_map(const int *vals, const int *scene, int *leaf_of_face, int m)
-{
-    const int L = scene[7];
-    PAMO_GRID_STRIDE(p, m) leaf_of_face[vals[p]] = p < L ? (int)p : -1;
-}
-
 __device__ __forceinline__ void store_child_box(BvhNode *nodes, int code, int self, float3 lo, float3 hi)
 {
     int par = code >> 2;
@@ -318,7 +312,6 @@ cudaError_t Lbvh::ensure(long long n)
     ALLOC(nodes, c * sizeof(BvhNode));
     ALLOC(parent, 2 * c * 4);
     ALLOC(flags, c * 4);
-    ALLOC(leaf_of_face, c * 4);
     ALLOC(scene, 64);
 #undef ALLOC
     cap = c;
@@ -327,14 +320,14 @@ cudaError_t Lbvh::ensure(long long n)
 
 void Lbvh::release()
 {
-    void *p[] = {keys, keys2, vals, vals2, hist, hist_scratch, nodes, parent, flags, leaf_of_face, scene};
+    void *p[] = {keys, keys2, vals, vals2, hist, hist_scratch, nodes, parent, flags, scene};
     for (void *q : p)
         if (q) cudaFree(q);
     keys = keys2 = nullptr;
     vals = vals2 = nullptr;
     hist = hist_scratch = nullptr;
     nodes = nullptr;
-    parent = flags = leaf_of_face = scene = nullptr;
+    parent = flags = scene = nullptr;
     cap = 0;
     leaves_built = 0;
 }
@@ -380,7 +373,6 @@ cudaError_t lbvh_build(Lbvh &b, const float4 *pts, const int4 *tris, int m, cuda
     if (m == 0) return cudaGetLastError();
     launch(k_count_leaves, 1, 1, 0, s, m, b.scene);
     launch(k_karras, grid_for(m), kThreads, 0, s, b.keys, b.scene, b.nodes, b.parent);
-    launch(k_leaf_map, grid_for(m), kThreads, 0, s, b.vals, b.scene, b.leaf_of_face, m);
     return cudaGetLastError();
 }
 

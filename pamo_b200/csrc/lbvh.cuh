@@ -1,4 +1,4 @@
-// Linear BVH over the faces of a mesh (stage 3 and the acceptance checks).
+// Morton order of a mesh's faces, and the linear BVH of stage 3 over it.
 //
 // Build: 30-bit Morton code of each face's box centre (10 bits per axis over the
 // scene box) -> stable LSD radix sort (4 x 8-bit digits, hand written) ->
@@ -7,13 +7,10 @@
 // so traversal reads one node per step and tests the two children.
 //
 // The leaf set is fixed per build (faces live at the build, sorted by their
-// geometry then); a caller that removes and renumbers faces may keep the tree by
-// rewriting the leaves' face indices (-1 for a removed face).  Refit recomputes every leaf box from the current
-// geometry (a dead face gets the empty box lo=+inf, hi=-inf, which overlaps
-// nothing) and rebuilds the inner boxes.
+// geometry then).  Refit recomputes every leaf box from the current geometry (a dead
+// face gets the empty box lo=+inf, hi=-inf, which overlaps nothing) and rebuilds the
+// inner boxes.
 #pragma once
-
-#include <cooperative_groups.h>
 
 #include "common.cuh"
 
@@ -49,7 +46,6 @@ struct Lbvh {
     // run of kRefitTile leaves (merged in shared memory by k_refit)
     int *parent = nullptr;
     int *flags = nullptr;       // [cap] refit arrival counters
-    int *leaf_of_face = nullptr;  // [cap]: sorted position of each face, -1 if not a leaf
     int *scene = nullptr;       // 6 ordered ints + n_dead + n_leaves
     int sort_tiles = 0;
     long long leaves_built = 0;  // faces of the last build: bound on the leaf count
@@ -72,8 +68,7 @@ cudaError_t morton_order(const float4 *pts, const int4 *tris, int m, int *scene,
 // (the round input), ordered by the Morton code of their box centre.
 cudaError_t lbvh_build(Lbvh &b, const float4 *pts, const int4 *tris, int m, cudaStream_t s);
 
-// Recomputes all boxes from the current geometry (pts, tris).  A leaf whose face
-// index is negative (a face removed after the build) gets the empty box.
+// Recomputes all boxes from the current geometry (pts, tris).
 cudaError_t lbvh_refit(Lbvh &b, const float4 *pts, const int4 *tris, int m, cudaStream_t s);
 
 }  // namespace pamo

@@ -16,7 +16,7 @@
 //   scan/scatter  collapsed list in edge order
 //   face pass     degenerate faces removed                           [:218-232]
 //   edge pass     coincident-endpoint collapses                      [:234-274]
-//   LBVH          build over the round's faces, refit, query of the faces touched
+//   packed tree   build over the round's faces, refit, query of the faces touched
 //                 by collapses, pair tests                           [bvh/self_intersect.cuh]
 //   undo passes   candidates, restore, re-check (<= 5)               [:776-878,1015-1040]
 //   scan          pts_map = exclusive scan of occupancy              [:1042-1045]
@@ -24,7 +24,6 @@
 // the minimum over every face touching either endpoint (the reference's per-face
 // minimum), which equals: key == vmin[u] == vmin[v] and no vertex of those faces
 // has a smaller vmin.
-#include <cooperative_groups.h>
 #include <cstdio>
 #include <cstring>
 
@@ -40,8 +39,6 @@ namespace pamo {
         cudaError_t _e = (expr);                          \
         if (_e != cudaSuccess) return map_cuda_error(_e); \
     } while (0)
-
-namespace cg = cooperative_groups;
 
 namespace {
 
