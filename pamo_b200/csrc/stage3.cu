@@ -1635,7 +1635,7 @@ __global__ void __launch_bounds__(128) k_accd(const float4 *q, const float4 *pv,
     const long long nb = min((long long)iscal[I_NB], cap_b);
     // A block whose primitives are farther apart than this (by their projections on the
     // axis of the class that detection found at this iterate) ends at its first step.
-    // On 733,000 blocks a pass takes 33 us so, and 50 with the FP64 bound below alone;
+    // On 733,000 blocks a pass takes 25 us so, and 50 with the FP64 bound below alone;
     // detection's distance in place of the gap took 17, but is no bound (axis_gap).
     const float far = ccd_far(*step_bound, slack, thick, max_iters);
     PAMO_GRID_STRIDE(b, nb)
