@@ -347,6 +347,47 @@ struct CostArgs {
     float4 *epos;
 };
 
+// What both forms of the edge cost make of the sums over an edge's one-rings.
+// The length term: the mean of the nedge edges there, whose lengths add up to sum, and
+// the edge's own.
+__device__ __forceinline__ float edge_length_term(float sum, int nedge, V3 v0, V3 v1, float tres, float edge_s)
+{
+    const float mean = sum / (float)nedge / edge_s * tres;
+    return mean + vnorm(vsub(v0, v1)) / edge_s * tres;
+}
+
+// The cost: the quadric's error at mid, the length term and the ntri skinny terms,
+// which add up to Qa.
+template <bool QUALITY>
+__device__ __forceinline__ uint32_t edge_cost_sum(const CostArgs &A, int u, int v, V3 mid, float elen, float Qa,
+                                                  int ntri, float tres, float edge_s)
+{
+    Qa = 5.0f * Qa;
+    if constexpr (QUALITY) {  // the quadric error in FP64 at the chosen position
+        const double *qu = A.quad64 + 10 * (size_t)u, *qv = A.quad64 + 10 * (size_t)v;
+        double q[10];
+        for (int k = 0; k < 10; ++k) q[k] = qu[k] + qv[k];
+        const double x = mid.x, y = mid.y, z = mid.z;
+        const double qe = x * (q[0] * x + q[1] * y + q[2] * z + q[3]) + y * (q[1] * x + q[4] * y + q[5] * z + q[6]) +
+                          z * (q[2] * x + q[5] * y + q[7] * z + q[8]) + (q[3] * x + q[6] * y + q[8] * z + q[9]);
+        const float cost = (float)(qe / ((double)edge_s * (double)edge_s));
+        return quantise_cost(cost + elen + Qa / (float)ntri * tres);
+    }
+    float4 a0 = A.quad[3 * u], a1 = A.quad[3 * u + 1], a2 = A.quad[3 * u + 2];
+    float4 b0 = A.quad[3 * v], b1 = A.quad[3 * v + 1], b2 = A.quad[3 * v + 2];
+    float m00 = a0.x + b0.x, m01 = a0.y + b0.y, m02 = a0.z + b0.z, m03 = a0.w + b0.w;
+    float m11 = a1.x + b1.x, m12 = a1.y + b1.y, m13 = a1.z + b1.z, m22 = a1.w + b1.w;
+    float m23 = a2.x + b2.x, m33 = a2.y + b2.y;
+    float x = mid.x, y = mid.y, z = mid.z, w = 1.0f;
+    float r0 = m00 * x + m01 * y + m02 * z + m03 * w;
+    float r1 = m01 * x + m11 * y + m12 * z + m13 * w;
+    float r2 = m02 * x + m12 * y + m22 * z + m23 * w;
+    float r3 = m03 * x + m13 * y + m23 * z + m33 * w;
+    float qe = r0 * x + r1 * y + r2 * z + r3 * w;
+    float cost = qe / (edge_s * edge_s);
+    return quantise_cost(cost + elen + Qa / (float)ntri * tres);
+}
+
 // Returns true when the reference writes a new cost for the edge.  QUALITY:
 // quality mode (FP64 quadric terms and the chosen collapse position in epos);
 // compiled separately so the reference's path carries none of it.
@@ -393,8 +434,7 @@ __device__ bool edge_cost_value(const CostArgs &A, int u, int v, bool inv_u, boo
         }
     }
     V3 v0 = v3(A.pts[u]), v1 = v3(A.pts[v]);
-    elen = elen / (float)nedge / edge_s * tres;
-    elen = elen + vnorm(vsub(v0, v1)) / edge_s * tres;
+    elen = edge_length_term(elen, nedge, v0, v1, tres, edge_s);
     // the collapse position: the midpoint (the reference), or in quality mode
     // the FP64 quadric's minimiser
     V3 mid;
@@ -429,31 +469,7 @@ __device__ bool edge_cost_value(const CostArgs &A, int u, int v, bool inv_u, boo
             ntri++;
         }
     }
-    Qa = 5.0f * Qa;
-    if constexpr (QUALITY) {  // the quadric error in FP64 at the chosen position
-        const double *qu = A.quad64 + 10 * (size_t)u, *qv = A.quad64 + 10 * (size_t)v;
-        double q[10];
-        for (int k = 0; k < 10; ++k) q[k] = qu[k] + qv[k];
-        const double x = mid.x, y = mid.y, z = mid.z;
-        const double qe = x * (q[0] * x + q[1] * y + q[2] * z + q[3]) + y * (q[1] * x + q[4] * y + q[5] * z + q[6]) +
-                          z * (q[2] * x + q[5] * y + q[7] * z + q[8]) + (q[3] * x + q[6] * y + q[8] * z + q[9]);
-        const float cost = (float)(qe / ((double)edge_s * (double)edge_s));
-        out = quantise_cost(cost + elen + Qa / (float)ntri * tres);
-        return true;
-    }
-    float4 a0 = A.quad[3 * u], a1 = A.quad[3 * u + 1], a2 = A.quad[3 * u + 2];
-    float4 b0 = A.quad[3 * v], b1 = A.quad[3 * v + 1], b2 = A.quad[3 * v + 2];
-    float m00 = a0.x + b0.x, m01 = a0.y + b0.y, m02 = a0.z + b0.z, m03 = a0.w + b0.w;
-    float m11 = a1.x + b1.x, m12 = a1.y + b1.y, m13 = a1.z + b1.z, m22 = a1.w + b1.w;
-    float m23 = a2.x + b2.x, m33 = a2.y + b2.y;
-    float x = mid.x, y = mid.y, z = mid.z, w = 1.0f;
-    float r0 = m00 * x + m01 * y + m02 * z + m03 * w;
-    float r1 = m01 * x + m11 * y + m12 * z + m13 * w;
-    float r2 = m02 * x + m12 * y + m22 * z + m23 * w;
-    float r3 = m03 * x + m13 * y + m23 * z + m33 * w;
-    float qe = r0 * x + r1 * y + r2 * z + r3 * w;
-    float cost = qe / (edge_s * edge_s);
-    out = quantise_cost(cost + elen + Qa / (float)ntri * tres);
+    out = edge_cost_sum<QUALITY>(A, u, v, mid, elen, Qa, ntri, tres, edge_s);
     return true;
 }
 
@@ -641,33 +657,8 @@ __device__ __forceinline__ bool edge_cost_group(const CostArgs &A, bool has, int
     const bool any_flip = (__ballot_sync(kAll, flip) >> shift & 255u) != 0;
     if (!live) return written;
     if (any_flip) return true;
-    elen = elen / (float)nedge / edge_s * tres;
-    elen = elen + vnorm(vsub(v0, v1)) / edge_s * tres;
-    Qa = 5.0f * Qa;
-    if constexpr (QUALITY) {  // the quadric error in FP64 at the chosen position
-        const double *qu = A.quad64 + 10 * (size_t)u, *qv = A.quad64 + 10 * (size_t)v;
-        double q[10];
-        for (int k = 0; k < 10; ++k) q[k] = qu[k] + qv[k];
-        const double x = mid.x, y = mid.y, z = mid.z;
-        const double qe = x * (q[0] * x + q[1] * y + q[2] * z + q[3]) + y * (q[1] * x + q[4] * y + q[5] * z + q[6]) +
-                          z * (q[2] * x + q[5] * y + q[7] * z + q[8]) + (q[3] * x + q[6] * y + q[8] * z + q[9]);
-        const float cost = (float)(qe / ((double)edge_s * (double)edge_s));
-        out = quantise_cost(cost + elen + Qa / (float)ntri * tres);
-        return true;
-    }
-    float4 a0 = A.quad[3 * u], a1 = A.quad[3 * u + 1], a2 = A.quad[3 * u + 2];
-    float4 b0 = A.quad[3 * v], b1 = A.quad[3 * v + 1], b2 = A.quad[3 * v + 2];
-    float m00 = a0.x + b0.x, m01 = a0.y + b0.y, m02 = a0.z + b0.z, m03 = a0.w + b0.w;
-    float m11 = a1.x + b1.x, m12 = a1.y + b1.y, m13 = a1.z + b1.z, m22 = a1.w + b1.w;
-    float m23 = a2.x + b2.x, m33 = a2.y + b2.y;
-    float x = mid.x, y = mid.y, z = mid.z, w = 1.0f;
-    float r0 = m00 * x + m01 * y + m02 * z + m03 * w;
-    float r1 = m01 * x + m11 * y + m12 * z + m13 * w;
-    float r2 = m02 * x + m12 * y + m22 * z + m23 * w;
-    float r3 = m03 * x + m13 * y + m23 * z + m33 * w;
-    float qe = r0 * x + r1 * y + r2 * z + r3 * w;
-    float cost = qe / (edge_s * edge_s);
-    out = quantise_cost(cost + elen + Qa / (float)ntri * tres);
+    elen = edge_length_term(elen, nedge, v0, v1, tres, edge_s);
+    out = edge_cost_sum<QUALITY>(A, u, v, mid, elen, Qa, ntri, tres, edge_s);
     return true;
 }
 
@@ -1748,12 +1739,18 @@ static cudaError_t undo_list_of(Stage2 &S, int *pos, cudaStream_t s)
                     s, &S.dcnt->scan_fault);
 }
 
-// A thread per edge follows a chain of a dozen faces (~33 us a pass at least,
-// however few the edges); a group of eight lanes halves that chain's time several
-// times over but spends ~1.3 times the instructions, as a ring of six leaves two
-// lanes idle.  The pass over a mesh of a few thousand faces takes 23 us by groups
-// and 44 by threads, that over 2M faces 1.3 times as long by groups; the two meet
-// near 100,000 faces (50,000 in quality mode, whose FP64 terms groups repeat).
+// A thread per edge follows a chain of a dozen faces (45 us a pass at least, however
+// few the edges); a group of eight lanes follows it in two steps, but spends more
+// instructions, as a ring of six leaves two lanes idle and FP64 terms are repeated.
+// The first rounds of a torus take, us a pass by threads / by groups,
+//   10k 47/25   34k 48/32   63k 54/53   80k 59/67   100k 60/75   200k 112/132   800k 344/485
+//   in quality mode  10k 49/30   34k 50/40   43k 54/57   50k 55/63   100k 63/97   800k 457/651
+// and later rounds, whose rings are uneven, favour the groups more.  Over whole loops
+// the passes add up, by the limit (all by threads, 50k, 64k, 80k, 100k, 130k, all by
+// groups), to 23.8, 22.8, 22.7, 22.6, 22.6, 22.7, 29.4 ms for a torus of 2M faces and
+// 4.35, 3.73, 3.72, 3.75, 3.77, 3.82, 4.14 for a sphere of 328k; in quality mode (30k,
+// 40k, 50k, 64k) to 30.8, 30.8, 30.7, 30.8 and 4.56, 4.53, 4.54, 4.59: flat about the
+// limits chosen.  A batch counts its packed faces, which is what fills the device.
 template <bool QUALITY>
 static void launch_edge_cost(const CostArgs &A, const int *order, int m, int L, const int *first_edge, cudaStream_t s)
 {
