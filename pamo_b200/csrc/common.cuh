@@ -64,7 +64,10 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
 // after another was a sixth of it: simplifying 5k faces 11.3 -> 9.6 ms, a batch of
 // 32 meshes 297 -> 261 ms.  A grid of more than kChainBlocks blocks is launched
 // plainly: set up early, its blocks land on the multiprocessors as they fall free
-// and stay where they are, unevenly (2M faces 70.1 -> 73.2 ms; 69.5 with the limit).
+// and stay where they are, unevenly.  Simplifying with the limit at 0 / 148 / 592 /
+// 888 / none takes 5.2 / 4.4 / 4.4 / 4.4 / 4.4 ms at 5k faces, 7.04 / 6.85 / 6.71 /
+// 6.71 / 6.86 at 100k, 11.4 / 11.3 / 11.4 / 11.4 / 11.5 at 350k and 38.1 / 38.1 /
+// 38.1 / 38.1 / 40.1 at 2M.
 constexpr unsigned kChainBlocks = 4 * kNumSMs;
 
 template <typename... KArgs, typename... Args>
