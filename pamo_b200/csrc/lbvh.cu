@@ -1,4 +1,7 @@
 #include "lbvh.cuh"
+
+#include <type_traits>
+
 #include "scan.cuh"
 
 namespace pamo {
@@ -316,6 +319,42 @@ cudaError_t Lbvh::ensure(long long n)
 #undef ALLOC
     cap = c;
     return cudaSuccess;
+}
+
+// one array after another from `at`, or from 0 to find the size
+static size_t lbvh_lay_out(Lbvh &b, unsigned char *at, long long n)
+{
+    size_t used = 0;
+    auto take = [&](auto *&p, size_t bytes) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(at + used);
+        used += (bytes + 255) & ~size_t(255);
+    };
+    const long long hist = 256 * ((n + kSortTile - 1) / kSortTile);
+    take(b.nodes, (size_t)n * sizeof(BvhNode));
+    take(b.keys, (size_t)n * 4);
+    take(b.keys2, (size_t)n * 4);
+    take(b.vals, (size_t)n * 4);
+    take(b.vals2, (size_t)n * 4);
+    take(b.hist, (size_t)hist * 4);
+    take(b.hist_scratch, (size_t)scan_scratch_ints(hist) * 4);
+    take(b.parent, (size_t)n * 8);
+    take(b.flags, (size_t)n * 4);
+    take(b.scene, 64);
+    return used;
+}
+
+size_t Lbvh::bytes(long long n)
+{
+    Lbvh b;
+    return lbvh_lay_out(b, nullptr, n);
+}
+
+cudaError_t Lbvh::place(void *memory, long long n, cudaStream_t s)
+{
+    lbvh_lay_out(*this, static_cast<unsigned char *>(memory), n);
+    cap = n;
+    leaves_built = 0;
+    return scan_scratch_init(hist_scratch, scan_scratch_ints(256 * ((n + kSortTile - 1) / kSortTile)), s);
 }
 
 void Lbvh::release()

@@ -1,4 +1,5 @@
-// Morton order of a mesh's faces, and the linear BVH of stage 3 over it.
+// Morton order of a mesh's faces, and the linear BVH over it (stage 3 and the mesh
+// distance of many samples).
 //
 // Build: 30-bit Morton code of each face's box centre (10 bits per axis over the
 // scene box) -> stable LSD radix sort (4 x 8-bit digits, hand written) ->
@@ -51,6 +52,10 @@ struct Lbvh {
     long long leaves_built = 0;  // faces of the last build: bound on the leaf count
 
     cudaError_t ensure(long long n_faces);
+    // the arrays in the caller's memory (bytes(n) of it, 256-byte aligned) instead;
+    // such a hierarchy is not released
+    cudaError_t place(void *memory, long long n_faces, cudaStream_t s);
+    static size_t bytes(long long n_faces);
     void release();
 };
 
