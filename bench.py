@@ -344,16 +344,16 @@ def _sample_fraction(args, sample_rounds):
 
 
 def roofline_edge_cost(phases, round_faces, peaks):
-    """HBM roofline of the edge-cost kernel (one launch per round).
+    """HBM roofline of the edge cost (one launch per round: k_edge_cost above
+    100,000 faces, k_edge_cost_group up to there).
 
     Algorithmic bytes per round with F faces (closed mesh: E = 1.5 F edges,
     V = 0.5 F vertices), each array read or written once: edges 8 B/edge,
     cost write 4 B/edge, CSR offsets 4 B/vertex, CSR entries 12 B/face, faces
     (int4) 16 B/face, points (float4) 16 B/vertex, quadrics 48 B/vertex,
     invalid flags 1 B/vertex, per-vertex key minimum read+write 16 B/vertex:
-    12 E + 85 V + 28 F = 88.5 B/face.  Traffic: DRAM bytes per face of the
-    round-0 launch on config 2 (ncu, profiles/stage2_kernels_c2_first_collapse_round.txt),
-    times the average faces per launch."""
+    12 E + 85 V + 28 F = 88.5 B/face.  Traffic: the captured DRAM bytes per face
+    (edge_cost_dram_bytes), averaged over the launches."""
     ph = phases.get("edge_cost")
     if not ph or not ph["ms"] or not round_faces:
         return None
@@ -361,19 +361,29 @@ def roofline_edge_cost(phases, round_faces, peaks):
     t = ph["ms"] / 1e3
     achieved = total_bytes / t / 1e9
     peak = peaks.get("hbm_gbs") or 6650.0
-    avg_faces = sum(round_faces) / max(len(round_faces), 1)
-    return {"bound": "hbm", "kernel": "k_edge_cost", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak,
-            "traffic": EDGE_COST_DRAM_BYTES_PER_FACE * avg_faces if EDGE_COST_DRAM_BYTES_PER_FACE else None,
+    by_groups = sum(f <= 100_000 for f in round_faces)
+    return {"bound": "hbm", "kernel": "k_edge_cost, k_edge_cost_group", "achieved": achieved, "peak": peak,
+            "unit": "GB/s", "frac": achieved / peak, "launches_by_groups": by_groups,
+            "traffic": sum(edge_cost_dram_bytes(f) for f in round_faces) / len(round_faces),
             "launches": ph["calls"], "avg_launch_ms": ph["ms"] / max(ph["calls"], 1),
             "bytes_per_launch_avg": total_bytes / max(ph["calls"], 1),
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks.get("hbm_gbs") else "fallback"}
 
 
-# DRAM read + write of k_edge_cost per input face of the launch, from an ncu
-# capture of round 0 of config 2 (2,097,152 faces): 904.0 MB read + 57.0 MB
-# written; profiles/stage2_kernels_c2_first_collapse_round.txt.
-EDGE_COST_DRAM_BYTES_PER_FACE = 458.2
+def edge_cost_dram_bytes(faces):
+    """DRAM read + write of an edge-cost launch, from ncu captures: 464.9 B/face on
+    2,097,152 faces, whose arrays exceed the L2
+    (profiles/stage2_kernels_c2_first_collapse_round.txt); 130.9 B/face on 131,072
+    (k_edge_cost) and 138.7 on 95,578 (k_edge_cost_group), whose arrays a cold L2
+    reads once (profiles/stage2_stage3_kernels_torus256_stages23.txt).  The line
+    between is drawn at 500,000 faces (about 126 MB of round arrays)."""
+    return (464.9 if faces > 500_000 else 130.9 if faces > 100_000 else 138.7) * faces
+
+
+# DRAM read + write of k_query per input face, from an ncu capture of round 0 on
+# 2,097,152 faces: 90.0 MB read + 10.0 MB written;
+# profiles/stage2_kernels_c2_first_collapse_round.txt.
+QUERY_DRAM_BYTES_PER_FACE = 47.7
 
 
 def roofline_query(phases, round_faces, peaks):
@@ -393,7 +403,7 @@ def roofline_query(phases, round_faces, peaks):
     achieved = total_bytes / t / 1e9
     peak = peaks.get("hbm_gbs") or 6650.0
     return {"bound": "hbm", "kernel": "k_query", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "traffic": None,  # not captured for this kernel
+            "frac": achieved / peak, "traffic": QUERY_DRAM_BYTES_PER_FACE * sum(round_faces) / len(round_faces),
             "launches": ph["calls"], "avg_launch_ms": ph["ms"] / max(ph["calls"], 1),
             "bytes_per_launch_avg": total_bytes / max(len(round_faces), 1),
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks.get("hbm_gbs") else "fallback"}

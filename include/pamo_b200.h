@@ -381,7 +381,7 @@ int pamo_bsr_pcg(pamo_ctx *ctx, int n, const int *d_row_ptr, const int *d_col, c
  * library do it: a host application that owns all device memory through its own
  * pool, or a latency-critical loop where cudaMalloc/cudaFree would synchronise
  * the device and stall its other streams.  Same inputs and output as
- * pamo_self_intersect, with no context.  All scratch lives in one ~11 MB
+ * pamo_self_intersect, with no context.  All scratch lives in one ~10 MB
  * file-scope device array that every GPU loading the library holds until the
  * process exits.  Limits: n_tris <= 32768, n_pts <= 65536 and at most 786,432
  * candidate pairs (box-overlapping face pairs) in total; larger inputs return

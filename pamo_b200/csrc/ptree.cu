@@ -52,10 +52,9 @@ __device__ __forceinline__ Box union8(Box b)
 // nodes of levels 1-3 (unions over eight lanes at a time), and the last block to
 // finish (a ticket, no waiting) does the levels above, one launch's worth of
 // latency instead of one atomic per node on the way up.  Bound by latency on
-// small meshes, by the leaves' gathers on large ones: 11 / 13 / 24 us a pass with
+// small meshes, by the leaves' gathers on large ones: 9 / 12 / 18 us a pass with
 // the query list, mean over the rounds of meshes of 5k / 200k / 2M faces, against
-// 27 / 44 / 84 us for the bottom-up refit of the binary hierarchy (22 / 39 / 74
-// in its kernel) and a launch for the list.
+// 29 / 44 / 83 us for the bottom-up refit of the binary hierarchy.
 __global__ void __launch_bounds__(kTreeTile) k_tree_refit(const __grid_constant__ TreeView T,
                                                           const float4 *__restrict__ pts,
                                                           const int4 *__restrict__ tris,

@@ -414,7 +414,7 @@ __device__ __forceinline__ uint32_t spread(uint32_t o, uint32_t f)
 // previous launch; all tiles in the first) do the work; a tile that changes marks
 // itself and its four neighbours in `dirty_out`.  Rows start outside at both
 // ends, so a few launches settle the grid.  With a byte per sample in 8^3 tiles a
-// launch took 66 us at R = 256; this one takes 5.
+// launch took 66 us at R = 256; this one takes 6 to 22, 12 on average.
 __global__ void __launch_bounds__(kThreads) k_s1_flood(Bits B, int *dev, const uint8_t *dirty_in, uint8_t *dirty_out)
 {
     __shared__ uint32_t o[(kTile + 2) * (kTile + 2)][kMaxWords];

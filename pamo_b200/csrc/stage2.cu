@@ -134,7 +134,7 @@ __device__ __forceinline__ int next_after(int4 t, int v);
 // entries over the planes in order.  One thread per vertex sorted its segment by
 // insertion in global memory and then followed the faces one by one, which made
 // the round's setup 32 / 59 / 94 us on meshes of 5k / 200k / 2M faces (mean over
-// the rounds); it is 27 / 52 / 92 us so.
+// the rounds); it was 27 / 52 / 92 us so, and is 21 / 48 / 91 with chained launches.
 constexpr int kRing = 32;  // longer segments are sorted and summed by one lane
 
 __global__ void __launch_bounds__(kThreads) k_vertex_quadric(const int *__restrict__ first_near, int *near_tris,
@@ -1026,9 +1026,9 @@ __device__ __forceinline__ int shared_indices(int4 a, int4 b)
 //
 // A walk is a chain of dependent loads, so its length sets the time: one thread
 // per query on a binary hierarchy followed ~100 nodes and loaded each leaf's
-// face, flag and corners one after another (81 / 141 / 239 us a pass, mean over
-// the rounds of meshes of 5k / 200k / 2M faces).  Here a step tests eight boxes,
-// and a leaf's record comes with its box: 18 / 28 / 82 us.  The pairs gather in
+// face, flag and corners one after another (90 / 120 / 222 us a pass with its query
+// list, mean over the rounds of meshes of 5k / 200k / 2M faces).  Here a step tests
+// eight boxes, and a leaf's record comes with its box: 19 / 27 / 83 us.  The pairs gather in
 // shared memory and leave 32 at a time, one counter update for each 32.
 constexpr int kQueryThreads = 256;
 
