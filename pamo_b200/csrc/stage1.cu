@@ -15,7 +15,7 @@
 //      warp per triangle walks the samples of its box grown by two voxels and
 //      lowers the sample's squared distance with a 64-bit atomic minimum (the
 //      bits of a non-negative double order like the value).  Two voxels of the
-//      band's three are enough for the same result: see kReach;
+//      band's three give the same result where the triangles have areas: see kReach;
 //   3. sign by flood fill: samples farther than half a voxel from every
 //      triangle are free, free samples 6-connected to the grid boundary are
 //      outside; the field is +-distance - 0.9/R.  From here on the grid is bits,
@@ -172,27 +172,51 @@ __global__ void k_s1_max(const float *pts, const int *tris, int m, const float *
     if ((threadIdx.x & 31) == 0) atomicMax(&dev[3], float_to_ordered(hi));
 }
 
-__global__ void k_s1_normalise(const float *pts, const int *tris, int m, const float *mean, const int *dev,
-                               float band, float margin, float *out)
+struct D3 {
+    double x, y, z;
+};
+__device__ __forceinline__ D3 dsub(D3 a, D3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ double ddot(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+
+// Whether point_tri_d2 gives the triangle's distances to 0.03 voxels at every sample
+// within the band (all that kReach needs).  Its barycentric terms are differences of
+// products of the size |ab| |ac| D^2, D <= L + 3 sqrt(3) / R being a sample's distance
+// from a corner and L the longest edge; some 160 roundings of 1.1e-16 of that size,
+// over the squared normal and times L, bound the closest point's error (here with a
+// factor of two, squared, and D^2 <= 2 (L^2 + 27 / R^2)).  A triangle without an area
+// gives NaN on one side of its line, a single point its distance.
+__device__ __forceinline__ bool distances_hold(const float *T, int R)
+{
+    const D3 a = {T[0], T[1], T[2]}, b = {T[3], T[4], T[5]}, c = {T[6], T[7], T[8]};
+    const D3 ab = dsub(b, a), ac = dsub(c, a), bc = dsub(c, b);
+    const D3 n = {ab.y * ac.z - ab.z * ac.y, ab.z * ac.x - ab.x * ac.z, ab.x * ac.y - ab.y * ac.x};
+    const double ab2 = ddot(ab, ab), ac2 = ddot(ac, ac), l2 = fmax(fmax(ab2, ac2), ddot(bc, bc)), nn = ddot(n, n);
+    const double k = 4e-14 * R / 0.03, d2 = l2 + 27.0 / ((double)R * R);
+    return (nn > 0.0 && 4.0 * k * k * ab2 * ac2 * l2 * d2 * d2 <= nn * nn) || l2 == 0.0;
+}
+
+// the triangles in the unit cube; dev[5]: one of them has distances that do not hold
+__global__ void k_s1_normalise(const float *pts, const int *tris, int m, const float *mean, int *dev,
+                               float band, float margin, int R, float *out)
 {
     float lo[3];
     for (int k = 0; k < 3; ++k) lo[k] = ordered_to_float(dev[k]);
     const float mx = ordered_to_float(dev[3]);
     PAMO_GRID_STRIDE(f, m)
     {
+        float T[9];
         for (int c = 0; c < 3; ++c) {
             const int v = tris[3 * f + c];
-            for (int k = 0; k < 3; ++k) out[9 * f + 3 * c + k] = (((pts[3 * v + k] - mean[k]) - lo[k]) / mx + band) / margin;
+            for (int k = 0; k < 3; ++k) {
+                T[3 * c + k] = (((pts[3 * v + k] - mean[k]) - lo[k]) / mx + band) / margin;
+                out[9 * f + 3 * c + k] = T[3 * c + k];
+            }
         }
+        if (!distances_hold(T, R)) dev[5] = 1;
     }
 }
 
 // ------------------------------------------------------- 2. unsigned distance
-struct D3 {
-    double x, y, z;
-};
-__device__ __forceinline__ D3 dsub(D3 a, D3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ double ddot(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 
 // squared distance from p to triangle abc; the closest point by the Voronoi
 // regions of the triangle (Ericson, Real-Time Collision Detection, 5.1.5), with
@@ -240,7 +264,10 @@ __device__ double point_tri_d2(D3 p, D3 a, D3 b, D3 c)
 // near (within 0.5), or free but not reached -- which no neighbour of an outside
 // sample is.  Distances of neighbours differ by at most a voxel, so B's is below
 // 1.9, and both ends lie within 2.  Any value of 2 or more in a farther sample
-// gives the same bits: free, and not within 0.9.  Against the band's 3 voxels a
+// gives the same bits: free, and not within 0.9.  That neighbours differ by a voxel
+// holds for distances, so for computed ones where they are distances: a triangle
+// without an area gives none on one side (NaN, dropped by the minimum), and one such
+// triangle takes the whole mesh back to the band (distances_hold).  Against 3 voxels a
 // small triangle's box has a third of the samples: 2.7 -> 1.6 ms for 500,000 faces
 // at R = 256, 8.8 -> 4.9 ms for 2,000,000.
 constexpr double kReach = 2.0;
@@ -258,9 +285,10 @@ __device__ __forceinline__ double s1_coord(int i, int R, double inv_r)
     return inv_r > 0.0 ? (i + 0.5) * inv_r : (i + 0.5) / R;
 }
 
-__global__ void __launch_bounds__(256, 3) k_s1_udist(const float *tris, int m, int R, double inv_r, double reach,
-                                                  unsigned long long *field)
+__global__ void __launch_bounds__(256, 3) k_s1_udist(const float *tris, int m, int R, double inv_r, double band,
+                                                  const int *dev, unsigned long long *field)
 {
+    const double reach = dev[5] ? band : kReach / R;
     const int lane = threadIdx.x & 31;
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -883,8 +911,8 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
     launch(k_s1_dev_init, 1, 32, 0, s, S.dev);
     launch(k_s1_min, grid_for(m), kThreads, 0, s, d_points, d_tris, m, mean_dev, S.dev);
     launch(k_s1_max, grid_for(m), kThreads, 0, s, d_points, d_tris, m, mean_dev, S.dev);
-    launch(k_s1_normalise, grid_for(m), kThreads, 0, s, d_points, d_tris, m, mean_dev, (const int *)S.dev,
-           (float)band, (float)margin, S.tris);
+    launch(k_s1_normalise, grid_for(m), kThreads, 0, s, d_points, d_tris, m, mean_dev, S.dev, (float)band,
+           (float)margin, R, S.tris);
     // 2. unsigned distance: squared distances start at band^2 (bits of a double)
     if (S.prof) S.prof->begin(PH_S1_DIST, s);
     const double b2 = band * band;
@@ -892,7 +920,8 @@ int remesh(Stage1 &S, const float *d_points, const int *d_tris, int n_pts, int m
     memcpy(&fill, &b2, 8);
     launch(k_s1_fill, grid_for(n3), kThreads, 0, s, S.field, n3, fill);  // cudaMemset only sets bytes
     const double inv_r = (R & (R - 1)) == 0 ? 1.0 / R : 0.0;
-    launch(k_s1_udist, grid_for(32LL * m), 256, 0, s, (const float *)S.tris, m, R, inv_r, kReach / R, S.field);
+    launch(k_s1_udist, grid_for(32LL * m), 256, 0, s, (const float *)S.tris, m, R, inv_r, band,
+           (const int *)S.dev, S.field);
     const int W = (R + 31) / 32, C = R - 1;
     const long long words = (long long)R * R * W;
     const Bits bits{R, W, S.bits, S.bits + words, S.bits + 2 * words, S.bits + 3 * words};
