@@ -117,11 +117,8 @@ __global__ void __launch_bounds__(kPairThreads) k_ck_pairs(const __grid_constant
                                                            unsigned long long *cnt)
 {
     __shared__ int2 s_pairs[kPairThreads / 32][64];  // leaves of f and g
-    __shared__ int s_off[kTreeMaxLevels];
-#pragma unroll
-    for (int l = 0; l < kTreeMaxLevels; ++l)
-        if (threadIdx.x == l) s_off[l] = T.off[l];
-    __syncthreads();
+    __shared__ int2 s_lvl[kTreeMaxLevels];
+    T.levels(s_lvl);
     int2 *buf = s_pairs[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
     const unsigned below = (1u << lane) - 1u;
@@ -150,11 +147,14 @@ __global__ void __launch_bounds__(kPairThreads) k_ck_pairs(const __grid_constant
         while (__any_sync(0xffffffffu, wk.run)) {
             bool hit = false, emit = false;
             const int node = 8 * wk.g + gl;
-            if (wk.run && T.holds(wk.lvl, node)) {
-                const size_t b = 2 * ((size_t)s_off[wk.lvl] + node);
+            if (wk.run) {
+                const int2 level = s_lvl[wk.lvl];
+                const size_t b = 2 * ((size_t)level.x + node);
                 const float4 lo = T.boxes[b], hi = T.boxes[b + 1];
-                const int g = wk.lvl == 0 ? T.leaf[node].w : kLeafDead;
-                hit = !(hi.x < qlo.x || qhi.x < lo.x || hi.y < qlo.y || qhi.y < lo.y || hi.z < qlo.z || qhi.z < lo.z);
+                const bool leaf = wk.lvl == 0 && node < T.L;
+                const int g = leaf ? T.leaf[node].w : kLeafDead;
+                hit = !(hi.x < qlo.x || qhi.x < lo.x || hi.y < qlo.y || qhi.y < lo.y || hi.z < qlo.z || qhi.z < lo.z) &&
+                      node <= level.y;
                 emit = hit && g > f;  // selected leaves have their face's number, the others a negative one
             }
             const unsigned hits = __ballot_sync(0xffffffffu, hit), em = __ballot_sync(0xffffffffu, emit);
@@ -362,7 +362,7 @@ struct HdEntry {
     int lvl, g;
 };
 
-__device__ __forceinline__ double nearest_d2(bool has, D3 p, const TreeView &T, const int *off, HdEntry *stack,
+__device__ __forceinline__ double nearest_d2(bool has, D3 p, const TreeView &T, const int2 *levels, HdEntry *stack,
                                              const float4 *__restrict__ pts)
 {
     constexpr unsigned kAll = 0xffffffffu;
@@ -373,8 +373,9 @@ __device__ __forceinline__ double nearest_d2(bool has, D3 p, const TreeView &T, 
     while (__any_sync(kAll, run)) {
         const int node = 8 * g + gl;
         double d = DBL_MAX;
-        if (run && T.holds(lvl, node)) {
-            const size_t b = 2 * ((size_t)off[lvl] + node);
+        const int2 level = levels[lvl];
+        if (run && node <= level.y) {
+            const size_t b = 2 * ((size_t)level.x + node);
             d = box_d2(T.boxes[b], T.boxes[b + 1], p);
             if (lvl == 0) {
                 const int4 t = d < best ? T.leaf[node] : make_int4(0, 0, 0, kLeafDead);
@@ -498,13 +499,8 @@ __global__ void __launch_bounds__(kHdThreads) k_hd_samples(const float4 *__restr
                                                            double *part_sum, double *part_edge)
 {
     __shared__ HdEntry s_stack[GROUP ? kHdThreads / 8 : 1][GROUP ? kHdStack : 1];
-    __shared__ int s_off[kTreeMaxLevels];
-    if constexpr (GROUP) {
-#pragma unroll
-        for (int l = 0; l < kTreeMaxLevels; ++l)
-            if (threadIdx.x == l) s_off[l] = T.off[l];
-        __syncthreads();
-    }
+    __shared__ int2 s_lvl[kTreeMaxLevels];
+    if constexpr (GROUP) T.levels(s_lvl);
     constexpr int kPer = GROUP ? 4 : 32;  // samples a warp
     const int lane = threadIdx.x & 31;
     const int S = (k + 1) * (k + 2) / 2;
@@ -534,7 +530,7 @@ __global__ void __launch_bounds__(kHdThreads) k_hd_samples(const float4 *__restr
         const D3 q = {a.x + su * (b.x - a.x) + sv * (c.x - a.x), a.y + su * (b.y - a.y) + sv * (c.y - a.y),
                       a.z + su * (b.z - a.z) + sv * (c.z - a.z)};
         double d2 = 0.0;
-        if constexpr (GROUP) d2 = nearest_d2(has, q, T, s_off, s_stack[threadIdx.x >> 3], pb);
+        if constexpr (GROUP) d2 = nearest_d2(has, q, T, s_lvl, s_stack[threadIdx.x >> 3], pb);
         else if (has) d2 = nearest_d2(q, V.nodes, V.parent, V.vals, V.scene[7], pb, fb);
         if (!has || (GROUP && (lane & 7) != 0)) continue;
         mx = fmax(mx, d2);

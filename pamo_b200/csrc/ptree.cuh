@@ -35,10 +35,17 @@ struct TreeView {
     int off[kTreeMaxLevels];
     int count[kTreeMaxLevels];  // nodes that cover a leaf or its tile's padding
 
-    // Whether node i of level l covers a leaf.  Every walk asks: the nodes of the
-    // levels' padding are empty, but a query box that is NaN or infinite on all
-    // axes is apart from none, and the children of padding lie outside the tree.
-    __device__ __forceinline__ bool holds(int l, int i) const { return i <= (L - 1) >> (3 * l); }
+    // A block's copy of what a walk needs of each level: where its boxes start, and the
+    // last node that covers a leaf.  A walk enters none beyond: the nodes of the levels'
+    // padding (which it may read) are empty, but a query box that is NaN or infinite on
+    // all axes is apart from none, and the children of padding lie outside the tree.
+    __device__ __forceinline__ void levels(int2 *shared) const
+    {
+#pragma unroll
+        for (int l = 0; l < kTreeMaxLevels; ++l)
+            if (threadIdx.x == l) shared[l] = make_int2(off[l], (L - 1) >> (3 * l));
+        __syncthreads();
+    }
 };
 
 // leaf_code: the face of a leaf, and whether it is selected (queries, and not

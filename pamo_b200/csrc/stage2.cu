@@ -1041,11 +1041,8 @@ __global__ void __launch_bounds__(kQueryThreads) k_query(const __grid_constant__
 {
     chain_wait();
     __shared__ uint2 s_pairs[kQueryThreads / 32][64];
-    __shared__ int s_off[kTreeMaxLevels];  // indexed by a lane's own level
-#pragma unroll
-    for (int l = 0; l < kTreeMaxLevels; ++l)
-        if (threadIdx.x == l) s_off[l] = T.off[l];
-    __syncthreads();
+    __shared__ int2 s_lvl[kTreeMaxLevels];  // indexed by a lane's own level
+    T.levels(s_lvl);
     uint2 *buf = s_pairs[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, gl = lane & 7, shift = lane & 24;
     const unsigned below = (1u << lane) - 1u;
@@ -1076,12 +1073,13 @@ __global__ void __launch_bounds__(kQueryThreads) k_query(const __grid_constant__
             bool hit = false, emit = false;
             int other = 0;
             const int node = 8 * wk.g + gl;
-            if (wk.run && T.holds(wk.lvl, node)) {
-                const size_t b = 2 * ((size_t)s_off[wk.lvl] + node);
+            if (wk.run) {
+                const int2 level = s_lvl[wk.lvl];
+                const size_t b = 2 * ((size_t)level.x + node);
                 const float4 lo = T.boxes[b], hi = T.boxes[b + 1];
-                const bool leaf = wk.lvl == 0;
+                const bool leaf = wk.lvl == 0 && node < T.L;
                 const int4 r = leaf ? T.leaf[node] : make_int4(-1, -1, -1, kLeafDead);
-                hit = box_overlap(lo, hi, qlo, qhi);
+                hit = box_overlap(lo, hi, qlo, qhi) && node <= level.y;
                 if (BATCH) {
                     const long long first = (long long)node << (3 * wk.lvl), end = ((long long)node + 1) << (3 * wk.lvl);
                     hit = hit && first < rg.y && end > rg.x;
